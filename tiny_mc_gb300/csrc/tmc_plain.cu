@@ -18,7 +18,20 @@
 
 namespace tmc {
 
-constexpr int CHUNK = 256;      // photon ids a warp claims per atomic
+// Photon ids a warp claims per atomic, 32 .. 256: a quarter of an even share of
+// the launch, so that every resident warp has photons and the last claims are
+// short.  A lane walks its warp's photons one after another, so a claim of
+// 256 is eight photons in a row per lane whatever else is idle: with it fixed
+// at 256, 2^19 high-albedo photons kept 2048 of 7296 warps busy (53.7 ms,
+// 40.5 ms now) and 32768 photons ran on 8 of 152 SMs (695 us, 167 us
+// now).  Below 32 a warp's lanes would need several claims to start.
+constexpr unsigned MIN_CHUNK = 32, MAX_CHUNK = 256;
+
+static unsigned claim_chunk(unsigned long long n_photons, unsigned long long warps)
+{
+    const unsigned long long share = n_photons / (4 * warps) / MIN_CHUNK * MIN_CHUNK;
+    return (unsigned)std::max<unsigned long long>(MIN_CHUNK, std::min<unsigned long long>(MAX_CHUNK, share));
+}
 
 struct PlainArgs {
     PhiloxKeys keys;
@@ -28,6 +41,7 @@ struct PlainArgs {
     unsigned long long *tally;   // [shells][4]: w lo, w hi, w2 lo, w2 hi
     unsigned long long *work;    // photon claim counter, zero at launch
     unsigned long long *steps;   // += photon steps, may be null
+    unsigned chunk;              // photon ids per claim
 };
 
 template <int BLOCK, class M, Hist H>
@@ -41,13 +55,14 @@ __global__ void __launch_bounds__(BLOCK) walk_plain(const PlainArgs a)
         smem[s] = 0;
     __syncthreads();
 
-    GlobalSource<CHUNK> src;
+    GlobalSource src;
     src.counter = a.work;
     src.n = a.n_photons;
     src.id_base = a.id_base;
+    src.chunk = a.chunk;
     uint32_t *my = smem + words + threadIdx.x;   // ring slot k: my[k * BLOCK]
     uint32_t *tally = PER_WARP ? smem + (threadIdx.x / 32) * 4 * S : smem;
-    const uint32_t steps = walk_loop<BLOCK, M, GlobalSource<CHUNK>, H, REFILL_MIN_SHORT>(
+    const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H, REFILL_MIN_SHORT>(
         a.c, src, a.keys, tally, a.tally, my);
 
     if constexpr (PER_WARP) {
@@ -103,7 +118,8 @@ static cudaError_t launch_t(const PlainLaunch &L, const DeviceCtx &ctx, int per_
         per_sm = std::min(per_sm, L.blocks_per_sm);
     unsigned long long grid = (unsigned long long)ctx.sms * per_sm;
     // no more blocks than there are photon chunks to hand out
-    const unsigned long long warps_needed = (L.n_photons + CHUNK - 1) / CHUNK;
+    const unsigned chunk = claim_chunk(L.n_photons, grid * (BLOCK / 32));
+    const unsigned long long warps_needed = (L.n_photons + chunk - 1) / chunk;
     const unsigned long long blocks_needed = (warps_needed + BLOCK / 32 - 1) / (BLOCK / 32);
     grid = std::max(1ull, std::min(grid, blocks_needed));
     if (L.max_blocks > 0)
@@ -120,6 +136,7 @@ static cudaError_t launch_t(const PlainLaunch &L, const DeviceCtx &ctx, int per_
     a.tally = reinterpret_cast<unsigned long long *>(L.d_tally);
     a.work = L.d_work;
     a.steps = L.d_steps;
+    a.chunk = chunk;
     walk_plain<BLOCK, M, H><<<(unsigned)grid, BLOCK, smem, stream>>>(a);
     return cudaGetLastError();
 }
@@ -157,8 +174,17 @@ static cudaError_t launch_b(const PlainLaunch &L, const DeviceCtx &ctx, cudaStre
 cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
     // 512 threads by default: 3 blocks of 512 and 6 of 256 both fill the SM's
-    // 1536 threads at 40 registers, and 512 measured 0.8% faster
-    switch (L.block ? L.block : 512) {
+    // 1536 threads at 40 registers, and 512 measured 0.8% faster.  A launch too
+    // small to give every SM a block of 512 takes blocks of 128, which spread
+    // the same warps over four times as many SMs.
+    const bool small = L.n_photons < (unsigned long long)ctx.sms * 512;
+    // a launch of no photons is a caller's set-up call: it loads both shapes
+    if (L.n_photons == 0 && !L.block) {
+        const cudaError_t e = launch_b<512>(L, ctx, stream);
+        if (e != cudaSuccess)
+            return e;
+    }
+    switch (L.block ? L.block : small ? 128 : 512) {
     case 128: return launch_b<128>(L, ctx, stream);
     case 256: return launch_b<256>(L, ctx, stream);
     case 512: return launch_b<512>(L, ctx, stream);

@@ -133,12 +133,12 @@ struct WalkConsts {
 };
 
 // Photon ids from a global 64-bit counter over [0, n): each warp claims
-// CHUNK ids per atomic.
-template <int CHUNK>
+// `chunk` ids per atomic.
 struct GlobalSource {
     unsigned long long *counter;
     unsigned long long n;
     unsigned long long id_base;
+    unsigned chunk;   // at least 32: one claim serves every lane of the warp
     unsigned long long cnext = 0, cend = 0;
     bool exhausted = false;
 
@@ -156,14 +156,14 @@ struct GlobalSource {
             unsigned long long base = 0;
             if (!exhausted) {
                 if (lane == 0)
-                    base = atomicAdd(counter, (unsigned long long)CHUNK);
+                    base = atomicAdd(counter, (unsigned long long)chunk);
                 base = __shfl_sync(FULL_MASK, base, 0);
                 exhausted = base >= n;
             }
             if (exhausted) {
                 cnext = cend;
             } else {
-                cend = min(base + (unsigned long long)CHUNK, n);
+                cend = min(base + (unsigned long long)chunk, n);
                 if (!got) {
                     id = base + (rank - take0);
                     got = id < cend;
