@@ -61,6 +61,45 @@ __device__ __forceinline__ uint4 philox4x32_10(uint32_t c0, uint32_t c1, uint32_
     return make_uint4(c0, c1, c2, c3);
 }
 
+// The parts of a photon's Philox blocks that do not depend on the block
+// number: the counter is {block, 0, id low, id high}, so half of the first
+// round and half of the second are the same for every block of a photon.
+struct PhotonKey {
+    uint32_t a, b, c, d;
+};
+
+__device__ __forceinline__ PhotonKey photon_key(unsigned long long pid, const PhiloxKeys &K)
+{
+    const unsigned long long p1 = (unsigned long long)PHILOX_M1 * (uint32_t)pid;
+    const unsigned long long q0 = (unsigned long long)PHILOX_M0 * ((uint32_t)(p1 >> 32) ^ K.k0[0]);
+    PhotonKey k;
+    k.a = (uint32_t)p1 ^ K.k0[1];
+    k.b = (uint32_t)(pid >> 32) ^ K.k1[0];
+    k.c = (uint32_t)(q0 >> 32) ^ K.k1[1];
+    k.d = (uint32_t)q0;
+    return k;
+}
+
+// philox4x32_10(blk, 0, id low, id high) with the photon's key parts.
+__device__ __forceinline__ uint4 philox_block(uint32_t blk, const PhotonKey &k, const PhiloxKeys &K)
+{
+    const unsigned long long p0 = (unsigned long long)PHILOX_M0 * blk;
+    const unsigned long long p1 = (unsigned long long)PHILOX_M1 * ((uint32_t)(p0 >> 32) ^ k.b);
+    uint32_t c0 = (uint32_t)(p1 >> 32) ^ k.a, c1 = (uint32_t)p1, c2 = (uint32_t)p0 ^ k.c, c3 = k.d;
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+        const unsigned long long q0 = (unsigned long long)PHILOX_M0 * c0;
+        const unsigned long long q1 = (unsigned long long)PHILOX_M1 * c2;
+        const uint32_t n0 = (uint32_t)(q1 >> 32) ^ c1 ^ K.k0[r];
+        const uint32_t n2 = (uint32_t)(q0 >> 32) ^ c3 ^ K.k1[r];
+        c1 = (uint32_t)q1;
+        c3 = (uint32_t)q0;
+        c0 = n0;
+        c2 = n2;
+    }
+    return make_uint4(c0, c1, c2, c3);
+}
+
 // rand() of photon.c: 31 bits of a Philox word; 0 becomes 1 so that
 // -log(rand()/RAND_MAX) is always finite (the reference's logf(0) case).
 __device__ __forceinline__ uint32_t rand31(uint32_t word)
@@ -116,10 +155,14 @@ __device__ __forceinline__ float log_exact(float x)
     return __fmaf_rn(kf, 0.693145751953125f, __fmaf_rn(kf, 1.42860682e-6f, lm));
 }
 
+// The forms that flush denormals: the same values as the plain ones without
+// their range checks (eight instructions less per photon step over the
+// logarithm and the two square roots).  U >= 2^-31 and 1 - t >= 2^-24 or 0; a
+// radius below 2^-63 mean free paths is taken as 0.
 __device__ __forceinline__ float sqrt_approx(float x)
 {
     float r;
-    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
@@ -144,10 +187,14 @@ struct ExactMath {
     {
         return __fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b));
     }
-    // sqrtf((1.0f - u*u) / t), photon.c:42-43
-    __device__ static __forceinline__ float dir_scale(float t, float u)
+    static constexpr float ONE = 1.0f;   // the launch direction's w
+    // photon.c:41-43 from an accepted try
+    __device__ static __forceinline__ void direction(float t, float xi1, float xi2, float &u, float &v, float &w)
     {
-        return __fsqrt_rn(__fdiv_rn(__fsub_rn(1.0f, __fmul_rn(u, u)), t));
+        u = fmaf(2.0f, t, -1.0f);
+        const float sc = __fsqrt_rn(__fdiv_rn(__fsub_rn(1.0f, __fmul_rn(u, u)), t));
+        v = __fmul_rn(xi1, sc);
+        w = __fmul_rn(xi2, sc);
     }
     __device__ static __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 };
@@ -155,46 +202,87 @@ struct ExactMath {
 // Hardware approximations (MUFU lg2 / sqrt), contraction allowed.
 struct FastMath {
     static constexpr uint32_t id = TMC_MATH_FAST;
-    __device__ static __forceinline__ float step_length(float U) { return -__logf(U); }
+    // twice the step; directions are kept halved (both scalings are exact)
+    __device__ static __forceinline__ float step_length(float U)
+    {
+        float l;
+        asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(U));
+        return l * (-2.0f * 0.693147182464599609375f);
+    }
     __device__ static __forceinline__ float move(float x, float t, float u) { return fmaf(t, u, x); }
     __device__ static __forceinline__ float radius_shells(float x, float y, float z, float spm)
     {
         return sqrt_approx(fmaf(x, x, fmaf(y, y, z * z))) * spm;
     }
     __device__ static __forceinline__ float norm2(float a, float b) { return fmaf(a, a, b * b); }
+    static constexpr float ONE = 0.5f;   // the launch direction's w, halved
     // (1-u^2)/t with u = 2t-1 is 4(1-t): sqrt of it is 2 sqrt(1-t)
-    __device__ static __forceinline__ float dir_scale(float t, float)
+    __device__ static __forceinline__ void direction(float t, float xi1, float xi2, float &u, float &v, float &w)
     {
-        return 2.0f * sqrt_approx(1.0f - t);
+        u = t - 0.5f;
+        const float sc = sqrt_approx(1.0f - t);
+        v = xi1 * sc;
+        w = xi2 * sc;
     }
     __device__ static __forceinline__ float mul(float a, float b) { return a * b; }
 };
 
 // ---------------------------------------------------------------- tallies
-// Fixed point of a deposit weight: rint(w * 2^40), returned as 32-bit halves,
-// for 0 <= w <= 1 (a deposit is at most 2^40 units).  hi = floor(w * 2^8);
-// the remainder w*2^40 - hi*2^32 is exact in one fused multiply-add (it is
-// the low part of w's own significand), and its correctly rounded conversion
-// is the low word: exact for w >= 2^-17, where w*2^40 is an integer, and
-// round-to-nearest-even below.  No branch, and no float->u64 conversion (that
-// one runs on the FP64 pipe).
-__device__ __forceinline__ void fx40_split(float w, uint32_t &lo, uint32_t &hi)
+// A photon's weight is kept times 2^20, so that w and w^2 in tally units of
+// 2^-40 are one multiplication away: w 2^40 = W 2^20 and fl(w w) 2^40 =
+// fl(W W) with W = w 2^20 (both scalings are exact; weights whose unscaled
+// product would be denormal deposit zero units either way).
+constexpr float WEIGHT_ONE = 0x1p20f;
+__device__ __forceinline__ float weight_units(float W) { return W * 0x1p20f; }
+__device__ __forceinline__ float weight2_units(float W) { return __fmul_rn(W, W); }
+
+// A deposit of q units (0 <= q <= 2^40, not necessarily whole) as 32-bit
+// halves of rint(q), round to nearest even.  Adding 2^55, whose float spacing
+// is 2^32, with rounding towards zero leaves floor(q / 2^32) in the low
+// mantissa bits: hi_bits = UNITS_HI_BIAS + that.  The rest is exact in float
+// (it is the low part of q's own significand) and below 2^32; its correctly
+// rounded conversion is the low word.  Five instructions, against six for a
+// truncating conversion and back.
+constexpr uint32_t UNITS_HI_BIAS = 0x5B000000u;   // the bits of 2^55f
+__device__ __forceinline__ void units_split(float q, uint32_t &lo, uint32_t &hi_bits)
 {
-    hi = __float2uint_rz(w * 0x1p8f);
-    const float rem = fmaf(-__uint2float_rn(hi), 0x1p32f, w * 0x1p40f);
-    lo = __float2uint_rn(rem);
+    const float a = __fadd_rz(q, 0x1p55f);
+    hi_bits = __float_as_uint(a);
+    lo = __float2uint_rn(__fsub_rn(q, __fsub_rn(a, 0x1p55f)));
 }
 
-// Add (hi:lo) to a 64-bit shared-memory tally kept as two 32-bit words, with
-// native 32-bit shared atomics: the carry out of the low word goes into the
-// high word, and a wrap of the high word carries 2^64 units into the 128-bit
-// global tally.  The global word receives only such carries until the final
-// flush, so no epoch barriers are needed however many photons a block walks.
-// wraps (may be null) additionally counts this tally's 2^64 wraps.
-__device__ __forceinline__ void tally_add(uint32_t *sh_lo, uint32_t *sh_hi,
-                                          unsigned long long *g_hi, uint32_t lo, uint32_t hi,
-                                          uint32_t *wraps = nullptr)
+// Shared-memory atomics by 32-bit shared address.
+__device__ __forceinline__ uint32_t atom_shared_add(uint32_t addr, uint32_t v)
 {
+    uint32_t old;
+    asm volatile("atom.shared.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v));
+    return old;
+}
+__device__ __forceinline__ void red_shared_add(uint32_t addr, uint32_t v)
+{
+    asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v));
+}
+
+// Add a deposit (units_split's halves) to a 64-bit shared-memory tally kept as
+// two 32-bit words, with native 32-bit shared atomics: the carry out of the
+// low word goes into the high word.  The caller bounds the sum below 2^64.
+__device__ __forceinline__ void tally_add_nowrap(uint32_t lo_addr, uint32_t hi_addr, uint32_t lo, uint32_t hi_bits)
+{
+    const uint32_t old = atom_shared_add(lo_addr, lo);
+    uint32_t hi;   // hi_bits - UNITS_HI_BIAS + (old + lo carries)
+    asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %1, %2;\n\taddc.u32 %0, %3, %4;\n\t}"
+        : "=r"(hi)
+        : "r"(old), "r"(lo), "r"(hi_bits), "n"(0u - UNITS_HI_BIAS));
+    red_shared_add(hi_addr, hi);
+}
+
+// The same where the sum may wrap: a wrap of the high word carries 2^64 units
+// into the 128-bit global tally, which receives only such carries until the
+// final flush.  wraps (may be null) additionally counts this tally's wraps.
+__device__ __forceinline__ void tally_add(uint32_t *sh_lo, uint32_t *sh_hi, unsigned long long *g_hi,
+                                          uint32_t lo, uint32_t hi_bits, uint32_t *wraps = nullptr)
+{
+    uint32_t hi = hi_bits - UNITS_HI_BIAS;
     const uint32_t old = atomicAdd(sh_lo, lo);
     hi += (old + lo < old) ? 1u : 0u;
     const uint32_t oh = atomicAdd(sh_hi, hi);
@@ -203,15 +291,6 @@ __device__ __forceinline__ void tally_add(uint32_t *sh_lo, uint32_t *sh_hi,
         if (wraps)
             atomicAdd(wraps, 1u);
     }
-}
-
-// tally_add for a 64-bit sum that cannot wrap (the caller bounds it): the
-// low word's carry goes into the high word, whose old value is not needed.
-__device__ __forceinline__ void tally_add_nowrap(uint32_t *sh_lo, uint32_t *sh_hi, uint32_t lo, uint32_t hi)
-{
-    const uint32_t old = atomicAdd(sh_lo, lo);
-    hi += (old + lo < old) ? 1u : 0u;
-    atomicAdd(sh_hi, hi);
 }
 
 // Flush a 64-bit partial sum into a 128-bit global tally.

@@ -5,7 +5,7 @@
 // tmc_walk.cuh.  Deposits go into shared-memory histograms of the problem's
 // shells: one per warp where that fits without costing occupancy, else one
 // per block; each is added into the 128-bit global tally every flush_steps
-// lane steps (2^18 for a warp's, 2^23 / threads for a block's) and at the
+// iterations (2^18 for a warp's, 2^23 / threads for a block's) and at the
 // end.
 // Shell counts whose histogram does not fit in shared memory at all
 // (params.h's SHELLS is any size in the reference) take the global form:
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(BLOCK) walk_plain(const PlainArgs a)
     src.chunk = a.chunk;
     uint32_t *my = smem + words + threadIdx.x;   // ring slot k: my[k * BLOCK]
     uint32_t *tally = PER_WARP ? smem + (threadIdx.x / 32) * 4 * S : smem;
-    const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H, REFILL_MIN_SHORT>(
+    const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H>(
         a.c, src, a.keys, tally, a.tally, my);
 
     if constexpr (PER_WARP) {
@@ -173,8 +173,7 @@ static cudaError_t launch_b(const PlainLaunch &L, const DeviceCtx &ctx, cudaStre
 
 cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
-    // 512 threads by default: 3 blocks of 512 and 6 of 256 both fill the SM's
-    // 1536 threads at 40 registers, and 512 measured 0.8% faster.  A launch too
+    // 512 threads by default: 512 measured 0.8% faster than 256.  A launch too
     // small to give every SM a block of 512 takes blocks of 128, which spread
     // the same warps over four times as many SMs.
     const bool small = L.n_photons < (unsigned long long)ctx.sms * 512;

@@ -162,9 +162,11 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
     uint32_t it_c = open[0].item;
 
     // ---- lane state
-    bool alive = false, want = true, pending = false;
-    uint32_t pid_lo = 0, pid_hi = 0, blk = 0, prod = 0, cur = 0;
-    float x = 0.f, y = 0.f, z = 0.f, u = 0.f, v = 0.f, w = 1.f, weight = 1.f;
+    using R = Ring<BLOCK>;
+    char *ring = reinterpret_cast<char *>(my);
+    LanePhoton p{};
+    R::drop(p);
+    bool want = true;                         // this lane takes another photon
     uint32_t lb = 0;                          // buffer of this lane's photon
     uint32_t steps = 0;                       // steps of this lane's photon
     // the constants of this lane's photon's item, read from the buffer's
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
             const uint32_t rb = rep & 1u;
             if (vopen[rb].item == END_ITEM)
                 break;
-            if (__any_sync(FULL_MASK, alive && lb == rb))
+            if (__any_sync(FULL_MASK, R::walking(p) && lb == rb))
                 break;
             // the done count, after this warp's deposits into the item
             unsigned last = 0;
@@ -273,19 +275,9 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
                 }
                 const bool mine = ((need >> lane) & 1u) && rank < k;
                 if (mine) {
-                    // launch, photon.c:12-18
                     const unsigned long long pid = open[cb].id_first + (cn + rank);
-                    pid_lo = (uint32_t)pid;
-                    pid_hi = (uint32_t)(pid >> 32);
+                    launch_photon<M>(p, pid, a.keys);
                     want = false;
-                    alive = true;
-                    blk = 0;
-                    cur = prod;
-                    pending = false;
-                    x = y = z = 0.f;
-                    u = v = 0.f;
-                    w = 1.f;
-                    weight = 1.f;
                     lb = cb;
                     steps = 0;
                     pc = open[cb].c;
@@ -325,7 +317,7 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
             want = false;
         }
 
-        const bool any_alive = __any_sync(FULL_MASK, alive);
+        const bool any_alive = __any_sync(FULL_MASK, R::walking(p));
         if (!any_alive) {
             if (it_c == END_ITEM && rep >= jc)
                 break;   // all photons walked, all items reported
@@ -345,99 +337,32 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
         }
         wait_start = 0;
 
-        // -------- refill once REFILL_MIN_SHORT_ITEMS walking lanes are short of the
-        // 6 words an iteration may use (or every walking lane is), as walk_loop
-        for (;;) {
-            const unsigned low = __ballot_sync(FULL_MASK, alive && (prod - cur) < 6u);
-            if (low == 0 ||
-                (__popc(low) < REFILL_MIN_SHORT_ITEMS && low != __ballot_sync(FULL_MASK, alive)))
-                break;
-            if (alive && (prod - cur) <= (uint32_t)(RING - 4)) {
-                const uint4 r = philox4x32_10(blk, 0u, pid_lo, pid_hi, a.keys);
-                ++blk;
-                const uint32_t p = prod & (RING - 1);
-                uint32_t *dst = my + p * BLOCK;
-                dst[0 * BLOCK] = r.x;
-                dst[1 * BLOCK] = r.y;
-                dst[2 * BLOCK] = r.z;
-                dst[3 * BLOCK] = r.w;
-                uint32_t *mir = dst + RING * BLOCK;
-                if (p <= 4u) {
-                    mir[0 * BLOCK] = r.x;
-                    mir[1 * BLOCK] = r.y;
-                }
-                if (p == 0u) {
-                    mir[2 * BLOCK] = r.z;
-                    mir[3 * BLOCK] = r.w;
-                }
-                prod += 4;
-            }
-        }
-
-        if (alive && (prod - cur) >= 6u) {   // a short lane waits for the next refill
-            const uint32_t *rd = my + (cur & (RING - 1)) * BLOCK;
-            if (!pending) {
-                // move, photon.c:21-24
-                const float U = uniform01(rd[0]);
-                rd += BLOCK;
-                ++cur;
-                const float t = M::step_length(U);
-                x = M::move(x, t, u);
-                y = M::move(y, t, v);
-                z = M::move(z, t, w);
-                // absorb, photon.c:26-32
-                const WalkConsts c = pc;
-                const float rr = M::radius_shells(x, y, z, c.spm);
-                const uint32_t shell = __float2uint_rz(fminf(rr, c.last));
-                const uint32_t S = c.shells;
-                uint32_t *t0 = smem + lb * HS + shell;
-                unsigned long long *g = pg;
-                uint32_t lo, hi;
-                fx40_split(weight, lo, hi);
-                tally_add(t0, t0 + S, &g[4 * shell + 1], lo, hi,
-                          shell == pps ? (uint32_t *)&open[lb].wraps : nullptr);
-                fx40_split(__fmul_rn(weight, weight), lo, hi);
-                tally_add(t0 + 2 * S, t0 + 3 * S, &g[4 * shell + 3], lo, hi);
-                weight = M::mul(weight, c.albedo);
-                ++steps;
-            }
-            // the next two tries of the rejection method, photon.c:36-40
-            const float xa1 = uniform_pm1(rd[0 * BLOCK]);
-            const float xa2 = uniform_pm1(rd[1 * BLOCK]);
-            const float xb1 = uniform_pm1(rd[2 * BLOCK]);
-            const float xb2 = uniform_pm1(rd[3 * BLOCK]);
-            const float ta = M::norm2(xa1, xa2);
-            const float tb = M::norm2(xb1, xb2);
-            const bool first = !(1.0f < ta);
-            const float xi1 = first ? xa1 : xb1;
-            const float xi2 = first ? xa2 : xb2;
-            const float tt = first ? ta : tb;
-            rd += first ? 2 * BLOCK : 4 * BLOCK;
-            cur += first ? 2u : 4u;
-            pending = (1.0f < tt);
-            if (!pending) {
-                // new direction, photon.c:41-43
-                u = fmaf(2.0f, tt, -1.0f);
-                const float sc = M::dir_scale(tt, u);
-                v = M::mul(xi1, sc);
-                w = M::mul(xi2, sc);
-                // roulette, photon.c:45-49
-                if (weight < 0.001f) {
-                    const float U = uniform01(rd[0]);
-                    ++cur;
-                    if (U > 0.1f) {
-                        alive = false;
-                        want = true;
-                        // the photon's steps into its item's 64-bit count
-                        uint32_t *sl = (uint32_t *)&open[lb].steps_lo;
-                        const uint32_t old = atomicAdd(sl, steps);
-                        if (old + steps < old)
-                            atomicAdd((uint32_t *)&open[lb].steps_hi, 1u);
-                    } else {
-                        weight = __fdiv_rn(weight, 0.1f);
-                    }
-                }
-            }
+        uint32_t *hist = smem + lb * HS;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            if (k % 2 == 0)
+                R::refill(p, ring, a.keys);
+            step_photon<BLOCK, M>(
+                p, ring, pc.spm, pc.last, pc.albedo,
+                [&](uint32_t shell, float weight) {
+                    const uint32_t S = pc.shells;
+                    uint32_t *t0 = hist + shell;
+                    uint32_t lo, hi;
+                    units_split(weight_units(weight), lo, hi);
+                    tally_add(t0, t0 + S, &pg[4 * shell + 1], lo, hi,
+                              shell == pps ? (uint32_t *)&open[lb].wraps : nullptr);
+                    units_split(weight2_units(weight), lo, hi);
+                    tally_add(t0 + 2 * S, t0 + 3 * S, &pg[4 * shell + 3], lo, hi);
+                    ++steps;
+                },
+                [&] {
+                    want = true;
+                    // the photon's steps into its item's 64-bit count
+                    uint32_t *sl = (uint32_t *)&open[lb].steps_lo;
+                    const uint32_t old = atomicAdd(sl, steps);
+                    if (old + steps < old)
+                        atomicAdd((uint32_t *)&open[lb].steps_hi, 1u);
+                });
         }
     }
     // every warp has left the loop (their waits are bounded)

@@ -16,24 +16,34 @@
 //    (p = 0.046) skips the move/absorb part on the next iteration, so lanes
 //    of a warp stay in lock-step instead of waiting for the lane with the
 //    most retries;
-//  * random words come from a per-thread ring of 16 words in shared memory,
-//    refilled four at a time from Philox; slots 16..21 mirror 0..5 so the
-//    <= 6 words one iteration reads are fixed offsets from one base.  An
-//    iteration needs >= 6 buffered words (it consumes at most six: step,
-//    four for two tries, roulette); the refill at the top runs once at least
-//    four walking lanes are short (a short lane waits an iteration or two
-//    rather than make the whole warp pay for a Philox block few lanes use),
-//    and then every lane with room refills, so Philox runs with most lanes
-//    active;
+//  * random words come from a per-thread ring of 16 words in shared memory;
+//    slots 16..20 mirror 0..4, so the <= 6 words one iteration reads (step,
+//    four for two tries, roulette) are fixed offsets from one base.  Every
+//    second iteration each lane computes two Philox blocks and stores them if
+//    its ring has room for eight words.  No vote decides on a refill: an
+//    iteration uses 3.4 words on average and a refill brings four per
+//    iteration, so a vote would save 6% of the Philox work and cost more
+//    than that; without it the loop is straight-line code whose Philox
+//    multiplies overlap the walk's arithmetic;
 //  * the two tallies of photon.c:30-31 go into a shared-memory histogram of
 //    64-bit fixed-point sums (sum of w and of w^2, 2^-40 units), each kept as
 //    two 32-bit words updated with native 32-bit shared atomics (a 64-bit
 //    shared atomicAdd is a compare-and-swap loop, 4x slower here).  The
 //    histogram is one per warp (the plain kernel, where that fits) or one per
-//    block; either way it is added into the 128-bit global tally and cleared
-//    each time one of its lanes' step count reaches a multiple of a bound
-//    (flush_steps), which keeps its 64-bit sums from wrapping, so a deposit
-//    needs no wrap check.
+//    block; either way a warp adds it into the 128-bit global tally and clears
+//    it every flush_steps iterations, which keeps its 64-bit sums from
+//    wrapping, so a deposit needs no wrap check.
+//
+// What bounds it: instruction issue, then the shared-memory pipe.  One photon
+// step takes 5.86 warp-instructions (8.34 before the loop took this form) at
+// 3.03 per clock per SM, shared-memory wavefronts 69% of peak (2^25 photons
+// of params.h optics, fast arithmetic).  2^26 such photons: 41.1 ms with voted
+// single-block refills, 35.1 with one unvoted block per iteration, 33.8 with
+// the loop body unrolled twice, 32.1 with two blocks every second iteration
+// (which share the round-key loads), 31.2 with four iterations per check for
+// finished photons.  Six and eight iterations gain under 1% more there and
+// leave lanes of short walks idle longer.  Occupancy does not matter at this
+// point: 48 warps per SM (40 registers) measured the same as 32.
 #pragma once
 
 #include "tmc_device.cuh"
@@ -41,18 +51,9 @@
 namespace tmc {
 
 constexpr int RING = 16;        // random words buffered per thread
-constexpr int MIRROR = 6;       // slots 16..21 repeat slots 0..5
+constexpr int MIRROR = 5;       // slots 16..20 repeat slots 0..4
 constexpr int SLOTS = RING + MIRROR;
-// The warp runs a Philox refill pass once this many walking lanes are short
-// of words (or every walking lane is).  Measured on the plain walk, 2^30
-// photons of params.h optics: 1 lane 716 ms, 2 lanes 683, 4 lanes 673, 8
-// lanes 681, 16 lanes 709.
-constexpr int REFILL_MIN_SHORT = 4;
-// The same for the batched kernels, whose warps run short of photons at the
-// end of every work item.  Measured on the 4096-problem sweep at 1/64 photon
-// scale: walk_batch (128 threads, 16 items) 1.04e11 photon-steps/s with 2
-// against 1.00e11 with 4; walk_stream (256, 16) 1.006e11 against 0.993e11.
-constexpr int REFILL_MIN_SHORT_ITEMS = 2;
+constexpr int TRIP = 4;         // iterations between checks for finished photons
 
 // Where a walk keeps its tallies.  Warp: one shared histogram per warp.
 // Block: one per block, shared by its warps.  Global: none; every deposit is
@@ -60,17 +61,14 @@ constexpr int REFILL_MIN_SHORT_ITEMS = 2;
 // histogram does not fit in shared memory).
 enum class Hist { Warp, Block, Global };
 
-// A shared histogram written by `lanes` lanes is added into the global tally
-// and cleared each time one of those lanes' step count reaches a multiple of
-// flush_steps(lanes), checked at the top of every iteration (in which a lane
-// steps at most once) for every lane that walks a photon or has just lost one
-// (a block's histogram skips lanes left without a photon at the end of a
-// small work item, which would otherwise flush on every iteration).  A lane's
-// count changes only while it walks, so every lane is checked at every
-// multiple it reaches and deposits at most flush_steps + 1 times between two
-// flushes.  A deposit adds at most 2^8 + 1 to a high word (w <= 1, plus the
-// low word's carry), so a high word stays below
-// lanes * 257 * (2^23 / lanes + 1) < 2^32: the 64-bit sums never wrap.
+// A warp adds the shared histogram it deposits into (its own, or its block's
+// of `lanes` lanes) into the global tally and clears it every
+// flush_steps(lanes) of its iterations.  A lane deposits at most once per
+// iteration, so between two flushes, whichever warps make them, every lane
+// deposits at most flush_steps times (its warp would have flushed).  A deposit
+// adds at most 2^8 + 1 to a high word (w <= 1, plus the low word's carry), so
+// a high word stays below lanes * 257 * (2^23 / lanes + 1) < 2^32: the 64-bit
+// sums never wrap.
 __host__ __device__ constexpr uint32_t flush_steps(uint32_t lanes)
 {
     return (1u << 23) / lanes;
@@ -221,15 +219,128 @@ struct SharedSource {
     }
 };
 
+// A lane's photon.  Ring positions are in bytes (slot x the W bytes between a
+// thread's slots) modulo 2^32: blk * 4 W is the end of the words produced,
+// cur the next word to use; their difference is the fill, and a lane without
+// a photon is kept at a fill of -W.
+struct LanePhoton {
+    PhotonKey key;
+    uint32_t blk = 0, cur = 0;
+    float x = 0.f, y = 0.f, z = 0.f, u = 0.f, v = 0.f, w = 0.f;
+    float weight = 0.f;   // times 2^20 (an exact scaling)
+    float t = 0.f;        // norm of the last try; above 1 the direction is still sought
+};
+
+template <int BLOCK>
+struct Ring {
+    static constexpr uint32_t W = BLOCK * 4;
+    static constexpr uint32_t MASK = RING * W - 1;
+    static constexpr uint32_t NO_PHOTON = W;   // cur - blk * 4 W of a lane without one
+
+    __device__ static __forceinline__ int fill(const LanePhoton &p) { return (int)(p.blk * (4 * W) - p.cur); }
+    __device__ static __forceinline__ bool walking(const LanePhoton &p) { return fill(p) >= 0; }
+    __device__ static __forceinline__ void drop(LanePhoton &p) { p.cur = p.blk * (4 * W) + NO_PHOTON; }
+    __device__ static __forceinline__ uint32_t word(const char *at, int slot)
+    {
+        return *reinterpret_cast<const uint32_t *>(at + slot * W);
+    }
+
+    // Two Philox blocks into the ring where it has room for them.
+    __device__ static __forceinline__ void refill(LanePhoton &p, char *ring, const PhiloxKeys &keys)
+    {
+        const uint4 r = philox_block(p.blk, p.key, keys);
+        const uint4 q = philox_block(p.blk + 1, p.key, keys);
+        if ((uint32_t)fill(p) <= (RING - 8) * W) {
+            const uint32_t off = (p.blk * (4 * W)) & MASK;
+            const uint32_t words[8] = {r.x, r.y, r.z, r.w, q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                *reinterpret_cast<uint32_t *>(ring + off + k * W) = words[k];
+            if (off == 0) {
+#pragma unroll
+                for (int k = 0; k < MIRROR; ++k)
+                    *reinterpret_cast<uint32_t *>(ring + off + (RING + k) * W) = words[k];
+            }
+            p.blk += 2;
+        }
+    }
+};
+
+// Photon launch, photon.c:12-18.
+template <class M>
+__device__ __forceinline__ void launch_photon(LanePhoton &p, unsigned long long pid, const PhiloxKeys &keys)
+{
+    p.key = photon_key(pid, keys);
+    p.blk = 0;
+    p.cur = 0;
+    p.x = p.y = p.z = 0.f;
+    p.u = p.v = 0.f;
+    p.w = M::ONE;
+    p.weight = WEIGHT_ONE;
+    p.t = 0.f;
+}
+
+// One iteration of a lane's photon if six words are buffered (else it waits
+// for the next refill): move, deposit and decay unless its direction is still
+// sought, then two tries for the next direction and the roulette.
+// deposit(shell, weight) tallies a step, died() is called at the photon's end.
+template <int BLOCK, class M, class Deposit, class Died>
+__device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, float spm, float last, float albedo,
+                                            Deposit deposit, Died died)
+{
+    using R = Ring<BLOCK>;
+    if (R::fill(p) < (int)(6 * R::W))
+        return;
+    const char *rd = ring + (p.cur & R::MASK);
+    if (!(p.t > 1.0f)) {
+        // move, photon.c:21-24
+        const float U = uniform01(R::word(rd, 0));
+        rd += R::W;
+        p.cur += R::W;
+        const float t = M::step_length(U);
+        p.x = M::move(p.x, t, p.u);
+        p.y = M::move(p.y, t, p.v);
+        p.z = M::move(p.z, t, p.w);
+        // absorb, photon.c:26-32 (clamp in float: same shell for every radius
+        // below 2^32 shells, and a NaN radius lands last)
+        deposit(__float2uint_rz(fminf(M::radius_shells(p.x, p.y, p.z, spm), last)), p.weight);
+        p.weight = M::mul(p.weight, albedo);
+    }
+    // the next two tries of the rejection method, photon.c:36-40; the second
+    // one's words are consumed only if the first is rejected
+    const float xa1 = uniform_pm1(R::word(rd, 0)), xa2 = uniform_pm1(R::word(rd, 1));
+    const float xb1 = uniform_pm1(R::word(rd, 2)), xb2 = uniform_pm1(R::word(rd, 3));
+    const float ta = M::norm2(xa1, xa2), tb = M::norm2(xb1, xb2);
+    const bool first = !(1.0f < ta);
+    const float xi1 = first ? xa1 : xb1;
+    const float xi2 = first ? xa2 : xb2;
+    p.t = first ? ta : tb;
+    p.cur += first ? 2 * R::W : 4 * R::W;
+    if (!(p.t > 1.0f)) {
+        M::direction(p.t, xi1, xi2, p.u, p.v, p.w);   // photon.c:41-43
+        // roulette, photon.c:45-49
+        if (p.weight < 0.001f * WEIGHT_ONE) {
+            const float U = uniform01(R::word(ring + (p.cur & R::MASK), 0));
+            p.cur += R::W;
+            if (U > 0.1f) {
+                R::drop(p);
+                died();
+            } else {
+                p.weight = __fdiv_rn(p.weight, 0.1f);
+            }
+        }
+    }
+}
+
 // Walk photons from `src` until it is exhausted and every lane's photon has
 // died.  Warp-collective: all 32 lanes of every warp call it.  tally: the
 // shared histogram (H = Warp: this warp's; Block: the block's), 4 * shells
 // words (low and high of sum w, then of sum w^2), flushed into g, the
-// problem's global 128-bit tally [shells][4], every flush_steps lane steps;
+// problem's global 128-bit tally [shells][4], every flush_steps iterations;
 // the caller flushes what is left.  probe_acc / probe_hi (Block only, may be
 // null): receive the w sums those flushes take from shell probe_shell.
 // Returns this thread's photon steps.
-template <int BLOCK, class M, class Source, Hist H, int MIN_SHORT = REFILL_MIN_SHORT_ITEMS>
+template <int BLOCK, class M, class Source, Hist H>
 __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               const PhiloxKeys &keys, uint32_t *tally,
                                               unsigned long long *g, uint32_t *my,
@@ -237,156 +348,65 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               uint32_t *probe_hi = nullptr,
                                               uint32_t probe_shell = 0)
 {
+    using R = Ring<BLOCK>;
+    constexpr uint32_t FLUSH_TRIPS = flush_steps(H == Hist::Warp ? 32u : (uint32_t)BLOCK) / TRIP;
     const uint32_t S = c.shells;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
+    char *ring = reinterpret_cast<char *>(my);
+    const uint32_t hist = (uint32_t)__cvta_generic_to_shared(tally);
 
-    bool alive = false, want = true, pending = false;
-    uint32_t pid_lo = 0, pid_hi = 0, blk = 0, prod = 0, cur = 0;
-    float x = 0.f, y = 0.f, z = 0.f, u = 0.f, v = 0.f, w = 1.f, weight = 1.f;
-    uint32_t steps = 0;
+    LanePhoton p{};
+    R::drop(p);
+    uint32_t steps = 0, trips = 0;
+    unsigned idle = 0;   // lanes that get no more photons
 
     for (;;) {
-        // -------- hand new photon ids to lanes whose photon died (shared
-        // histograms: also flush it when a lane's step count reaches a
-        // multiple of the flush bound)
-        constexpr bool SHARED = H != Hist::Global;
-        constexpr uint32_t FLUSH_MASK = flush_steps(H == Hist::Warp ? 32u : (uint32_t)BLOCK) - 1u;
-        const bool at_bound = (steps & FLUSH_MASK) == 0u && (H == Hist::Warp || alive || want);
-        const unsigned need = __ballot_sync(FULL_MASK, want || (SHARED && at_bound));
-        if (need) {
-            unsigned want_mask = need;
-            if constexpr (SHARED) {
-                if (__any_sync(FULL_MASK, at_bound)) {
-                    if constexpr (H == Hist::Warp)
-                        warp_flush_tally(tally, S, g);
-                    else
-                        swap_flush_tally(tally, S, g, probe_acc, probe_hi, probe_shell);
-                }
-                want_mask = __ballot_sync(FULL_MASK, want);
-            }
+        // -------- hand new photon ids to lanes whose photon died
+        const unsigned dead = __ballot_sync(FULL_MASK, !R::walking(p));
+        if (dead != idle) {
+            const unsigned need = dead & ~idle;
             unsigned long long pid = 0;
-            const bool got = want_mask ? src.next(want_mask, __popc(want_mask & lt_mask), lane, pid)
-                                       : false;
-            if (want) {
-                want = false;
-                alive = got;
-                // launch, photon.c:12-18
-                pid_lo = (uint32_t)pid;
-                pid_hi = (uint32_t)(pid >> 32);
-                blk = 0;
-                cur = prod;   // drop words buffered for the previous photon
-                pending = false;
-                x = y = z = 0.f;
-                u = v = 0.f;
-                w = 1.f;
-                weight = 1.f;
-            }
-            // lanes change from alive to idle only here
-            if (__ballot_sync(FULL_MASK, alive) == 0)
+            const bool got = src.next(need, __popc(need & lt_mask), lane, pid) && ((need >> lane) & 1u);
+            if (got)
+                launch_photon<M>(p, pid, keys);
+            idle = dead & ~__ballot_sync(FULL_MASK, got);
+            if (idle == FULL_MASK)
                 break;
         }
-
-        // -------- refill: an iteration needs >= 6 buffered words (it uses
-        // <= 6).  The warp runs Philox only once MIN_SHORT walking lanes
-        // are short (or every walking lane is): a refill costs the
-        // whole warp the same issue slots however many lanes take part, so a
-        // short lane waits instead (the others, using >= 2 words each per
-        // iteration, soon join it).  A fresh photon starts empty and needs two
-        // passes.
-        for (;;) {
-            const unsigned low = __ballot_sync(FULL_MASK, alive && (prod - cur) < 6u);
-            if (low == 0 ||
-                (__popc(low) < MIN_SHORT && low != __ballot_sync(FULL_MASK, alive)))
-                break;
-            if (alive && (prod - cur) <= (uint32_t)(RING - 4)) {
-                const uint4 r = philox4x32_10(blk, 0u, pid_lo, pid_hi, keys);
-                ++blk;
-                const uint32_t p = prod & (RING - 1);
-                uint32_t *dst = my + p * BLOCK;
-                dst[0 * BLOCK] = r.x;
-                dst[1 * BLOCK] = r.y;
-                dst[2 * BLOCK] = r.z;
-                dst[3 * BLOCK] = r.w;
-                // mirror: slots 16..19 repeat 0..3, slots 20..21 repeat 4..5
-                uint32_t *mir = dst + RING * BLOCK;
-                if (p <= 4u) {
-                    mir[0 * BLOCK] = r.x;
-                    mir[1 * BLOCK] = r.y;
-                }
-                if (p == 0u) {
-                    mir[2 * BLOCK] = r.z;
-                    mir[3 * BLOCK] = r.w;
-                }
-                prod += 4;
+        if constexpr (H != Hist::Global) {
+            if (++trips == FLUSH_TRIPS) {
+                trips = 0;
+                if constexpr (H == Hist::Warp)
+                    warp_flush_tally(tally, S, g);
+                else
+                    swap_flush_tally(tally, S, g, probe_acc, probe_hi, probe_shell);
             }
         }
-
-        if (alive && (prod - cur) >= 6u) {   // a short lane waits for the next refill
-            // the <= 6 words this iteration may read, from one base
-            const uint32_t *rd = my + (cur & (RING - 1)) * BLOCK;
-            if (!pending) {
-                // move, photon.c:21-24
-                const float U = uniform01(rd[0]);
-                rd += BLOCK;
-                ++cur;
-                const float t = M::step_length(U);
-                x = M::move(x, t, u);
-                y = M::move(y, t, v);
-                z = M::move(z, t, w);
-                // absorb, photon.c:26-32 (clamp in float: same shell for every
-                // radius below 2^32 shells, and a NaN radius lands last)
-                const float rr = M::radius_shells(x, y, z, c.spm);
-                const uint32_t shell = __float2uint_rz(fminf(rr, c.last));
-                uint32_t lo, hi;
-                if constexpr (H == Hist::Global) {
-                    fx40_split(weight, lo, hi);
-                    flush128(&g[4 * shell + 0], &g[4 * shell + 1], ((unsigned long long)hi << 32) | lo);
-                    fx40_split(__fmul_rn(weight, weight), lo, hi);
-                    flush128(&g[4 * shell + 2], &g[4 * shell + 3], ((unsigned long long)hi << 32) | lo);
-                } else {
-                    uint32_t *t0 = tally + shell;
-                    fx40_split(weight, lo, hi);
-                    tally_add_nowrap(t0, t0 + S, lo, hi);
-                    fx40_split(__fmul_rn(weight, weight), lo, hi);
-                    tally_add_nowrap(t0 + 2 * S, t0 + 3 * S, lo, hi);
-                }
-                weight = M::mul(weight, c.albedo);
-                ++steps;
-            }
-            // the next two tries of the rejection method, photon.c:36-40; the
-            // second one's words are consumed only if the first is rejected
-            const float xa1 = uniform_pm1(rd[0 * BLOCK]);
-            const float xa2 = uniform_pm1(rd[1 * BLOCK]);
-            const float xb1 = uniform_pm1(rd[2 * BLOCK]);
-            const float xb2 = uniform_pm1(rd[3 * BLOCK]);
-            const float ta = M::norm2(xa1, xa2);
-            const float tb = M::norm2(xb1, xb2);
-            const bool first = !(1.0f < ta);
-            const float xi1 = first ? xa1 : xb1;
-            const float xi2 = first ? xa2 : xb2;
-            const float tt = first ? ta : tb;
-            rd += first ? 2 * BLOCK : 4 * BLOCK;
-            cur += first ? 2u : 4u;
-            pending = (1.0f < tt);
-            if (!pending) {
-                // new direction, photon.c:41-43
-                u = fmaf(2.0f, tt, -1.0f);
-                const float sc = M::dir_scale(tt, u);
-                v = M::mul(xi1, sc);
-                w = M::mul(xi2, sc);
-                // roulette, photon.c:45-49
-                if (weight < 0.001f) {
-                    const float U = uniform01(rd[0]);
-                    ++cur;
-                    if (U > 0.1f) {
-                        alive = false;
-                        want = true;
+#pragma unroll
+        for (int k = 0; k < TRIP; ++k) {
+            if (k % 2 == 0)
+                R::refill(p, ring, keys);
+            step_photon<BLOCK, M>(
+                p, ring, c.spm, c.last, c.albedo,
+                [&](uint32_t shell, float weight) {
+                    uint32_t lo, hi;
+                    if constexpr (H == Hist::Global) {
+                        unsigned long long *gs = g + 4 * (size_t)shell;
+                        units_split(weight_units(weight), lo, hi);
+                        flush128(&gs[0], &gs[1], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
+                        units_split(weight2_units(weight), lo, hi);
+                        flush128(&gs[2], &gs[3], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
                     } else {
-                        weight = __fdiv_rn(weight, 0.1f);
+                        const uint32_t at = hist + 4 * shell;
+                        units_split(weight_units(weight), lo, hi);
+                        tally_add_nowrap(at, at + 4 * S, lo, hi);
+                        units_split(weight2_units(weight), lo, hi);
+                        tally_add_nowrap(at + 8 * S, at + 12 * S, lo, hi);
                     }
-                }
-            }
+                    ++steps;
+                },
+                [] {});
         }
     }
     return steps;
