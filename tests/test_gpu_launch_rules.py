@@ -42,3 +42,30 @@ def test_claim_sizes_agree(tmc_mod, n, math):
         tmc_mod.set_plain_launch(0, 0, 0)
     assert got[1] == ref[1]
     assert np.array_equal(got[0], ref[0])
+
+
+@pytest.mark.parametrize("math", ["exact", "fast"])
+@pytest.mark.parametrize("optics", [PARAMS_H, HIGH_ALBEDO, dict(shells=20000, microns_per_shell=5.0, mu_a=2.0, mu_s=20.0),
+                                    dict(shells=7, microns_per_shell=50.0, mu_a=10.0, mu_s=1.0),
+                                    dict(shells=101, microns_per_shell=50.0, mu_a=0.5, mu_s=50.0)])
+def test_whole_warp_walk_equals_lane_walk(tmc_mod, optics, math):
+    """Photons walked one to a warp (small launches, and the last photons of
+    every warp) against the same photons in the middle of a large launch, all
+    of whose other photons are subtracted: the tallies are sums over photons."""
+    tmc_mod.set_plain_launch(0, 0, 0)
+    n = 257
+    base = 5 << 20
+    few, few_steps = gpu_fx(tmc_mod, n, seed=4, base=base, math=math, **optics)
+    parts = [gpu_fx(tmc_mod, k, seed=4, base=b, math=math, **optics) for k, b in ((1, base), (n - 1, base + 1))]
+    assert sum(s for _, s in parts) == few_steps
+
+    def ints(t):
+        return [(int(r[1]) << 64 | int(r[0]), int(r[3]) << 64 | int(r[2])) for r in t]
+    summed = [tuple(x + y for x, y in zip(a, b)) for a, b in zip(ints(parts[0][0]), ints(parts[1][0]))]
+    assert summed == ints(few)
+    many = 40000 if optics is not HIGH_ALBEDO else 20000
+    before = gpu_fx(tmc_mod, many, seed=4, base=base - many, math=math, **optics)
+    both = gpu_fx(tmc_mod, many + n, seed=4, base=base - many, math=math, **optics)
+    assert both[1] - before[1] == few_steps
+    diff = [tuple(x - y for x, y in zip(a, b)) for a, b in zip(ints(both[0]), ints(before[0]))]
+    assert diff == ints(few)

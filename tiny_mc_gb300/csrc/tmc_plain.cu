@@ -12,23 +12,36 @@
 // deposits go straight into the 128-bit global tally with 64-bit atomics.  The
 // sums are the same integers in every form.
 #include <algorithm>
+#include <cmath>
 
 #include "tmc_internal.h"
 #include "tmc_walk.cuh"
 
 namespace tmc {
 
-// Photon ids a warp claims per atomic, 32 .. 256: a quarter of an even share of
-// the launch, so that every resident warp has photons and the last claims are
-// short.  A lane walks its warp's photons one after another, so a claim of
-// 256 is eight photons in a row per lane whatever else is idle: with it fixed
-// at 256, 2^19 high-albedo photons kept 2048 of 7296 warps busy (53.7 ms,
-// 40.5 ms now) and 32768 photons ran on 8 of 152 SMs (695 us, 167 us
-// now).  Below 32 a warp's lanes would need several claims to start.
+// Photon ids a warp claims per atomic.
+//
+// Large launches: a quarter of an even share, 32 to 256, so that every
+// resident warp has photons and the last claims are short.  A lane walks its
+// warp's photons one after another, so a claim of 256 is eight photons in a
+// row per lane whatever else is idle: with it fixed at 256, 2^19 high-albedo
+// photons kept 2048 of 7296 warps busy (53.7 ms against 40.5) and 32768
+// photons ran on 8 of 152 SMs (695 us against 167).
+//
+// Small launches: one photon, which the whole warp then walks (warp_steps).
+// With k steps to the first roulette that costs about n (k / 32 + 4) rounds
+// of 730 warp-instructions on the launch's schedulers, while on lanes it takes
+// the latency of k iterations whatever n.  Measured, lanes -> whole warps:
+// params.h optics (k = 73) 5000 photons 73 -> 67 us, 12000 75 -> 145 us; high
+// albedo (k = 6905) 4099 photons 4.2 -> 1.0 ms, 12000 4.3 -> 2.3 ms, 24000
+// 4.7 -> 4.7 ms.
 constexpr unsigned MIN_CHUNK = 32, MAX_CHUNK = 256;
 
-static unsigned claim_chunk(unsigned long long n_photons, unsigned long long warps)
+static unsigned claim_chunk(unsigned long long n_photons, unsigned long long warps, int sms, float albedo)
 {
+    const double k = albedo > 0.0f ? std::log(0.001) / std::log((double)albedo) : 0.0;
+    if ((double)n_photons < 28.0 * 4 * sms * k / (k + 128.0))
+        return 1;
     const unsigned long long share = n_photons / (4 * warps) / MIN_CHUNK * MIN_CHUNK;
     return (unsigned)std::max<unsigned long long>(MIN_CHUNK, std::min<unsigned long long>(MAX_CHUNK, share));
 }
@@ -118,7 +131,7 @@ static cudaError_t launch_t(const PlainLaunch &L, const DeviceCtx &ctx, int per_
         per_sm = std::min(per_sm, L.blocks_per_sm);
     unsigned long long grid = (unsigned long long)ctx.sms * per_sm;
     // no more blocks than there are photon chunks to hand out
-    const unsigned chunk = claim_chunk(L.n_photons, grid * (BLOCK / 32));
+    const unsigned chunk = claim_chunk(L.n_photons, grid * (BLOCK / 32), ctx.sms, L.d.albedo);
     const unsigned long long warps_needed = (L.n_photons + chunk - 1) / chunk;
     const unsigned long long blocks_needed = (warps_needed + BLOCK / 32 - 1) / (BLOCK / 32);
     grid = std::max(1ull, std::min(grid, blocks_needed));

@@ -54,6 +54,12 @@ constexpr int RING = 16;        // random words buffered per thread
 constexpr int MIRROR = 5;       // slots 16..20 repeat slots 0..4
 constexpr int SLOTS = RING + MIRROR;
 constexpr int TRIP = 4;         // iterations between checks for finished photons
+// The whole warp walks its photons one after another (warp_steps) once the
+// source has no more and at most this many are left.  A lane-loop iteration is
+// ~190 warp-instructions however few lanes walk, a photon's step by the whole
+// warp ~23, so 8 is where the issue slots break even.  4096-problem sweep at a
+// reduced scale: 788 ms without, 608 (6), 619 (10), 615 (16), 812 ms (24).
+constexpr int WARP_WALK_MAX = 8;
 
 // Where a walk keeps its tallies.  Warp: one shared histogram per warp.
 // Block: one per block, shared by its warps.  Global: none; every deposit is
@@ -136,7 +142,7 @@ struct GlobalSource {
     unsigned long long *counter;
     unsigned long long n;
     unsigned long long id_base;
-    unsigned chunk;   // at least 32: one claim serves every lane of the warp
+    unsigned chunk;   // below 32: lanes a claim leaves without a photon get none
     unsigned long long cnext = 0, cend = 0;
     bool exhausted = false;
 
@@ -264,6 +270,24 @@ struct Ring {
             p.blk += 2;
         }
     }
+
+    // Words of the photon's stream used so far, as whole blocks and a rest.
+    __device__ static __forceinline__ void position(const LanePhoton &p, uint32_t &block, uint32_t &rest)
+    {
+        const uint32_t words = (uint32_t)fill(p) / W;
+        block = p.blk - (words + 3) / 4;
+        rest = (0u - words) & 3u;
+    }
+    // Continue from a position with nothing buffered.
+    __device__ static __forceinline__ void restart(LanePhoton &p, uint32_t block, uint32_t rest, char *ring,
+                                                   const PhiloxKeys &keys)
+    {
+        const uint32_t even = block & ~1u;   // refills fill half a ring
+        p.blk = even;
+        p.cur = even * (4 * W);
+        refill(p, ring, keys);
+        p.cur += (4 * (block - even) + rest) * W;
+    }
 };
 
 // Photon launch, photon.c:12-18.
@@ -332,6 +356,211 @@ __device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, flo
     }
 }
 
+// ------------------------------------------------- one photon, whole warp
+// A photon's steps are a serial chain only through its position in the random
+// stream and the sums x += t u; everything else of a step follows from its
+// words.  With few photons left in a warp, all 32 lanes therefore walk ONE
+// photon, up to 32 steps at a time, in the same arithmetic and order:
+//
+//  * lane l computes Philox block l of the next 32 (128 words) and the
+//    outcome of a rejection try at each of its four word positions; ballots
+//    give, for a step starting at any position, where the next one starts;
+//  * lane k finds the k-th step's start by applying that map k times
+//    (doubling it by shuffles), then step k's length and new direction;
+//  * the sums run over the steps in order, x, y and z in a lane each and the
+//    repeatedly multiplied weight in a fourth: the only serial part;
+//  * radius and deposit are again one step per lane.  A roulette ends a round.
+//
+// A round is ~730 warp-instructions (exact arithmetic) for 32 steps, bound by
+// latency on an idle SM and by issue on a full one.  One high-albedo photon
+// (7168 steps): 2.31 ms on its lane, 0.30 ms here.  4099 of them, one to a warp
+// at a time: 4.2 -> 1.0 ms.
+struct WarpPhoton {   // the same in every lane
+    PhotonKey key;
+    uint32_t block, rest;   // words used: 4 block + rest
+    float x, y, z, u, v, w, weight;
+};
+
+// Scratch of the warp: four rows of 32 words, `stride` bytes apart.
+struct WarpScratch {
+    char *rows;
+    uint32_t stride;
+    __device__ __forceinline__ char *row(uint32_t r) const { return rows + r * stride; }
+    __device__ __forceinline__ uint32_t word(uint32_t p) const
+    {
+        return *reinterpret_cast<const uint32_t *>(rows + (p >> 5) * stride + (p & 31u) * 4);
+    }
+};
+
+// Where a step starting at word 127 would end: not within the round, like any
+// step whose successor is not below 127.  The map sends those to 127, which it
+// sends to itself, so looking a position up needs no bounds check.
+constexpr uint32_t NO_STEP = 127;
+
+// next[p], p < 128, of a map packed four positions to a lane.
+__device__ __forceinline__ uint32_t map_at(uint32_t packed, uint32_t p)
+{
+    return __byte_perm(__shfl_sync(FULL_MASK, packed, (int)(p >> 2)), 0u, 0x4440u | (p & 3u));
+}
+
+// Start of the step after one whose tries are bit 0 of c, then of d, then
+// bit 1 of c, ...: at_c / at_d is the position of the first try of either.
+__device__ __forceinline__ uint32_t after_try(uint32_t c, uint32_t d, uint32_t at_c, uint32_t at_d)
+{
+    const uint32_t any = c | d;
+    const uint32_t k = __ffs((int)any) - 1;
+    const uint32_t at = ((c >> (k & 31u)) & 1u) ? at_c : at_d;
+    return any ? min(at + 4 * k + 2, NO_STEP) : NO_STEP;
+}
+
+// Up to 32 steps of the photon.  deposit(mine, shell, weight) is called by
+// every lane (mine: this lane holds a step).  Returns the number of steps, 0 if
+// a step needs more words than a round has (the caller then walks it on one
+// lane); dead is set when the roulette ended the photon.
+template <class M>
+__device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const WarpScratch &sc, const WalkConsts &c,
+                                               const PhiloxKeys &keys, uint32_t &shell_out, float &weight_out)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint4 r = philox_block(p.block + lane, p.key, keys);
+    __syncwarp();   // the rows' earlier contents are read
+    *reinterpret_cast<uint4 *>(sc.row(lane >> 3) + (lane & 7u) * 16) = r;
+
+    // tries at this lane's four positions, then the map
+    const float f0 = uniform_pm1(r.x), f1 = uniform_pm1(r.y), f2 = uniform_pm1(r.z), f3 = uniform_pm1(r.w);
+    const float f4 = __shfl_down_sync(FULL_MASK, f0, 1);
+    const uint32_t a0 = __ballot_sync(FULL_MASK, !(1.0f < M::norm2(f0, f1)));
+    const uint32_t a1 = __ballot_sync(FULL_MASK, !(1.0f < M::norm2(f1, f2)));
+    const uint32_t a2 = __ballot_sync(FULL_MASK, !(1.0f < M::norm2(f2, f3)));
+    const uint32_t a3 = __ballot_sync(FULL_MASK, lane < 31u && !(1.0f < M::norm2(f3, f4)));
+    const uint32_t b0 = a0 >> lane, b1 = a1 >> lane, b2 = a2 >> lane, b3 = a3 >> lane;
+    const uint32_t at = 4 * lane;
+    uint32_t map = after_try(b1, b3, at + 1, at + 3);                 // step at 4l: tries at 4l+1, 4l+3, ...
+    map |= after_try(b2, b0 >> 1, at + 2, at + 4) << 8;
+    map |= after_try(b3, b1 >> 1, at + 3, at + 5) << 16;
+    map |= after_try(b0 >> 1, b2 >> 1, at + 4, at + 6) << 24;
+
+    // step `lane` starts at the lane-fold image of the first step's start
+    uint32_t start = p.rest, power = map;
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+        const uint32_t to = map_at(power, start);
+        if ((lane >> b) & 1u)
+            start = to;
+        if (b < 4) {
+            const uint32_t q0 = map_at(power, power & 255u), q1 = map_at(power, (power >> 8) & 255u);
+            const uint32_t q2 = map_at(power, (power >> 16) & 255u), q3 = map_at(power, power >> 24);
+            power = __byte_perm(__byte_perm(q0, q1, 0x0040u), __byte_perm(q2, q3, 0x0040u), 0x5410u);
+        }
+    }
+    const uint32_t next = map_at(map, start);
+    const bool whole = next != NO_STEP;
+    uint32_t n = __popc(__ballot_sync(FULL_MASK, whole));   // a prefix of the lanes
+    if (n == 0)
+        return 0;
+
+    // step length, new direction
+    __syncwarp();
+    const float t = M::step_length(uniform01(sc.word(start)));
+    const float xi1 = uniform_pm1(sc.word(next - 2)), xi2 = uniform_pm1(sc.word(next - 1));
+    float nu, nv, nw;
+    M::direction(M::norm2(xi1, xi2), xi1, xi2, nu, nv, nw);
+    float u = __shfl_up_sync(FULL_MASK, nu, 1), v = __shfl_up_sync(FULL_MASK, nv, 1);
+    float w = __shfl_up_sync(FULL_MASK, nw, 1);
+    if (lane == 0) {
+        u = p.u;
+        v = p.v;
+        w = p.w;
+    }
+    __syncwarp();
+    reinterpret_cast<float *>(sc.row(0))[lane] = t;
+    reinterpret_cast<float *>(sc.row(1))[lane] = u;
+    reinterpret_cast<float *>(sc.row(2))[lane] = v;
+    reinterpret_cast<float *>(sc.row(3))[lane] = w;
+    __syncwarp();
+
+    // the moves in order: lanes 0..2 sum x, y and z, lane 3 decays the weight,
+    // and leave what step j deposits with in word j of the rows (weight in 0)
+    float sum = lane == 0 ? p.x : lane == 1 ? p.y : p.z, decay = p.weight;
+    float *const along = reinterpret_cast<float *>(sc.row(min(lane + 1, 3u)));
+    float *const out = lane == 3 ? reinterpret_cast<float *>(sc.row(0)) : along;
+    const float *const lengths = reinterpret_cast<const float *>(sc.row(0));
+#pragma unroll 2
+    for (uint32_t j = 0; j < 32; j += 4) {
+        const float4 t4 = *reinterpret_cast<const float4 *>(lengths + j);
+        const float4 d4 = *reinterpret_cast<const float4 *>(along + j);
+        float4 r4;
+        r4.x = sum = M::move(sum, t4.x, d4.x);
+        r4.y = sum = M::move(sum, t4.y, d4.y);
+        r4.z = sum = M::move(sum, t4.z, d4.z);
+        r4.w = sum = M::move(sum, t4.w, d4.w);
+        const float w1 = M::mul(decay, c.albedo), w2 = M::mul(w1, c.albedo), w3 = M::mul(w2, c.albedo);
+        if (lane == 3)
+            r4 = make_float4(decay, w1, w2, w3);
+        decay = M::mul(w3, c.albedo);
+        __syncwarp();
+        if (lane < 4)
+            *reinterpret_cast<float4 *>(out + j) = r4;
+    }
+    __syncwarp();
+    const float weight = reinterpret_cast<const float *>(sc.row(0))[lane];
+    const float x = reinterpret_cast<const float *>(sc.row(1))[lane];
+    const float y = reinterpret_cast<const float *>(sc.row(2))[lane];
+    const float z = reinterpret_cast<const float *>(sc.row(3))[lane];
+    const float decayed = M::mul(weight, c.albedo);
+    const uint32_t low = __ballot_sync(FULL_MASK, whole && decayed < 0.001f * WEIGHT_ONE);
+    if (low)
+        n = __ffs((int)low);   // the steps up to the first roulette
+    shell_out = __float2uint_rz(fminf(M::radius_shells(x, y, z, c.spm), c.last));
+    weight_out = weight;
+
+    const int l = (int)n - 1;
+    p.x = __shfl_sync(FULL_MASK, x, l);
+    p.y = __shfl_sync(FULL_MASK, y, l);
+    p.z = __shfl_sync(FULL_MASK, z, l);
+    p.u = __shfl_sync(FULL_MASK, nu, l);
+    p.v = __shfl_sync(FULL_MASK, nv, l);
+    p.w = __shfl_sync(FULL_MASK, nw, l);
+    p.weight = __shfl_sync(FULL_MASK, decayed, l);
+    uint32_t to = __shfl_sync(FULL_MASK, next, l);
+    dead = false;
+    if (low) {
+        // roulette, photon.c:45-49; its word may lie behind the round's
+        const uint4 q = philox_block(p.block + (to >> 2), p.key, keys);
+        const uint32_t i = to & 3u;
+        const float U = uniform01(i == 0u ? q.x : i == 1u ? q.y : i == 2u ? q.z : q.w);
+        ++to;
+        dead = U > 0.1f;
+        p.weight = __fdiv_rn(p.weight, 0.1f);
+    }
+    p.block += to >> 2;
+    p.rest = to & 3u;
+    return n;
+}
+
+// The photon of lane `l`, in every lane.
+template <int BLOCK>
+__device__ __forceinline__ WarpPhoton broadcast_photon(const LanePhoton &p, int l)
+{
+    WarpPhoton q;
+    uint32_t block, rest;
+    Ring<BLOCK>::position(p, block, rest);
+    q.key.a = __shfl_sync(FULL_MASK, p.key.a, l);
+    q.key.b = __shfl_sync(FULL_MASK, p.key.b, l);
+    q.key.c = __shfl_sync(FULL_MASK, p.key.c, l);
+    q.key.d = __shfl_sync(FULL_MASK, p.key.d, l);
+    q.block = __shfl_sync(FULL_MASK, block, l);
+    q.rest = __shfl_sync(FULL_MASK, rest, l);
+    q.x = __shfl_sync(FULL_MASK, p.x, l);
+    q.y = __shfl_sync(FULL_MASK, p.y, l);
+    q.z = __shfl_sync(FULL_MASK, p.z, l);
+    q.u = __shfl_sync(FULL_MASK, p.u, l);
+    q.v = __shfl_sync(FULL_MASK, p.v, l);
+    q.w = __shfl_sync(FULL_MASK, p.w, l);
+    q.weight = __shfl_sync(FULL_MASK, p.weight, l);
+    return q;
+}
+
 // Walk photons from `src` until it is exhausted and every lane's photon has
 // died.  Warp-collective: all 32 lanes of every warp call it.  tally: the
 // shared histogram (H = Warp: this warp's; Block: the block's), 4 * shells
@@ -361,6 +590,23 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
     uint32_t steps = 0, trips = 0;
     unsigned idle = 0;   // lanes that get no more photons
 
+    auto deposit = [&](uint32_t shell, float weight) {
+        uint32_t lo, hi;
+        if constexpr (H == Hist::Global) {
+            unsigned long long *gs = g + 4 * (size_t)shell;
+            units_split(weight_units(weight), lo, hi);
+            flush128(&gs[0], &gs[1], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
+            units_split(weight2_units(weight), lo, hi);
+            flush128(&gs[2], &gs[3], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
+        } else {
+            const uint32_t at = hist + 4 * shell;
+            units_split(weight_units(weight), lo, hi);
+            tally_add_nowrap(at, at + 4 * S, lo, hi);
+            units_split(weight2_units(weight), lo, hi);
+            tally_add_nowrap(at + 8 * S, at + 12 * S, lo, hi);
+        }
+        ++steps;
+    };
     for (;;) {
         // -------- hand new photon ids to lanes whose photon died
         const unsigned dead = __ballot_sync(FULL_MASK, !R::walking(p));
@@ -374,8 +620,50 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
             if (idle == FULL_MASK)
                 break;
         }
+        // -------- few photons left: the whole warp walks them one by one
+        if (idle && 32 - __popc(idle) <= WARP_WALK_MAX) {
+            // a photon whose direction is still sought waits for the lane loop
+            unsigned todo = __ballot_sync(FULL_MASK, R::walking(p) && !(p.t > 1.0f));
+            const WarpScratch sc{ring - 4 * lane, R::W};
+            while (todo && trips < FLUSH_TRIPS - 1) {
+                const int l = __ffs((int)todo) - 1;
+                todo &= todo - 1;
+                WarpPhoton q = broadcast_photon<BLOCK>(p, l);
+                bool over = false;
+                uint32_t n;
+                do {
+                    uint32_t shell;
+                    float weight;
+                    n = warp_steps<M>(q, over, sc, c, keys, shell, weight);
+                    if (lane < n)
+                        deposit(shell, weight);
+                    if constexpr (H != Hist::Global)
+                        ++trips;
+                } while (n && !over && trips < FLUSH_TRIPS - 1);
+                if ((int)lane == l) {
+                    if (over) {
+                        R::drop(p);
+                    } else {   // a flush is due, or a step took over 124 words: back to its lane
+                        p.x = q.x; p.y = q.y; p.z = q.z;
+                        p.u = q.u; p.v = q.v; p.w = q.w;
+                        p.weight = q.weight;
+                        p.blk = q.block + 4;   // position() below: 16 - rest words left
+                        p.cur = q.block * (4 * R::W) + q.rest * R::W;
+                    }
+                }
+            }
+            // the rings were scratch: refill those still in use
+            __syncwarp();
+            if (R::walking(p)) {
+                uint32_t block, rest;
+                R::position(p, block, rest);
+                R::restart(p, block, rest, ring, keys);
+            }
+            if (__any_sync(FULL_MASK, !R::walking(p) && !((idle >> lane) & 1u)))
+                continue;
+        }
         if constexpr (H != Hist::Global) {
-            if (++trips == FLUSH_TRIPS) {
+            if (++trips >= FLUSH_TRIPS) {   // TRIP deposits of a lane at most since the last count
                 trips = 0;
                 if constexpr (H == Hist::Warp)
                     warp_flush_tally(tally, S, g);
@@ -387,26 +675,7 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
         for (int k = 0; k < TRIP; ++k) {
             if (k % 2 == 0)
                 R::refill(p, ring, keys);
-            step_photon<BLOCK, M>(
-                p, ring, c.spm, c.last, c.albedo,
-                [&](uint32_t shell, float weight) {
-                    uint32_t lo, hi;
-                    if constexpr (H == Hist::Global) {
-                        unsigned long long *gs = g + 4 * (size_t)shell;
-                        units_split(weight_units(weight), lo, hi);
-                        flush128(&gs[0], &gs[1], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
-                        units_split(weight2_units(weight), lo, hi);
-                        flush128(&gs[2], &gs[3], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
-                    } else {
-                        const uint32_t at = hist + 4 * shell;
-                        units_split(weight_units(weight), lo, hi);
-                        tally_add_nowrap(at, at + 4 * S, lo, hi);
-                        units_split(weight2_units(weight), lo, hi);
-                        tally_add_nowrap(at + 8 * S, at + 12 * S, lo, hi);
-                    }
-                    ++steps;
-                },
-                [] {});
+            step_photon<BLOCK, M>(p, ring, c.spm, c.last, c.albedo, deposit, [] {});
         }
     }
     return steps;
