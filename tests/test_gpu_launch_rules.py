@@ -69,3 +69,29 @@ def test_whole_warp_walk_equals_lane_walk(tmc_mod, optics, math):
     assert both[1] - before[1] == few_steps
     diff = [tuple(x - y for x, y in zip(a, b)) for a, b in zip(ints(both[0]), ints(before[0]))]
     assert diff == ints(few)
+
+
+@pytest.mark.parametrize("shells", [1, 2, 31, 33, 130])
+def test_last_shell_cells(tmc_mod, oracle_mod, shells):
+    """An optically thin medium, nearly every deposit in the last shell: its
+    per-lane cells add up to the oracle's tallies in the plain and batched forms
+    (probe shell included: a served request's error is checked elsewhere)."""
+    from test_gpu_parity import as_array
+    from tiny_mc_gb300.sweep import PROBLEM_DTYPE
+    optics = dict(shells=shells, microns_per_shell=10.0, mu_a=1.0, mu_s=4.0)
+    n = 20011
+    tmc_mod.set_plain_launch(0, 0, 0)
+    ref, _, ref_steps = oracle_fx(oracle_mod, n, seed=9, **optics)
+    got, steps = gpu_fx(tmc_mod, n, seed=9, **optics)
+    assert steps == ref_steps and np.array_equal(got, ref)
+    pr = np.zeros(1, PROBLEM_DTYPE)
+    for k, v in optics.items():
+        pr[k] = v
+    pr["n_photons"] = n
+    for block, stream in ((128, False), (512, False), (128, True), (256, True)):
+        b = tmc_mod.Batch(pr, seed=9, math="exact")
+        b.set_config(block, 8, False, stream)
+        b.run()
+        t, s = b.read()
+        b.close()
+        assert int(s[0]) == ref_steps and np.array_equal(as_array(t), ref), (block, stream)

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(BLOCK) walk_batch(const BatchArgs a)
     __shared__ BatchItemDev sh_itm;
     __shared__ BatchProblemDev sh_pr;
     __shared__ unsigned long long sh_qidx;
-    uint32_t *my = smem + 4 * a.max_shells + threadIdx.x;
+    uint32_t *my = smem + 4 * hist_cells(a.max_shells) + threadIdx.x;
     if (QUEUE && threadIdx.x == 0 && a.q_live)
         atomicAdd(a.q_live, 1u);
 
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(BLOCK) walk_batch(const BatchArgs a)
         const BatchItemDev item = QUEUE ? sh_itm : a.items[it];
         const BatchProblemDev pr = QUEUE ? sh_pr : a.problems[item.problem];
         const uint32_t S = pr.c.shells;
-        for (uint32_t s = threadIdx.x; s < 4 * S; s += BLOCK)
+        for (uint32_t s = threadIdx.x; s < 4 * hist_cells(S); s += BLOCK)
             smem[s] = 0;
         __syncthreads();
 
@@ -108,9 +108,13 @@ __global__ void __launch_bounds__(BLOCK) walk_batch(const BatchArgs a)
         flush_tally<BLOCK>(smem, S, g);
         // this item's own sum of w in the probe shell, 128-bit: what the
         // walk's flushes took from the shell plus what is left in it
-        const unsigned long long rest = ((unsigned long long)smem[S + ps] << 32) | smem[ps];
-        const unsigned long long probe_lo = sh_probe_acc + rest;
-        const uint32_t probe_hi = sh_probe_hi + (probe_lo < rest ? 1u : 0u);
+        unsigned long long probe_lo = 0;
+        uint32_t probe_hi = 0;
+        if (probe && threadIdx.x < 32) {
+            const unsigned long long rest = shell_sum(smem, S, ps);
+            probe_lo = sh_probe_acc + rest;
+            probe_hi = sh_probe_hi + (probe_lo < rest ? 1u : 0u);
+        }
         if (a.item_probe && threadIdx.x == 0) {
             a.item_probe[2 * (size_t)it] = probe_lo;
             a.item_probe[2 * (size_t)it + 1] = probe_hi;
@@ -151,7 +155,7 @@ static cudaError_t walk_batch_config(int sms, size_t smem, int *grid)
 
 size_t walk_batch_smem(uint32_t max_shells, int block)
 {
-    return (size_t)16 * max_shells + (size_t)4 * SLOTS * block;
+    return (size_t)16 * hist_cells(max_shells) + (size_t)4 * SLOTS * block;
 }
 
 template <bool QUEUE>

@@ -62,8 +62,9 @@ __global__ void __launch_bounds__(BLOCK) walk_plain(const PlainArgs a)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     constexpr bool PER_WARP = H == Hist::Warp;
-    const uint32_t S = H == Hist::Global ? 0u : a.c.shells;   // words per histogram / 4
-    const uint32_t words = (PER_WARP ? BLOCK / 32 : 1) * 4 * S;
+    const uint32_t S = a.c.shells;
+    const uint32_t hist = H == Hist::Global ? 0u : 4 * hist_cells(S);   // words per histogram
+    const uint32_t words = (PER_WARP ? BLOCK / 32 : 1) * hist;
     for (uint32_t s = threadIdx.x; s < words; s += BLOCK)
         smem[s] = 0;
     __syncthreads();
@@ -74,12 +75,12 @@ __global__ void __launch_bounds__(BLOCK) walk_plain(const PlainArgs a)
     src.id_base = a.id_base;
     src.chunk = a.chunk;
     uint32_t *my = smem + words + threadIdx.x;   // ring slot k: my[k * BLOCK]
-    uint32_t *tally = PER_WARP ? smem + (threadIdx.x / 32) * 4 * S : smem;
+    uint32_t *tally = PER_WARP ? smem + (threadIdx.x / 32) * hist : smem;
     const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H>(
         a.c, src, a.keys, tally, a.tally, my);
 
     if constexpr (PER_WARP) {
-        warp_flush_tally(tally, S, a.tally);
+        warp_flush_tally<false>(tally, S, a.tally);
     } else if constexpr (H == Hist::Block) {
         __syncthreads();
         flush_tally<BLOCK>(smem, S, a.tally);
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(BLOCK) walk_plain(const PlainArgs a)
 
 static size_t plain_smem_bytes(uint32_t shells, int block, Hist h)
 {
-    const size_t hist = h == Hist::Global ? 0 : (size_t)16 * shells * (h == Hist::Warp ? block / 32 : 1);
+    const size_t hist = h == Hist::Global ? 0 : (size_t)16 * hist_cells(shells) * (h == Hist::Warp ? block / 32 : 1);
     return hist + (size_t)4 * SLOTS * block;
 }
 

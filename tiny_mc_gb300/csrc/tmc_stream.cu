@@ -45,6 +45,13 @@ namespace tmc {
 namespace {
 
 constexpr uint32_t END_ITEM = 0xffffffffu;
+
+// Extra cells of the last shell: LAST_CELLS - 1 where both histograms and the
+// rings then fit the 227 KB a block can have (less the kernel's own record).
+__host__ __device__ constexpr uint32_t stream_spread(uint32_t max_shells, int block)
+{
+    return 32ull * hist_cells(max_shells) + 4ull * SLOTS * block <= 232448 - 512 ? LAST_CELLS - 1 : 0;
+}
 constexpr unsigned long long DEFAULT_WAIT_LIMIT_NS = QUEUE_DEFAULT_WAIT_LIMIT_NS;
 constexpr uint32_t BUF_FREE = 0, BUF_CLAIMING = 1, BUF_OPEN = 2;
 
@@ -129,7 +136,10 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
     constexpr unsigned NWARPS = BLOCK / 32;
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ OpenItem open[2];
-    const uint32_t HS = 4 * a.max_shells;          // words per histogram
+    // last shell's cells: one per lane (as hist_cells), or one where the two
+    // histograms would not fit in shared memory otherwise
+    const uint32_t spread = stream_spread(a.max_shells, BLOCK);
+    const uint32_t HS = 4 * (a.max_shells + spread);   // words per histogram
     uint32_t *my = smem + 2 * HS + threadIdx.x;    // ring slot k: my[k * BLOCK]
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -198,18 +208,22 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
                 // every warp is done with item `rep`: flush, probe, reset, free
                 __threadfence_block();
                 const uint32_t it = vopen[rb].item;
-                const uint32_t S = vopen[rb].c.shells;
+                const uint32_t S = vopen[rb].c.shells, C = S + spread;
                 uint32_t *hist = smem + rb * HS;
                 unsigned long long *gg = open[rb].g;
-                for (uint32_t s = lane; s < S; s += 32) {
-                    flush128(&gg[4 * s + 0], &gg[4 * s + 1],
-                             ((unsigned long long)hist[S + s] << 32) | hist[s]);
-                    flush128(&gg[4 * s + 2], &gg[4 * s + 3],
-                             ((unsigned long long)hist[3 * S + s] << 32) | hist[2 * S + s]);
-                }
                 const uint32_t p = vopen[rb].ps;
-                const unsigned long long probe_lo = ((unsigned long long)hist[S + p] << 32) | hist[p];
-                const unsigned long long probe_hi = vopen[rb].wraps;
+                unsigned long long probe_lo = 0, probe_hi = vopen[rb].wraps;
+                for (uint32_t s = lane; s < C; s += 32) {
+                    unsigned long long *gs = gg + 4 * (size_t)min(s, S - 1);
+                    flush128(&gs[0], &gs[1], ((unsigned long long)hist[C + s] << 32) | hist[s]);
+                    flush128(&gs[2], &gs[3], ((unsigned long long)hist[3 * C + s] << 32) | hist[2 * C + s]);
+                }
+                // the probe shell's sum: one cell, or all of the last shell's
+                for (uint32_t s = p; s < (p == S - 1 ? C : p + 1); ++s) {
+                    const unsigned long long v = ((unsigned long long)hist[C + s] << 32) | hist[s];
+                    probe_lo += v;
+                    probe_hi += probe_lo < v ? 1u : 0u;
+                }
                 if (lane == 0) {
                     const unsigned long long st =
                         ((unsigned long long)vopen[rb].steps_hi << 32) | vopen[rb].steps_lo;
@@ -231,7 +245,7 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
                     }
                 }
                 __syncwarp();
-                for (uint32_t s = lane; s < 4 * S; s += 32)
+                for (uint32_t s = lane; s < 4 * C; s += 32)
                     hist[s] = 0;
                 __threadfence_block();
                 __syncwarp();
@@ -343,16 +357,17 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
             if (k % 2 == 0)
                 R::refill(p, ring, a.keys);
             step_photon<BLOCK, M>(
-                p, ring, pc.spm, pc.last, pc.albedo,
-                [&](uint32_t shell, float weight) {
-                    const uint32_t S = pc.shells;
-                    uint32_t *t0 = hist + shell;
+                p, ring, pc.spm, pc.last, pc.last + (float)(lane & spread), pc.albedo,
+                [&](uint32_t cell, float weight) {
+                    const uint32_t C = pc.shells + spread;
+                    const uint32_t shell = min(cell, pc.shells - 1);
+                    uint32_t *t0 = hist + cell;
                     uint32_t lo, hi;
                     units_split(weight_units(weight), lo, hi);
-                    tally_add(t0, t0 + S, &pg[4 * shell + 1], lo, hi,
+                    tally_add(t0, t0 + C, &pg[4 * shell + 1], lo, hi,
                               shell == pps ? (uint32_t *)&open[lb].wraps : nullptr);
                     units_split(weight2_units(weight), lo, hi);
-                    tally_add(t0 + 2 * S, t0 + 3 * S, &pg[4 * shell + 3], lo, hi);
+                    tally_add(t0 + 2 * C, t0 + 3 * C, &pg[4 * shell + 3], lo, hi);
                     ++steps;
                 },
                 [&] {
@@ -373,7 +388,7 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
 
 size_t walk_stream_smem(uint32_t max_shells, int block)
 {
-    return (size_t)32 * max_shells + (size_t)4 * SLOTS * block;
+    return (size_t)32 * (max_shells + stream_spread(max_shells, block)) + (size_t)4 * SLOTS * block;
 }
 
 template <int BLOCK, class M, bool QUEUE>

@@ -82,49 +82,75 @@ __host__ __device__ constexpr uint32_t flush_steps(uint32_t lanes)
 static_assert(512ull * 257ull * ((1ull << 23) / 512 + 1) < (1ull << 32), "high word bound");
 static_assert(32ull * 257ull * ((1ull << 23) / 32 + 1) < (1ull << 32), "high word bound");
 
-// Add a warp's own histogram (4 * S words) into the 128-bit global tally and
-// clear it.  Warp-collective.
-__device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g)
+// Cells of a shared histogram.  Every photon beyond the last shell deposits
+// into it (photon.c:27-29): in an optically thin problem nearly all lanes of a
+// warp at once, and shared atomics on one word take their turns.  So the last
+// shell has 32 cells, one per lane, which the flushes add up.  2^20 high-albedo
+// photons (1001 shells of 10 um, many walks leave): 46.8 -> 44.8 ms; the reduced
+// 4096-problem sweep 609 -> 555 ms.
+constexpr uint32_t LAST_CELLS = 32;
+__host__ __device__ constexpr uint32_t hist_cells(uint32_t shells) { return shells + LAST_CELLS - 1; }
+
+// Take the 64-bit sum of cell s: `clear` by plain loads and stores, else by
+// atomic exchanges against zero while other warps deposit.
+template <bool EXCHANGE>
+__device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *hi)
 {
-    __syncwarp();
-    for (uint32_t s = threadIdx.x & 31u; s < S; s += 32) {
-        flush128(&g[4 * s + 0], &g[4 * s + 1], ((unsigned long long)tally[S + s] << 32) | tally[s]);
-        flush128(&g[4 * s + 2], &g[4 * s + 3],
-                 ((unsigned long long)tally[3 * S + s] << 32) | tally[2 * S + s]);
-        tally[s] = 0;
-        tally[S + s] = 0;
-        tally[2 * S + s] = 0;
-        tally[3 * S + s] = 0;
+    uint32_t l, h;
+    if constexpr (EXCHANGE) {
+        l = atomicExch(lo, 0u);
+        h = atomicExch(hi, 0u);
+    } else {
+        l = *lo;
+        h = *hi;
+        *lo = 0;
+        *hi = 0;
     }
-    __syncwarp();
+    return ((unsigned long long)h << 32) | l;
 }
 
-// Add a block's histogram into the 128-bit global tally and clear it, by one
+// Add a histogram into the 128-bit global tally and clear it.
+// EXCHANGE = false: a warp's own histogram.  EXCHANGE = true: a block's, by one
 // warp while the others keep depositing: every word is taken with an atomic
 // exchange against zero.  Sums stay exact: a deposit's low-word overflow is
 // carried into a high word by the depositing lane, whichever side of an
 // exchange either add lands on, and every word's content reaches the global
 // tally at one flush or the next.  probe_acc / probe_hi (shared, may be
 // null): the 128-bit running sum of the w words taken from shell
-// probe_shell.  Warp-collective.
-__device__ __forceinline__ void swap_flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g,
-                                                 unsigned long long *probe_acc, uint32_t *probe_hi,
-                                                 uint32_t probe_shell)
+// probe_shell.  Warp-collective.  The last shell's cells are added up first
+// (their total obeys the bound below, so it fits 64 bits).
+template <bool EXCHANGE>
+__device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g,
+                                                 unsigned long long *probe_acc = nullptr,
+                                                 uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
 {
-    for (uint32_t s = threadIdx.x & 31u; s < S; s += 32) {
-        const uint32_t lo = atomicExch(&tally[s], 0u);
-        const uint32_t hi = atomicExch(&tally[S + s], 0u);
-        const unsigned long long v = ((unsigned long long)hi << 32) | lo;
+    const uint32_t C = hist_cells(S), lane = threadIdx.x & 31u;
+    __syncwarp();
+    for (uint32_t s = lane; s < S - 1; s += 32) {
+        const unsigned long long v = take_cell<EXCHANGE>(&tally[s], &tally[C + s]);
         flush128(&g[4 * s + 0], &g[4 * s + 1], v);
-        if (probe_acc && s == probe_shell && v) {
+        if (EXCHANGE && probe_acc && s == probe_shell && v) {
             const unsigned long long old = atomicAdd(probe_acc, v);
             if (old + v < old)
                 atomicAdd(probe_hi, 1u);
         }
-        const uint32_t lo2 = atomicExch(&tally[2 * S + s], 0u);
-        const uint32_t hi2 = atomicExch(&tally[3 * S + s], 0u);
-        flush128(&g[4 * s + 2], &g[4 * s + 3], ((unsigned long long)hi2 << 32) | lo2);
+        flush128(&g[4 * s + 2], &g[4 * s + 3], take_cell<EXCHANGE>(&tally[2 * C + s], &tally[3 * C + s]));
     }
+    __syncwarp();
+    const uint32_t s = S - 1 + lane;
+    const unsigned long long v = warp_sum_u64(take_cell<EXCHANGE>(&tally[s], &tally[C + s]));
+    const unsigned long long v2 = warp_sum_u64(take_cell<EXCHANGE>(&tally[2 * C + s], &tally[3 * C + s]));
+    if (lane == 0) {
+        unsigned long long *gl = g + 4 * (size_t)(S - 1);
+        flush128(&gl[0], &gl[1], v);
+        if (EXCHANGE && probe_acc && S - 1 == probe_shell && v) {
+            const unsigned long long old = atomicAdd(probe_acc, v);
+            if (old + v < old)
+                atomicAdd(probe_hi, 1u);
+        }
+        flush128(&gl[2], &gl[3], v2);
+    }
+    __syncwarp();
 }
 
 // Per-problem constants of photon.c:8-9 (computed on the host in float,
@@ -307,10 +333,12 @@ __device__ __forceinline__ void launch_photon(LanePhoton &p, unsigned long long 
 // One iteration of a lane's photon if six words are buffered (else it waits
 // for the next refill): move, deposit and decay unless its direction is still
 // sought, then two tries for the next direction and the roulette.
-// deposit(shell, weight) tallies a step, died() is called at the photon's end.
+// deposit(cell, weight) tallies a step, died() is called at the photon's end.
+// A radius below `last` shells goes to its shell's cell, any other (NaN too) to
+// cell `beyond`.
 template <int BLOCK, class M, class Deposit, class Died>
-__device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, float spm, float last, float albedo,
-                                            Deposit deposit, Died died)
+__device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, float spm, float last, float beyond,
+                                            float albedo, Deposit deposit, Died died)
 {
     using R = Ring<BLOCK>;
     if (R::fill(p) < (int)(6 * R::W))
@@ -326,8 +354,9 @@ __device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, flo
         p.y = M::move(p.y, t, p.v);
         p.z = M::move(p.z, t, p.w);
         // absorb, photon.c:26-32 (clamp in float: same shell for every radius
-        // below 2^32 shells, and a NaN radius lands last)
-        deposit(__float2uint_rz(fminf(M::radius_shells(p.x, p.y, p.z, spm), last)), p.weight);
+        // below 2^32 shells)
+        const float r = M::radius_shells(p.x, p.y, p.z, spm);
+        deposit(__float2uint_rz(r < last ? r : beyond), p.weight);
         p.weight = M::mul(p.weight, albedo);
     }
     // the next two tries of the rejection method, photon.c:36-40; the second
@@ -419,7 +448,8 @@ __device__ __forceinline__ uint32_t after_try(uint32_t c, uint32_t d, uint32_t a
 // lane); dead is set when the roulette ended the photon.
 template <class M>
 __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const WarpScratch &sc, const WalkConsts &c,
-                                               const PhiloxKeys &keys, uint32_t &shell_out, float &weight_out)
+                                               const PhiloxKeys &keys, float beyond, uint32_t &cell_out,
+                                               float &weight_out)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uint4 r = philox_block(p.block + lane, p.key, keys);
@@ -511,7 +541,8 @@ __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const 
     const uint32_t low = __ballot_sync(FULL_MASK, whole && decayed < 0.001f * WEIGHT_ONE);
     if (low)
         n = __ffs((int)low);   // the steps up to the first roulette
-    shell_out = __float2uint_rz(fminf(M::radius_shells(x, y, z, c.spm), c.last));
+    const float radius = M::radius_shells(x, y, z, c.spm);
+    cell_out = __float2uint_rz(radius < c.last ? radius : beyond);
     weight_out = weight;
 
     const int l = (int)n - 1;
@@ -563,7 +594,7 @@ __device__ __forceinline__ WarpPhoton broadcast_photon(const LanePhoton &p, int 
 
 // Walk photons from `src` until it is exhausted and every lane's photon has
 // died.  Warp-collective: all 32 lanes of every warp call it.  tally: the
-// shared histogram (H = Warp: this warp's; Block: the block's), 4 * shells
+// shared histogram (H = Warp: this warp's; Block: the block's), 4 * hist_cells
 // words (low and high of sum w, then of sum w^2), flushed into g, the
 // problem's global 128-bit tally [shells][4], every flush_steps iterations;
 // the caller flushes what is left.  probe_acc / probe_hi (Block only, may be
@@ -590,20 +621,23 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
     uint32_t steps = 0, trips = 0;
     unsigned idle = 0;   // lanes that get no more photons
 
-    auto deposit = [&](uint32_t shell, float weight) {
+    const float beyond = H == Hist::Global ? c.last : c.last + (float)lane;
+    const uint32_t plane = 4 * hist_cells(S);   // bytes between a cell's words
+
+    auto deposit = [&](uint32_t cell, float weight) {
         uint32_t lo, hi;
         if constexpr (H == Hist::Global) {
-            unsigned long long *gs = g + 4 * (size_t)shell;
+            unsigned long long *gs = g + 4 * (size_t)cell;
             units_split(weight_units(weight), lo, hi);
             flush128(&gs[0], &gs[1], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
             units_split(weight2_units(weight), lo, hi);
             flush128(&gs[2], &gs[3], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
         } else {
-            const uint32_t at = hist + 4 * shell;
+            const uint32_t at = hist + 4 * cell;
             units_split(weight_units(weight), lo, hi);
-            tally_add_nowrap(at, at + 4 * S, lo, hi);
+            tally_add_nowrap(at, at + plane, lo, hi);
             units_split(weight2_units(weight), lo, hi);
-            tally_add_nowrap(at + 8 * S, at + 12 * S, lo, hi);
+            tally_add_nowrap(at + 2 * plane, at + 3 * plane, lo, hi);
         }
         ++steps;
     };
@@ -632,11 +666,11 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                 bool over = false;
                 uint32_t n;
                 do {
-                    uint32_t shell;
+                    uint32_t cell;
                     float weight;
-                    n = warp_steps<M>(q, over, sc, c, keys, shell, weight);
+                    n = warp_steps<M>(q, over, sc, c, keys, beyond, cell, weight);
                     if (lane < n)
-                        deposit(shell, weight);
+                        deposit(cell, weight);
                     if constexpr (H != Hist::Global)
                         ++trips;
                 } while (n && !over && trips < FLUSH_TRIPS - 1);
@@ -665,32 +699,49 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
         if constexpr (H != Hist::Global) {
             if (++trips >= FLUSH_TRIPS) {   // TRIP deposits of a lane at most since the last count
                 trips = 0;
-                if constexpr (H == Hist::Warp)
-                    warp_flush_tally(tally, S, g);
-                else
-                    swap_flush_tally(tally, S, g, probe_acc, probe_hi, probe_shell);
+                warp_flush_tally<H == Hist::Block>(tally, S, g, probe_acc, probe_hi, probe_shell);
             }
         }
 #pragma unroll
         for (int k = 0; k < TRIP; ++k) {
             if (k % 2 == 0)
                 R::refill(p, ring, keys);
-            step_photon<BLOCK, M>(p, ring, c.spm, c.last, c.albedo, deposit, [] {});
+            step_photon<BLOCK, M>(p, ring, c.spm, c.last, beyond, c.albedo, deposit, [] {});
         }
     }
     return steps;
 }
 
-// Add a block's shared histogram (4 * shells words) into a 128-bit global
-// tally [shells][4].  Block-collective, after a barrier.
+// Add what is left in a block's histogram to a 128-bit global tally
+// [shells][4], after a barrier.  Block-collective.
 template <int BLOCK>
-__device__ __forceinline__ void flush_tally(const uint32_t *tally, uint32_t S, unsigned long long *g)
+__device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g)
 {
-    for (uint32_t s = threadIdx.x; s < S; s += BLOCK) {
-        flush128(&g[4 * s + 0], &g[4 * s + 1], ((unsigned long long)tally[S + s] << 32) | tally[s]);
-        flush128(&g[4 * s + 2], &g[4 * s + 3],
-                 ((unsigned long long)tally[3 * S + s] << 32) | tally[2 * S + s]);
+    const uint32_t C = hist_cells(S);
+    for (uint32_t s = threadIdx.x; s < S - 1; s += BLOCK) {
+        flush128(&g[4 * s + 0], &g[4 * s + 1], ((unsigned long long)tally[C + s] << 32) | tally[s]);
+        flush128(&g[4 * s + 2], &g[4 * s + 3], ((unsigned long long)tally[3 * C + s] << 32) | tally[2 * C + s]);
     }
+    if (threadIdx.x < 32) {
+        const uint32_t s = S - 1 + threadIdx.x;
+        const unsigned long long v = warp_sum_u64(((unsigned long long)tally[C + s] << 32) | tally[s]);
+        const unsigned long long v2 = warp_sum_u64(((unsigned long long)tally[3 * C + s] << 32) | tally[2 * C + s]);
+        if (threadIdx.x == 0) {
+            flush128(&g[4 * (size_t)(S - 1) + 0], &g[4 * (size_t)(S - 1) + 1], v);
+            flush128(&g[4 * (size_t)(S - 1) + 2], &g[4 * (size_t)(S - 1) + 3], v2);
+        }
+    }
+}
+
+// The 64-bit sum of w that a block's histogram holds for shell s.  Called by
+// the first warp.
+__device__ __forceinline__ unsigned long long shell_sum(const uint32_t *tally, uint32_t S, uint32_t s)
+{
+    const uint32_t C = hist_cells(S);
+    if (s + 1 < S)
+        return ((unsigned long long)tally[C + s] << 32) | tally[s];
+    const uint32_t at = s + (threadIdx.x & 31u);
+    return warp_sum_u64(((unsigned long long)tally[C + at] << 32) | tally[at]);
 }
 
 }  // namespace tmc
