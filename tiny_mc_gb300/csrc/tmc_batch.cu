@@ -39,7 +39,7 @@ namespace tmc {
 // back-off while nothing is published (bounded: see queue_idle_verdict), and
 // each finished item's completion is appended to the completion ring.
 template <int BLOCK, class M, bool QUEUE>
-__global__ void __launch_bounds__(BLOCK) walk_batch(const BatchArgs a)
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_batch(const BatchArgs a)
 {
     constexpr uint32_t END = 0xffffffffu;
     extern __shared__ __align__(16) uint32_t smem[];

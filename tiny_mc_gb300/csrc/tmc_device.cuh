@@ -107,11 +107,18 @@ __device__ __forceinline__ uint32_t rand31(uint32_t word)
     return max(word >> 1, 1u);
 }
 
-// rand()/(float)RAND_MAX: (float)RAND_MAX is exactly 2^31, so the quotient is
-// the correctly rounded int->float conversion scaled by 2^-31 (exact).
-__device__ __forceinline__ float uniform01(uint32_t word)
+// The 31 bits as a float, rounded once; 0 stays 0.
+__device__ __forceinline__ float rand_float(uint32_t word)
 {
-    return __uint2float_rn(rand31(word)) * 0x1p-31f;
+    return __uint2float_rn(word >> 1);
+}
+
+// rand()/(float)RAND_MAX: (float)RAND_MAX is exactly 2^31, so the quotient is
+// the correctly rounded int->float conversion scaled by 2^-31 (exact).  The
+// 0 -> 1 mapping commutes with the conversion.
+__device__ __forceinline__ float uniform01(float r)
+{
+    return fmaxf(r, 1.0f) * 0x1p-31f;
 }
 
 // 2.0f*rand()/(float)RAND_MAX - 1.0f: 2*fl(r)/2^31 is exact, so one fused
@@ -119,9 +126,9 @@ __device__ __forceinline__ float uniform01(uint32_t word)
 // rand31's 0 -> 1 mapping is left out here because it cannot change the
 // result: -1 + 2^-30 rounds to -1.0f (the float spacing next to -1 is 2^-24),
 // the same value r = 0 gives.
-__device__ __forceinline__ float uniform_pm1(uint32_t word)
+__device__ __forceinline__ float uniform_pm1(float r)
 {
-    return fmaf(__uint2float_rn(word >> 1), 0x1p-30f, -1.0f);
+    return fmaf(r, 0x1p-30f, -1.0f);
 }
 
 // ------------------------------------------------------------ arithmetic
@@ -188,6 +195,7 @@ struct ExactMath {
         return __fadd_rn(__fmul_rn(a, a), __fmul_rn(b, b));
     }
     static constexpr float ONE = 1.0f;   // the launch direction's w
+    static constexpr bool CHEAP_DIRECTION = false;
     // photon.c:41-43 from an accepted try
     __device__ static __forceinline__ void direction(float t, float xi1, float xi2, float &u, float &v, float &w)
     {
@@ -216,6 +224,7 @@ struct FastMath {
     }
     __device__ static __forceinline__ float norm2(float a, float b) { return fmaf(a, a, b * b); }
     static constexpr float ONE = 0.5f;   // the launch direction's w, halved
+    static constexpr bool CHEAP_DIRECTION = true;
     // (1-u^2)/t with u = 2t-1 is 4(1-t): sqrt of it is 2 sqrt(1-t)
     __device__ static __forceinline__ void direction(float t, float xi1, float xi2, float &u, float &v, float &w)
     {

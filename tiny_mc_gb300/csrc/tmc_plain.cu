@@ -58,7 +58,7 @@ struct PlainArgs {
 };
 
 template <int BLOCK, class M, Hist H>
-__global__ void __launch_bounds__(BLOCK) walk_plain(const PlainArgs a)
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArgs a)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     constexpr bool PER_WARP = H == Hist::Warp;
@@ -119,27 +119,19 @@ static cudaError_t occupancy(const DeviceCtx &ctx, size_t smem, int &per_sm)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_plain<BLOCK, M, H>, BLOCK, smem);
 }
 
-template <int BLOCK, class M, Hist H>
-static cudaError_t launch_t(const PlainLaunch &L, const DeviceCtx &ctx, int per_sm, cudaStream_t stream)
+// Grid and arguments of a launch of `block`-thread blocks, per_sm resident.
+static unsigned plain_args(const PlainLaunch &L, const DeviceCtx &ctx, int block, int per_sm, PlainArgs &a)
 {
-    const size_t smem = plain_smem_bytes(L.d.shells, BLOCK, H);
-    cudaError_t e = set_smem<BLOCK, M, H>(smem);
-    if (e != cudaSuccess)
-        return e;
-    if (per_sm < 1)
-        return cudaErrorInvalidConfiguration;
     if (L.blocks_per_sm > 0)
         per_sm = std::min(per_sm, L.blocks_per_sm);
     unsigned long long grid = (unsigned long long)ctx.sms * per_sm;
     // no more blocks than there are photon chunks to hand out
-    const unsigned chunk = claim_chunk(L.n_photons, grid * (BLOCK / 32), ctx.sms, L.d.albedo);
-    const unsigned long long warps_needed = (L.n_photons + chunk - 1) / chunk;
-    const unsigned long long blocks_needed = (warps_needed + BLOCK / 32 - 1) / (BLOCK / 32);
+    a.chunk = claim_chunk(L.n_photons, grid * (block / 32), ctx.sms, L.d.albedo);
+    const unsigned long long warps_needed = (L.n_photons + a.chunk - 1) / a.chunk;
+    const unsigned long long blocks_needed = (warps_needed + block / 32 - 1) / (block / 32);
     grid = std::max(1ull, std::min(grid, blocks_needed));
     if (L.max_blocks > 0)
         grid = std::min(grid, (unsigned long long)L.max_blocks);
-
-    PlainArgs a;
     a.keys = make_philox_keys(L.p->seed);
     a.c.albedo = L.d.albedo;
     a.c.spm = L.d.spm;
@@ -150,8 +142,21 @@ static cudaError_t launch_t(const PlainLaunch &L, const DeviceCtx &ctx, int per_
     a.tally = reinterpret_cast<unsigned long long *>(L.d_tally);
     a.work = L.d_work;
     a.steps = L.d_steps;
-    a.chunk = chunk;
-    walk_plain<BLOCK, M, H><<<(unsigned)grid, BLOCK, smem, stream>>>(a);
+    return (unsigned)grid;
+}
+
+template <int BLOCK, class M, Hist H>
+static cudaError_t launch_t(const PlainLaunch &L, const DeviceCtx &ctx, int per_sm, cudaStream_t stream)
+{
+    const size_t smem = plain_smem_bytes(L.d.shells, BLOCK, H);
+    cudaError_t e = set_smem<BLOCK, M, H>(smem);
+    if (e != cudaSuccess)
+        return e;
+    if (per_sm < 1)
+        return cudaErrorInvalidConfiguration;
+    PlainArgs a;
+    const unsigned grid = plain_args(L, ctx, BLOCK, per_sm, a);
+    walk_plain<BLOCK, M, H><<<grid, BLOCK, smem, stream>>>(a);
     return cudaGetLastError();
 }
 

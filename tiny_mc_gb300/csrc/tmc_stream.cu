@@ -128,6 +128,41 @@ __device__ __forceinline__ bool open_item(const BatchArgs &a, OpenItem *o)
     return false;
 }
 
+// step_photon's tally of a lane: its photon's item's histogram and record.
+template <class M>
+struct StreamTally {
+    uint32_t *hist;
+    uint32_t cells, last, probe;
+    float albedo;
+    unsigned long long *g;
+    OpenItem *item;
+    uint32_t &steps;   // of this lane's photon
+    bool &want;
+
+    __device__ __forceinline__ void step(LanePhoton &p, uint32_t cell)
+    {
+        const uint32_t shell = min(cell, last);
+        uint32_t *t0 = hist + cell;
+        uint32_t lo, hi;
+        units_split(weight_units(p.weight), lo, hi);
+        tally_add(t0, t0 + cells, &g[4 * shell + 1], lo, hi, shell == probe ? &item->wraps : nullptr);
+        units_split(weight2_units(p.weight), lo, hi);
+        tally_add(t0 + 2 * cells, t0 + 3 * cells, &g[4 * shell + 3], lo, hi);
+        p.weight = M::mul(p.weight, albedo);
+        ++steps;
+    }
+    __device__ __forceinline__ bool low(const LanePhoton &p) const { return p.weight < 0.001f * WEIGHT_ONE; }
+    __device__ __forceinline__ void survived(LanePhoton &p) { p.weight = __fdiv_rn(p.weight, 0.1f); }
+    __device__ __forceinline__ void died(LanePhoton &)
+    {
+        want = true;
+        // the photon's steps into its item's 64-bit count
+        const uint32_t old = atomicAdd(&item->steps_lo, steps);
+        if (old + steps < old)
+            atomicAdd(&item->steps_hi, 1u);
+    }
+};
+
 }  // namespace
 
 template <int BLOCK, class M, bool QUEUE>
@@ -351,33 +386,12 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
         }
         wait_start = 0;
 
-        uint32_t *hist = smem + lb * HS;
+        StreamTally<M> tally{smem + lb * HS, pc.shells + spread, pc.shells - 1, pps, pc.albedo, pg, &open[lb], steps, want};
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             if (k % 2 == 0)
                 R::refill(p, ring, a.keys);
-            step_photon<BLOCK, M>(
-                p, ring, pc.spm, pc.last, pc.last + (float)(lane & spread), pc.albedo,
-                [&](uint32_t cell, float weight) {
-                    const uint32_t C = pc.shells + spread;
-                    const uint32_t shell = min(cell, pc.shells - 1);
-                    uint32_t *t0 = hist + cell;
-                    uint32_t lo, hi;
-                    units_split(weight_units(weight), lo, hi);
-                    tally_add(t0, t0 + C, &pg[4 * shell + 1], lo, hi,
-                              shell == pps ? (uint32_t *)&open[lb].wraps : nullptr);
-                    units_split(weight2_units(weight), lo, hi);
-                    tally_add(t0 + 2 * C, t0 + 3 * C, &pg[4 * shell + 3], lo, hi);
-                    ++steps;
-                },
-                [&] {
-                    want = true;
-                    // the photon's steps into its item's 64-bit count
-                    uint32_t *sl = (uint32_t *)&open[lb].steps_lo;
-                    const uint32_t old = atomicAdd(sl, steps);
-                    if (old + steps < old)
-                        atomicAdd((uint32_t *)&open[lb].steps_hi, 1u);
-                });
+            step_photon<BLOCK, M>(p, ring, pc.spm, pc.last, pc.last + (float)(lane & spread), tally);
         }
     }
     // every warp has left the loop (their waits are bounded)

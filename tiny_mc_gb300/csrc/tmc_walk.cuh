@@ -16,8 +16,8 @@
 //    (p = 0.046) skips the move/absorb part on the next iteration, so lanes
 //    of a warp stay in lock-step instead of waiting for the lane with the
 //    most retries;
-//  * random words come from a per-thread ring of 16 words in shared memory;
-//    slots 16..20 mirror 0..4, so the <= 6 words one iteration reads (step,
+//  * random words come, as floats, from a per-thread ring of 16 slots in shared
+//    memory; slots 16..20 mirror 0..4, so the <= 6 words one iteration reads (step,
 //    four for two tries, roulette) are fixed offsets from one base.  Every
 //    second iteration each lane computes two Philox blocks and stores them if
 //    its ring has room for eight words.  No vote decides on a refill: an
@@ -53,7 +53,17 @@ namespace tmc {
 constexpr int RING = 16;        // random words buffered per thread
 constexpr int MIRROR = 5;       // slots 16..20 repeat slots 0..4
 constexpr int SLOTS = RING + MIRROR;
-constexpr int TRIP = 4;         // iterations between checks for finished photons
+
+// Iterations of the unrolled loop body, between checks for finished photons.  A
+// check is ~60 warp-instructions when a photon has ended, a lane whose photon
+// ended waits half a body, and every pass through the loop moves the lane's
+// state between registers (5 instructions per step with a body of 4).  2^26
+// photons of params.h optics: 27.8 ms with 4, 27.3 with 6, 26.9 with 8; 2^20
+// high-albedo 44.1, 42.5, 42.3; 2^22 photons of three steps (albedo 0.09)
+// 0.152, 0.169, 0.175 ms.  (Two passes through a body of 4 per check: 27.9.)
+constexpr int TRIP = 8, SHORT_TRIP = 4;
+constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the first roulette
+
 // The whole warp walks its photons one after another (warp_steps) once the
 // source has no more and at most this many are left.  A lane-loop iteration is
 // ~190 warp-instructions however few lanes walk, a photon's step by the whole
@@ -260,7 +270,10 @@ struct LanePhoton {
     uint32_t blk = 0, cur = 0;
     float x = 0.f, y = 0.f, z = 0.f, u = 0.f, v = 0.f, w = 0.f;
     float weight = 0.f;   // times 2^20 (an exact scaling)
-    float t = 0.f;        // norm of the last try; above 1 the direction is still sought
+    // Norm of the last try; above 1 the direction is still sought, and cur is
+    // one word before the next try's (where a step's own word would be), so
+    // that tries are always words 1 .. 4 from cur.
+    float t = 0.f;
 };
 
 template <int BLOCK>
@@ -272,29 +285,44 @@ struct Ring {
     __device__ static __forceinline__ int fill(const LanePhoton &p) { return (int)(p.blk * (4 * W) - p.cur); }
     __device__ static __forceinline__ bool walking(const LanePhoton &p) { return fill(p) >= 0; }
     __device__ static __forceinline__ void drop(LanePhoton &p) { p.cur = p.blk * (4 * W) + NO_PHOTON; }
-    __device__ static __forceinline__ uint32_t word(const char *at, int slot)
+    // A photon its lane cannot go on with: kept at a fill below -W until the
+    // whole warp walks it.
+    static constexpr uint32_t ASIDE = 4 * RING * W;
+    __device__ static __forceinline__ void set_aside(LanePhoton &p) { p.cur += ASIDE; }
+    __device__ static __forceinline__ bool aside(const LanePhoton &p) { return fill(p) < -(int)W; }
+    __device__ static __forceinline__ float real(const char *at, int slot)
     {
-        return *reinterpret_cast<const uint32_t *>(at + slot * W);
+        return *reinterpret_cast<const float *>(at + slot * W);
     }
 
-    // Two Philox blocks into the ring where it has room for them.
+    // Two Philox blocks into the ring where it has room for them (a lane
+    // without a photon, or set aside, has a negative fill: no room).
     __device__ static __forceinline__ void refill(LanePhoton &p, char *ring, const PhiloxKeys &keys)
     {
         const uint4 r = philox_block(p.blk, p.key, keys);
         const uint4 q = philox_block(p.blk + 1, p.key, keys);
-        if ((uint32_t)fill(p) <= (RING - 8) * W) {
-            const uint32_t off = (p.blk * (4 * W)) & MASK;
-            const uint32_t words[8] = {r.x, r.y, r.z, r.w, q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                *reinterpret_cast<uint32_t *>(ring + off + k * W) = words[k];
-            if (off == 0) {
-#pragma unroll
-                for (int k = 0; k < MIRROR; ++k)
-                    *reinterpret_cast<uint32_t *>(ring + off + (RING + k) * W) = words[k];
-            }
+        const uint32_t off = (p.blk * (4 * W)) & MASK;
+        const uint32_t filled = (uint32_t)fill(p);
+        const uint32_t at = (uint32_t)__cvta_generic_to_shared(ring) + off;
+        // predicated stores: branches around them cost more than the stores
+        asm volatile("{\n\t.reg .pred p, q;\n\t"
+                     "setp.le.u32 p, %0, %11;\n\tsetp.eq.and.u32 q, %1, 0, p;\n\t"
+                     "@p st.shared.f32 [%2], %3;\n\t@p st.shared.f32 [%2+%12], %4;\n\t"
+                     "@p st.shared.f32 [%2+%13], %5;\n\t@p st.shared.f32 [%2+%14], %6;\n\t"
+                     "@p st.shared.f32 [%2+%15], %7;\n\t@p st.shared.f32 [%2+%16], %8;\n\t"
+                     "@p st.shared.f32 [%2+%17], %9;\n\t@p st.shared.f32 [%2+%18], %10;\n\t"
+                     "@q st.shared.f32 [%2+%19], %3;\n\t@q st.shared.f32 [%2+%20], %4;\n\t"
+                     "@q st.shared.f32 [%2+%21], %5;\n\t@q st.shared.f32 [%2+%22], %6;\n\t"
+                     "@q st.shared.f32 [%2+%23], %7;\n\t}" ::"r"(filled),
+                     "r"(off), "r"(at), "f"(rand_float(r.x)), "f"(rand_float(r.y)), "f"(rand_float(r.z)),
+                     "f"(rand_float(r.w)), "f"(rand_float(q.x)), "f"(rand_float(q.y)), "f"(rand_float(q.z)),
+                     "f"(rand_float(q.w)), "n"((RING - 8) * W), "n"(W), "n"(2 * W), "n"(3 * W), "n"(4 * W),
+                     "n"(5 * W), "n"(6 * W), "n"(7 * W), "n"(RING * W), "n"((RING + 1) * W), "n"((RING + 2) * W),
+                     "n"((RING + 3) * W), "n"((RING + 4) * W)
+                     : "memory");
+        static_assert(MIRROR == 5, "the mirror stores above");
+        if (filled <= (RING - 8) * W)
             p.blk += 2;
-        }
     }
 
     // Words of the photon's stream used so far, as whole blocks and a rest.
@@ -333,12 +361,13 @@ __device__ __forceinline__ void launch_photon(LanePhoton &p, unsigned long long 
 // One iteration of a lane's photon if six words are buffered (else it waits
 // for the next refill): move, deposit and decay unless its direction is still
 // sought, then two tries for the next direction and the roulette.
-// deposit(cell, weight) tallies a step, died() is called at the photon's end.
 // A radius below `last` shells goes to its shell's cell, any other (NaN too) to
-// cell `beyond`.
-template <int BLOCK, class M, class Deposit, class Died>
+// cell `beyond`.  The tally keeps the photon's weight: step(p, cell) deposits
+// and decays it, low(p) says whether it is below the roulette's threshold,
+// survived(p) and died(p) are the roulette's outcomes.
+template <int BLOCK, class M, class Tally>
 __device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, float spm, float last, float beyond,
-                                            float albedo, Deposit deposit, Died died)
+                                            Tally &tally)
 {
     using R = Ring<BLOCK>;
     if (R::fill(p) < (int)(6 * R::W))
@@ -346,41 +375,39 @@ __device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, flo
     const char *rd = ring + (p.cur & R::MASK);
     if (!(p.t > 1.0f)) {
         // move, photon.c:21-24
-        const float U = uniform01(R::word(rd, 0));
-        rd += R::W;
-        p.cur += R::W;
-        const float t = M::step_length(U);
+        const float t = M::step_length(uniform01(R::real(rd, 0)));
         p.x = M::move(p.x, t, p.u);
         p.y = M::move(p.y, t, p.v);
         p.z = M::move(p.z, t, p.w);
         // absorb, photon.c:26-32 (clamp in float: same shell for every radius
         // below 2^32 shells)
         const float r = M::radius_shells(p.x, p.y, p.z, spm);
-        deposit(__float2uint_rz(r < last ? r : beyond), p.weight);
-        p.weight = M::mul(p.weight, albedo);
+        tally.step(p, __float2uint_rz(r < last ? r : beyond));
     }
     // the next two tries of the rejection method, photon.c:36-40; the second
     // one's words are consumed only if the first is rejected
-    const float xa1 = uniform_pm1(R::word(rd, 0)), xa2 = uniform_pm1(R::word(rd, 1));
-    const float xb1 = uniform_pm1(R::word(rd, 2)), xb2 = uniform_pm1(R::word(rd, 3));
+    const float xa1 = uniform_pm1(R::real(rd, 1)), xa2 = uniform_pm1(R::real(rd, 2));
+    const float xb1 = uniform_pm1(R::real(rd, 3)), xb2 = uniform_pm1(R::real(rd, 4));
     const float ta = M::norm2(xa1, xa2), tb = M::norm2(xb1, xb2);
     const bool first = !(1.0f < ta);
     const float xi1 = first ? xa1 : xb1;
     const float xi2 = first ? xa2 : xb2;
     p.t = first ? ta : tb;
-    p.cur += first ? 2 * R::W : 4 * R::W;
-    if (!(p.t > 1.0f)) {
-        M::direction(p.t, xi1, xi2, p.u, p.v, p.w);   // photon.c:41-43
-        // roulette, photon.c:45-49
-        if (p.weight < 0.001f * WEIGHT_ONE) {
-            const float U = uniform01(R::word(ring + (p.cur & R::MASK), 0));
-            p.cur += R::W;
-            if (U > 0.1f) {
-                R::drop(p);
-                died();
-            } else {
-                p.weight = __fdiv_rn(p.weight, 0.1f);
-            }
+    const bool sought = p.t > 1.0f;
+    p.cur += first ? 3 * R::W : sought ? 4 * R::W : 5 * R::W;
+    // new direction, photon.c:41-43 (that of a rejected try is not used; where
+    // it costs little it is computed all the same, without a branch)
+    if (M::CHEAP_DIRECTION || !sought)
+        M::direction(p.t, xi1, xi2, p.u, p.v, p.w);
+    // roulette, photon.c:45-49
+    if (!sought && tally.low(p)) {
+        const float U = uniform01(R::real(ring + (p.cur & R::MASK), 0));
+        p.cur += R::W;
+        if (U > 0.1f) {
+            R::drop(p);
+            tally.died(p);
+        } else {
+            tally.survived(p);
         }
     }
 }
@@ -442,10 +469,17 @@ __device__ __forceinline__ uint32_t after_try(uint32_t c, uint32_t d, uint32_t a
     return any ? min(at + 4 * k + 2, NO_STEP) : NO_STEP;
 }
 
-// Up to 32 steps of the photon.  deposit(mine, shell, weight) is called by
-// every lane (mine: this lane holds a step).  Returns the number of steps, 0 if
-// a step needs more words than a round has (the caller then walks it on one
-// lane); dead is set when the roulette ended the photon.
+// Word `at` of the photon's stream, counted from block p.block.
+__device__ __forceinline__ uint32_t stream_word(const WarpPhoton &p, uint32_t at, const PhiloxKeys &keys)
+{
+    const uint4 q = philox_block(p.block + (at >> 2), p.key, keys);
+    const uint32_t i = at & 3u;
+    return i == 0u ? q.x : i == 1u ? q.y : i == 2u ? q.z : q.w;
+}
+
+// Up to 32 steps of the photon; returns their number n >= 1.  Lanes below n
+// hold a step each: the cell it deposits into and the weight.  dead is set when
+// the roulette ended the photon.
 template <class M>
 __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const WarpScratch &sc, const WalkConsts &c,
                                                const PhiloxKeys &keys, float beyond, uint32_t &cell_out,
@@ -457,7 +491,8 @@ __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const 
     *reinterpret_cast<uint4 *>(sc.row(lane >> 3) + (lane & 7u) * 16) = r;
 
     // tries at this lane's four positions, then the map
-    const float f0 = uniform_pm1(r.x), f1 = uniform_pm1(r.y), f2 = uniform_pm1(r.z), f3 = uniform_pm1(r.w);
+    const float f0 = uniform_pm1(rand_float(r.x)), f1 = uniform_pm1(rand_float(r.y));
+    const float f2 = uniform_pm1(rand_float(r.z)), f3 = uniform_pm1(rand_float(r.w));
     const float f4 = __shfl_down_sync(FULL_MASK, f0, 1);
     const uint32_t a0 = __ballot_sync(FULL_MASK, !(1.0f < M::norm2(f0, f1)));
     const uint32_t a1 = __ballot_sync(FULL_MASK, !(1.0f < M::norm2(f1, f2)));
@@ -483,16 +518,27 @@ __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const 
             power = __byte_perm(__byte_perm(q0, q1, 0x0040u), __byte_perm(q2, q3, 0x0040u), 0x5410u);
         }
     }
-    const uint32_t next = map_at(map, start);
+    uint32_t next = map_at(map, start);
     const bool whole = next != NO_STEP;
     uint32_t n = __popc(__ballot_sync(FULL_MASK, whole));   // a prefix of the lanes
-    if (n == 0)
-        return 0;
+    __syncwarp();
+    uint32_t w_step = sc.word(start), w_xi1 = sc.word(next - 2), w_xi2 = sc.word(next - 1);
+    if (n == 0) {   // the first step alone needs more words than a round has
+        next = p.rest;
+        w_step = stream_word(p, next++, keys);
+#pragma unroll 1
+        for (bool second = false;; second = !second) {
+            w_xi1 = w_xi2;
+            w_xi2 = stream_word(p, next++, keys);
+            if (second && !(1.0f < M::norm2(uniform_pm1(rand_float(w_xi1)), uniform_pm1(rand_float(w_xi2)))))
+                break;
+        }
+        n = 1;
+    }
 
     // step length, new direction
-    __syncwarp();
-    const float t = M::step_length(uniform01(sc.word(start)));
-    const float xi1 = uniform_pm1(sc.word(next - 2)), xi2 = uniform_pm1(sc.word(next - 1));
+    const float t = M::step_length(uniform01(rand_float(w_step)));
+    const float xi1 = uniform_pm1(rand_float(w_xi1)), xi2 = uniform_pm1(rand_float(w_xi2));
     float nu, nv, nw;
     M::direction(M::norm2(xi1, xi2), xi1, xi2, nu, nv, nw);
     float u = __shfl_up_sync(FULL_MASK, nu, 1), v = __shfl_up_sync(FULL_MASK, nv, 1);
@@ -538,7 +584,7 @@ __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const 
     const float y = reinterpret_cast<const float *>(sc.row(2))[lane];
     const float z = reinterpret_cast<const float *>(sc.row(3))[lane];
     const float decayed = M::mul(weight, c.albedo);
-    const uint32_t low = __ballot_sync(FULL_MASK, whole && decayed < 0.001f * WEIGHT_ONE);
+    const uint32_t low = __ballot_sync(FULL_MASK, lane < n && decayed < 0.001f * WEIGHT_ONE);
     if (low)
         n = __ffs((int)low);   // the steps up to the first roulette
     const float radius = M::radius_shells(x, y, z, c.spm);
@@ -557,9 +603,7 @@ __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const 
     dead = false;
     if (low) {
         // roulette, photon.c:45-49; its word may lie behind the round's
-        const uint4 q = philox_block(p.block + (to >> 2), p.key, keys);
-        const uint32_t i = to & 3u;
-        const float U = uniform01(i == 0u ? q.x : i == 1u ? q.y : i == 2u ? q.z : q.w);
+        const float U = uniform01(rand_float(stream_word(p, to, keys)));
         ++to;
         dead = U > 0.1f;
         p.weight = __fdiv_rn(p.weight, 0.1f);
@@ -569,62 +613,70 @@ __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const 
     return n;
 }
 
-// The photon of lane `l`, in every lane.
+// While the whole warp walks a photon, the lanes' photons are put away in the
+// ring rows behind the scratch, a column per lane (what the rings hold is
+// drawn again afterwards).  Kept in registers they and warp_steps' values
+// exceed 64, and the compiler spills in the lane loop: 4.6 local-memory
+// accesses per photon step.
+enum SavedWord { S_KEY, S_BLOCK = 4, S_REST, S_X, S_Y, S_Z, S_U, S_V, S_W, S_WEIGHT, S_T, S_ROW, SAVED_WORDS };
+constexpr int SAVED_ROW = 4;
+static_assert(SAVED_ROW + SAVED_WORDS <= SLOTS, "saved photons fit in the ring");
+
 template <int BLOCK>
-__device__ __forceinline__ WarpPhoton broadcast_photon(const LanePhoton &p, int l)
-{
-    WarpPhoton q;
-    uint32_t block, rest;
-    Ring<BLOCK>::position(p, block, rest);
-    q.key.a = __shfl_sync(FULL_MASK, p.key.a, l);
-    q.key.b = __shfl_sync(FULL_MASK, p.key.b, l);
-    q.key.c = __shfl_sync(FULL_MASK, p.key.c, l);
-    q.key.d = __shfl_sync(FULL_MASK, p.key.d, l);
-    q.block = __shfl_sync(FULL_MASK, block, l);
-    q.rest = __shfl_sync(FULL_MASK, rest, l);
-    q.x = __shfl_sync(FULL_MASK, p.x, l);
-    q.y = __shfl_sync(FULL_MASK, p.y, l);
-    q.z = __shfl_sync(FULL_MASK, p.z, l);
-    q.u = __shfl_sync(FULL_MASK, p.u, l);
-    q.v = __shfl_sync(FULL_MASK, p.v, l);
-    q.w = __shfl_sync(FULL_MASK, p.w, l);
-    q.weight = __shfl_sync(FULL_MASK, p.weight, l);
-    return q;
-}
+struct SavedPhotons {
+    char *rows;   // the warp's ring columns
+    __device__ __forceinline__ uint32_t &word(int l, int k) const
+    {
+        return *reinterpret_cast<uint32_t *>(rows + (SAVED_ROW + k) * Ring<BLOCK>::W + 4 * l);
+    }
+    __device__ __forceinline__ float real(int l, int k) const { return __uint_as_float(word(l, k)); }
+    __device__ __forceinline__ void put(int l, int k, float v) const { word(l, k) = __float_as_uint(v); }
 
-// Walk photons from `src` until it is exhausted and every lane's photon has
-// died.  Warp-collective: all 32 lanes of every warp call it.  tally: the
-// shared histogram (H = Warp: this warp's; Block: the block's), 4 * hist_cells
-// words (low and high of sum w, then of sum w^2), flushed into g, the
-// problem's global 128-bit tally [shells][4], every flush_steps iterations;
-// the caller flushes what is left.  probe_acc / probe_hi (Block only, may be
-// null): receive the w sums those flushes take from shell probe_shell.
-// Returns this thread's photon steps.
-template <int BLOCK, class M, class Source, Hist H>
-__device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
-                                              const PhiloxKeys &keys, uint32_t *tally,
-                                              unsigned long long *g, uint32_t *my,
-                                              unsigned long long *probe_acc = nullptr,
-                                              uint32_t *probe_hi = nullptr,
-                                              uint32_t probe_shell = 0)
-{
-    using R = Ring<BLOCK>;
-    constexpr uint32_t FLUSH_TRIPS = flush_steps(H == Hist::Warp ? 32u : (uint32_t)BLOCK) / TRIP;
-    const uint32_t S = c.shells;
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    char *ring = reinterpret_cast<char *>(my);
-    const uint32_t hist = (uint32_t)__cvta_generic_to_shared(tally);
+    __device__ __forceinline__ void save(int l, const LanePhoton &p, float weight, uint32_t row) const
+    {
+        uint32_t block, rest;
+        Ring<BLOCK>::position(p, block, rest);
+        word(l, S_KEY) = p.key.a;
+        word(l, S_KEY + 1) = p.key.b;
+        word(l, S_KEY + 2) = p.key.c;
+        word(l, S_KEY + 3) = p.key.d;
+        put(l, S_T, p.t);
+        put_walk(l, WarpPhoton{{}, block, rest, p.x, p.y, p.z, p.u, p.v, p.w, weight}, row);
+    }
+    __device__ __forceinline__ void put_walk(int l, const WarpPhoton &q, uint32_t row) const
+    {
+        word(l, S_BLOCK) = q.block;
+        word(l, S_REST) = q.rest;
+        put(l, S_X, q.x);
+        put(l, S_Y, q.y);
+        put(l, S_Z, q.z);
+        put(l, S_U, q.u);
+        put(l, S_V, q.v);
+        put(l, S_W, q.w);
+        put(l, S_WEIGHT, q.weight);
+        word(l, S_ROW) = row;
+    }
+    __device__ __forceinline__ WarpPhoton get(int l) const
+    {
+        return WarpPhoton{{word(l, S_KEY), word(l, S_KEY + 1), word(l, S_KEY + 2), word(l, S_KEY + 3)},
+                          word(l, S_BLOCK), word(l, S_REST),
+                          real(l, S_X), real(l, S_Y), real(l, S_Z), real(l, S_U), real(l, S_V), real(l, S_W),
+                          real(l, S_WEIGHT)};
+    }
+};
 
-    LanePhoton p{};
-    R::drop(p);
-    uint32_t steps = 0, trips = 0;
-    unsigned idle = 0;   // lanes that get no more photons
+// Tally objects of step_photon: `whole` deposits a step of a photon that the
+// whole warp walks.
+template <class M, Hist H>
+struct WeightTally {
+    uint32_t hist;            // shared address of the histogram
+    uint32_t plane;           // bytes between a cell's words
+    unsigned long long *g;    // global tally (H = Global)
+    float albedo;
+    uint32_t steps = 0;
 
-    const float beyond = H == Hist::Global ? c.last : c.last + (float)lane;
-    const uint32_t plane = 4 * hist_cells(S);   // bytes between a cell's words
-
-    auto deposit = [&](uint32_t cell, float weight) {
+    __device__ __forceinline__ void deposit(uint32_t cell, float weight)
+    {
         uint32_t lo, hi;
         if constexpr (H == Hist::Global) {
             unsigned long long *gs = g + 4 * (size_t)cell;
@@ -640,76 +692,157 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
             tally_add_nowrap(at + 2 * plane, at + 3 * plane, lo, hi);
         }
         ++steps;
-    };
+    }
+    __device__ __forceinline__ void launched() {}
+    __device__ __forceinline__ void step(LanePhoton &p, uint32_t cell)
+    {
+        deposit(cell, p.weight);
+        p.weight = M::mul(p.weight, albedo);
+    }
+    __device__ __forceinline__ bool low(const LanePhoton &p) const { return p.weight < 0.001f * WEIGHT_ONE; }
+    __device__ __forceinline__ void survived(LanePhoton &p) { p.weight = __fdiv_rn(p.weight, 0.1f); }
+    __device__ __forceinline__ void died(LanePhoton &) {}
+    // for the whole warp's walk: the weight, and the table's row (counts only)
+    __device__ __forceinline__ float weight(const LanePhoton &p) const { return p.weight; }
+    __device__ __forceinline__ uint32_t row_of(const LanePhoton &) const { return 0; }
+    __device__ __forceinline__ uint32_t row_after(uint32_t, uint32_t) const { return 0; }
+    __device__ __forceinline__ void resume(LanePhoton &, uint32_t) {}
+    __device__ __forceinline__ void whole(uint32_t, uint32_t cell, float weight) { deposit(cell, weight); }
+};
+
+// Walk photons from `src` until it is exhausted and every lane's photon has
+// died.  Warp-collective: all 32 lanes of every warp call it.  flush() empties
+// the shared histogram into the global tally; it is called at the latest every
+// FLUSH iterations.
+template <int BLOCK, class M, bool COUNTS, uint32_t FLUSH, int TRIP, class Source, class Tally, class Flush>
+__device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, Source &src, const PhiloxKeys &keys,
+                                             uint32_t *my, Tally &tally, Flush flush)
+{
+    using R = Ring<BLOCK>;
+    constexpr uint32_t FLUSH_TRIPS = FLUSH / TRIP;   // 0: never
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    char *ring = reinterpret_cast<char *>(my);
+
+    LanePhoton p{};
+    R::drop(p);
+    uint32_t trips = 0;
+    unsigned idle = 0;   // lanes that get no more photons
+
     for (;;) {
         // -------- hand new photon ids to lanes whose photon died
         const unsigned dead = __ballot_sync(FULL_MASK, !R::walking(p));
+        unsigned todo = 0;   // photons for the whole warp
         if (dead != idle) {
-            const unsigned need = dead & ~idle;
-            unsigned long long pid = 0;
-            const bool got = src.next(need, __popc(need & lt_mask), lane, pid) && ((need >> lane) & 1u);
-            if (got)
-                launch_photon<M>(p, pid, keys);
-            idle = dead & ~__ballot_sync(FULL_MASK, got);
-            if (idle == FULL_MASK)
-                break;
+            if constexpr (COUNTS)
+                todo = __ballot_sync(FULL_MASK, R::aside(p));
+            const unsigned need = dead & ~idle & ~todo;
+            if (need) {
+                unsigned long long pid = 0;
+                const bool got = src.next(need, __popc(need & lt_mask), lane, pid) && ((need >> lane) & 1u);
+                if (got) {
+                    launch_photon<M>(p, pid, keys);
+                    tally.launched();
+                }
+                idle = dead & ~todo & ~__ballot_sync(FULL_MASK, got);
+                if (idle == FULL_MASK)
+                    break;
+            }
         }
         // -------- few photons left: the whole warp walks them one by one
         if (idle && 32 - __popc(idle) <= WARP_WALK_MAX) {
-            // a photon whose direction is still sought waits for the lane loop
-            unsigned todo = __ballot_sync(FULL_MASK, R::walking(p) && !(p.t > 1.0f));
+            // (a photon whose direction is still sought waits for the lane loop)
+            todo |= __ballot_sync(FULL_MASK, R::walking(p) && !(p.t > 1.0f));
+        }
+        if (todo) {
             const WarpScratch sc{ring - 4 * lane, R::W};
-            while (todo && trips < FLUSH_TRIPS - 1) {
+            if (COUNTS && R::aside(p))
+                p.cur -= R::ASIDE;
+            unsigned left = __ballot_sync(FULL_MASK, R::walking(p));   // lanes with a photon
+            const unsigned had = left;
+            const SavedPhotons<BLOCK> saved{sc.rows};
+            __syncwarp();
+            saved.save((int)lane, p, tally.weight(p), tally.row_of(p));
+            __syncwarp();
+            while (todo && (FLUSH_TRIPS == 0 || trips < FLUSH_TRIPS)) {
                 const int l = __ffs((int)todo) - 1;
                 todo &= todo - 1;
-                WarpPhoton q = broadcast_photon<BLOCK>(p, l);
+                WarpPhoton q = saved.get(l);
+                uint32_t row = saved.word(l, S_ROW);
                 bool over = false;
-                uint32_t n;
                 do {
                     uint32_t cell;
                     float weight;
-                    n = warp_steps<M>(q, over, sc, c, keys, beyond, cell, weight);
+                    const uint32_t n = warp_steps<M>(q, over, sc, c, keys, beyond, cell, weight);
                     if (lane < n)
-                        deposit(cell, weight);
-                    if constexpr (H != Hist::Global)
+                        tally.whole(tally.row_after(row, lane), cell, weight);
+                    row = tally.row_after(row, n);
+                    if constexpr (FLUSH_TRIPS != 0)
                         ++trips;
-                } while (n && !over && trips < FLUSH_TRIPS - 1);
-                if ((int)lane == l) {
-                    if (over) {
-                        R::drop(p);
-                    } else {   // a flush is due, or a step took over 124 words: back to its lane
-                        p.x = q.x; p.y = q.y; p.z = q.z;
-                        p.u = q.u; p.v = q.v; p.w = q.w;
-                        p.weight = q.weight;
-                        p.blk = q.block + 4;   // position() below: 16 - rest words left
-                        p.cur = q.block * (4 * R::W) + q.rest * R::W;
-                    }
-                }
+                } while (!over && (FLUSH_TRIPS == 0 || trips < FLUSH_TRIPS));
+                if (over)
+                    left &= ~(1u << l);
+                else if ((int)lane == l)   // a flush is due first: back to its lane
+                    saved.put_walk(l, q, row);
             }
-            // the rings were scratch: refill those still in use
+            // back to the lanes, with fresh rings
             __syncwarp();
-            if (R::walking(p)) {
-                uint32_t block, rest;
-                R::position(p, block, rest);
-                R::restart(p, block, rest, ring, keys);
+            const WarpPhoton q = saved.get((int)lane);
+            const uint32_t row = saved.word((int)lane, S_ROW);
+            p.t = saved.real((int)lane, S_T);
+            __syncwarp();
+            p.key = q.key;
+            p.x = q.x; p.y = q.y; p.z = q.z;
+            p.u = q.u; p.v = q.v; p.w = q.w;
+            p.weight = q.weight;
+            if ((left >> lane) & 1u) {
+                R::restart(p, q.block, q.rest, ring, keys);
+                tally.resume(p, row);
+            } else {
+                R::drop(p);
             }
-            if (__any_sync(FULL_MASK, !R::walking(p) && !((idle >> lane) & 1u)))
+            if (left != had)
                 continue;
         }
-        if constexpr (H != Hist::Global) {
-            if (++trips >= FLUSH_TRIPS) {   // TRIP deposits of a lane at most since the last count
+        if constexpr (FLUSH_TRIPS != 0) {
+            if (trips == FLUSH_TRIPS) {   // a trip stands for TRIP deposits of a lane at most
                 trips = 0;
-                warp_flush_tally<H == Hist::Block>(tally, S, g, probe_acc, probe_hi, probe_shell);
+                flush();
             }
+            ++trips;
         }
 #pragma unroll
         for (int k = 0; k < TRIP; ++k) {
             if (k % 2 == 0)
                 R::refill(p, ring, keys);
-            step_photon<BLOCK, M>(p, ring, c.spm, c.last, beyond, c.albedo, deposit, [] {});
+            step_photon<BLOCK, M>(p, ring, c.spm, c.last, beyond, tally);
         }
     }
-    return steps;
+}
+
+// walk_photons with a shared histogram of 64-bit sums (H = Warp: this warp's;
+// Block: the block's), 4 * hist_cells words (low and high of sum w, then of sum
+// w^2), flushed into g, the problem's global 128-bit tally [shells][4], every
+// flush_steps iterations (the caller flushes what is left), or with none (H =
+// Global).  probe_acc / probe_hi (Block only, may be null): receive the w sums
+// those flushes take from shell probe_shell.  Returns this thread's photon
+// steps.
+template <int BLOCK, class M, class Source, Hist H>
+__device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
+                                              const PhiloxKeys &keys, uint32_t *tally,
+                                              unsigned long long *g, uint32_t *my,
+                                              unsigned long long *probe_acc = nullptr,
+                                              uint32_t *probe_hi = nullptr,
+                                              uint32_t probe_shell = 0)
+{
+    constexpr uint32_t FLUSH = H == Hist::Global ? 0u : flush_steps(H == Hist::Warp ? 32u : (uint32_t)BLOCK);
+    const float beyond = H == Hist::Global ? c.last : c.last + (float)(threadIdx.x & 31u);
+    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally), 4 * hist_cells(c.shells), g, c.albedo};
+    walk_photons<BLOCK, M, false, FLUSH, TRIP>(c, beyond, src, keys, my, t, [&] {
+        if constexpr (H != Hist::Global)
+            warp_flush_tally<H == Hist::Block>(tally, c.shells, g, probe_acc, probe_hi, probe_shell);
+    });
+    return t.steps;
 }
 
 // Add what is left in a block's histogram to a 128-bit global tally
