@@ -95,3 +95,41 @@ def test_last_shell_cells(tmc_mod, oracle_mod, shells):
         t, s = b.read()
         b.close()
         assert int(s[0]) == ref_steps and np.array_equal(as_array(t), ref), (block, stream)
+
+
+# Optics for the count table: rows up to the second, third or fourth roulette,
+# the largest shell count and albedo that still take it, one shell, albedo 0,
+# and walks of a few steps; then two the table is too large for.
+COUNT_OPTICS = [PARAMS_H, dict(shells=1, microns_per_shell=50.0, mu_a=2.0, mu_s=20.0),
+                dict(shells=101, microns_per_shell=50.0, mu_a=10.0, mu_s=1.0),
+                dict(shells=101, microns_per_shell=50.0, mu_a=1.0, mu_s=0.0),
+                dict(shells=501, microns_per_shell=20.0, mu_a=5.0, mu_s=5.0),
+                dict(shells=130, microns_per_shell=50.0, mu_a=2.0, mu_s=16.0),
+                dict(shells=101, microns_per_shell=50.0, mu_a=1.0, mu_s=12.0),
+                dict(shells=1001, microns_per_shell=50.0, mu_a=1.0, mu_s=9.0)]
+
+
+@pytest.mark.parametrize("math", ["exact", "fast"])
+@pytest.mark.parametrize("optics", COUNT_OPTICS)
+def test_counts_equal_sums(tmc_mod, optics, math):
+    """The per-(step, shell) counts of default launches give the tallies and
+    steps of the 64-bit sums (a given block size takes those), for enough
+    photons that some outlive the table and lanes walk several each."""
+    n = SMALL * 5 + 13
+    tmc_mod.set_plain_launch(0, 0, 0)
+    got = gpu_fx(tmc_mod, n, seed=6, base=1 << 34, math=math, **optics)
+    tmc_mod.set_plain_launch(0, 1, 3)          # few blocks: hundreds of photons per lane
+    few = gpu_fx(tmc_mod, n, seed=6, base=1 << 34, math=math, **optics)
+    tmc_mod.set_plain_launch(512, 0, 0)
+    ref = gpu_fx(tmc_mod, n, seed=6, base=1 << 34, math=math, **optics)
+    tmc_mod.set_plain_launch(0, 0, 0)
+    assert got[1] == ref[1] and few[1] == ref[1]
+    assert np.array_equal(got[0], ref[0]) and np.array_equal(few[0], ref[0])
+
+
+def test_counts_equal_oracle(tmc_mod, oracle_mod):
+    tmc_mod.set_plain_launch(0, 0, 0)
+    n = SMALL + 7
+    got, steps = gpu_fx(tmc_mod, n, seed=12, **PARAMS_H)
+    ref, _, ref_steps = oracle_fx(oracle_mod, n, seed=12, **PARAMS_H)
+    assert steps == ref_steps and np.array_equal(got, ref)

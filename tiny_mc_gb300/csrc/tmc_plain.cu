@@ -7,6 +7,8 @@
 // per block; each is added into the 128-bit global tally every flush_steps
 // iterations (2^18 for a warp's, 2^23 / threads for a block's) and at the
 // end.
+// Short walks over not too many shells (params.h's among them) take
+// walk_counts: one count per (step, shell) and block instead of the sums.
 // Shell counts whose histogram does not fit in shared memory at all
 // (params.h's SHELLS is any size in the reference) take the global form:
 // deposits go straight into the 128-bit global tally with 64-bit atomics.  The
@@ -55,6 +57,7 @@ struct PlainArgs {
     unsigned long long *work;    // photon claim counter, zero at launch
     unsigned long long *steps;   // += photon steps, may be null
     unsigned chunk;              // photon ids per claim
+    uint32_t rows;               // walk_counts: steps with counts
 };
 
 template <int BLOCK, class M, Hist H>
@@ -90,6 +93,101 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArg
         if ((threadIdx.x & 31u) == 0 && tot)
             atomicAdd(a.steps, tot);
     }
+}
+
+// One count per (step, shell): see CountTable.  Rows end behind a roulette.
+constexpr int COUNT_BLOCK = 512;
+
+__host__ __device__ constexpr uint32_t count_words(uint32_t rows, uint32_t shells)
+{
+    return ((rows + 1) * (hist_cells(shells) + 2) + 3) / 4 * 4;
+}
+
+template <class M, int TRIP>
+__global__ void __launch_bounds__(COUNT_BLOCK, 2) walk_counts(const PlainArgs a)
+{
+    extern __shared__ __align__(16) uint32_t smem[];
+    const uint32_t S = a.c.shells, C = hist_cells(S), stride = C + 2, rows = a.rows;
+    const uint32_t words = count_words(rows, S);
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+    const CountTable table{base, base + 4 * rows * stride, 4 * stride, 4 * C};
+    for (uint32_t s = threadIdx.x; s < words; s += COUNT_BLOCK)
+        smem[s] = 0;
+    __syncthreads();
+    // each row's weight and the row behind the next roulette, photon.c:32, 45-49
+    for (uint32_t n = threadIdx.x; n <= rows; n += COUNT_BLOCK) {
+        float weight = WEIGHT_ONE;
+        for (uint32_t k = 0;; ++k) {
+            if (k == n)
+                smem[n * stride + C] = __float_as_uint(weight);
+            weight = M::mul(weight, a.c.albedo);
+            const bool low = weight < 0.001f * WEIGHT_ONE;
+            if (k >= n && (low || k >= rows)) {
+                smem[n * stride + C + 1] = base + 4 * (k + 1) * stride;
+                break;
+            }
+            if (low)
+                weight = __fdiv_rn(weight, 0.1f);
+        }
+    }
+    __syncthreads();
+
+    GlobalSource src;
+    src.counter = a.work;
+    src.n = a.n_photons;
+    src.id_base = a.id_base;
+    src.chunk = a.chunk;
+    CountTally<M, COUNT_BLOCK> tally{table, S - 1, a.tally, table.base};
+    auto add_steps = [&](unsigned long long n) {
+        if (a.steps) {
+            n = warp_sum_u64(n);
+            if ((threadIdx.x & 31u) == 0 && n)
+                atomicAdd(a.steps, n);
+        }
+    };
+    // a warp adds at most 2^27 to a count between its flushes: 2^31 for a block
+    walk_photons<COUNT_BLOCK, M, true, (1u << 22), TRIP>(
+        a.c, a.c.last + (float)(threadIdx.x & 31u), src, a.keys, smem + words + threadIdx.x, tally, [&] {
+            add_steps(flush_counts<true>(smem, rows, S, threadIdx.x & 31u, 32, 0, 1, a.tally));
+        });
+
+    __syncthreads();
+    // the last shell's cells into its first, then shells x row groups
+    for (uint32_t n = threadIdx.x / 32; n < rows; n += COUNT_BLOCK / 32) {
+        uint32_t *at = smem + n * stride + S - 1;
+        uint32_t v = at[threadIdx.x & 31u];
+        v = __reduce_add_sync(FULL_MASK, v);
+        if ((threadIdx.x & 31u) == 0)
+            *at = v;
+    }
+    __syncthreads();
+    const uint32_t across = min((S + 31) / 32 * 32, (uint32_t)COUNT_BLOCK), groups = COUNT_BLOCK / across;
+    unsigned long long counted = tally.steps;
+    if (threadIdx.x < groups * across)
+        counted += flush_counts<false>(smem, rows, S, threadIdx.x % across, across, threadIdx.x / across, groups,
+                                       a.tally);
+    add_steps(counted);
+}
+
+// Rows up to the fourth, third or second roulette, whichever count table still
+// leaves two blocks per SM; 0 if none does.
+static uint32_t count_rows(const Derived &d, size_t smem_optin)
+{
+    const size_t most = (smem_optin + 1024) / 2 - 1024;   // of an SM's shared memory, less a block's own 1 KB
+    uint32_t rows = 0;
+    float weight = WEIGHT_ONE;
+    int roulettes = 0;
+    for (uint32_t n = 1; roulettes < 4; ++n) {
+        if (4 * (size_t)(count_words(n, d.shells) + SLOTS * COUNT_BLOCK) > most)
+            break;
+        weight *= d.albedo;
+        if (weight < 0.001f * WEIGHT_ONE) {
+            weight /= 0.1f;
+            if (++roulettes >= 2)
+                rows = n;
+        }
+    }
+    return rows;
 }
 
 static size_t plain_smem_bytes(uint32_t shells, int block, Hist h)
@@ -142,6 +240,7 @@ static unsigned plain_args(const PlainLaunch &L, const DeviceCtx &ctx, int block
     a.tally = reinterpret_cast<unsigned long long *>(L.d_tally);
     a.work = L.d_work;
     a.steps = L.d_steps;
+    a.rows = 0;
     return (unsigned)grid;
 }
 
@@ -158,6 +257,34 @@ static cudaError_t launch_t(const PlainLaunch &L, const DeviceCtx &ctx, int per_
     const unsigned grid = plain_args(L, ctx, BLOCK, per_sm, a);
     walk_plain<BLOCK, M, H><<<grid, BLOCK, smem, stream>>>(a);
     return cudaGetLastError();
+}
+
+template <class M, int TRIP>
+static cudaError_t launch_counts_t(const PlainLaunch &L, const DeviceCtx &ctx, uint32_t rows, cudaStream_t stream)
+{
+    const size_t smem = 4 * (size_t)(count_words(rows, L.d.shells) + SLOTS * COUNT_BLOCK);
+    cudaError_t e = cudaFuncSetAttribute(walk_counts<M, TRIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per_sm = 0;
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_counts<M, TRIP>, COUNT_BLOCK, smem);
+    if (e != cudaSuccess)
+        return e;
+    if (per_sm < 1)
+        return cudaErrorInvalidConfiguration;
+    PlainArgs a;
+    const unsigned grid = plain_args(L, ctx, COUNT_BLOCK, per_sm, a);
+    a.rows = rows;
+    walk_counts<M, TRIP><<<grid, COUNT_BLOCK, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+static cudaError_t launch_counts(const PlainLaunch &L, const DeviceCtx &ctx, uint32_t rows, cudaStream_t stream)
+{
+    if (L.p->math == TMC_MATH_FAST)
+        return L.d.albedo < SHORT_ALBEDO ? launch_counts_t<FastMath, SHORT_TRIP>(L, ctx, rows, stream)
+                                         : launch_counts_t<FastMath, TRIP>(L, ctx, rows, stream);
+    return L.d.albedo < SHORT_ALBEDO ? launch_counts_t<ExactMath, SHORT_TRIP>(L, ctx, rows, stream)
+                                     : launch_counts_t<ExactMath, TRIP>(L, ctx, rows, stream);
 }
 
 // Per-warp histograms where they fit at the occupancy a per-block histogram
@@ -190,17 +317,45 @@ static cudaError_t launch_b(const PlainLaunch &L, const DeviceCtx &ctx, cudaStre
                                       : launch_m<BLOCK, ExactMath>(L, ctx, stream);
 }
 
+template <class M>
+static cudaError_t load_kernels()
+{
+    const void *kernels[] = {
+        (const void *)walk_plain<128, M, Hist::Warp>, (const void *)walk_plain<128, M, Hist::Block>,
+        (const void *)walk_plain<128, M, Hist::Global>, (const void *)walk_plain<512, M, Hist::Warp>,
+        (const void *)walk_plain<512, M, Hist::Block>, (const void *)walk_plain<512, M, Hist::Global>,
+        (const void *)walk_counts<M, TRIP>, (const void *)walk_counts<M, SHORT_TRIP>};
+    for (const void *k : kernels) {
+        cudaFuncAttributes attr;
+        const cudaError_t e = cudaFuncGetAttributes(&attr, k);
+        if (e != cudaSuccess)
+            return e;
+    }
+    return cudaSuccess;
+}
+
 cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
     // 512 threads by default: 512 measured 0.8% faster than 256.  A launch too
     // small to give every SM a block of 512 takes blocks of 128, which spread
     // the same warps over four times as many SMs.
     const bool small = L.n_photons < (unsigned long long)ctx.sms * 512;
-    // a launch of no photons is a caller's set-up call: it loads both shapes
+    // a launch of no photons is a caller's set-up call: it loads every kernel
+    // a call of its arithmetic may take
     if (L.n_photons == 0 && !L.block) {
-        const cudaError_t e = launch_b<512>(L, ctx, stream);
+        const cudaError_t e = L.p->math == TMC_MATH_FAST ? load_kernels<FastMath>() : load_kernels<ExactMath>();
         if (e != cudaSuccess)
             return e;
+    }
+    // Counts instead of sums wherever their table fits: 2^24 photons of params.h
+    // optics 7.63 -> 6.86 ms, 2^25 in exact arithmetic 20.0 -> 18.4 ms, 2^22 at
+    // albedo 0.09 0.25 -> 0.15 ms, 131072 159 -> 126 us.  Not in small launches,
+    // where setting the table up and adding it costs more (32768 photons 98 us
+    // against 83).
+    if (L.block == 0 && !small) {
+        const uint32_t rows = count_rows(L.d, ctx.smem_optin);
+        if (rows)
+            return launch_counts(L, ctx, rows, stream);
     }
     switch (L.block ? L.block : small ? 128 : 512) {
     case 128: return launch_b<128>(L, ctx, stream);

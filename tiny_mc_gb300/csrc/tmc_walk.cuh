@@ -74,8 +74,9 @@ constexpr int WARP_WALK_MAX = 8;
 // Where a walk keeps its tallies.  Warp: one shared histogram per warp.
 // Block: one per block, shared by its warps.  Global: none; every deposit is
 // a 64-bit atomic add into the 128-bit global tally (shell counts whose
-// histogram does not fit in shared memory).
-enum class Hist { Warp, Block, Global };
+// histogram does not fit in shared memory).  Count: one count per (step, shell)
+// of a block (CountTable).
+enum class Hist { Warp, Block, Global, Count };
 
 // A warp adds the shared histogram it deposits into (its own, or its block's
 // of `lanes` lanes) into the global tally and clears it every
@@ -161,6 +162,87 @@ __device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, un
         flush128(&gl[2], &gl[3], v2);
     }
     __syncwarp();
+}
+
+// ------------------------------------------- counts per step and shell
+// A photon's weight is a function of the number of its steps alone: it decays
+// by one multiplication a step, and whether a roulette follows, and what
+// survivors are multiplied by, depends on the weight only.  So instead of two
+// 64-bit sums per shell (four atomics, two conversions and two carries a step),
+// a block can keep one 32-bit count per (step number, shell) and multiply by the
+// step's tally units at the end: the same integers, one atomic a step and no
+// weight in the loop.  It takes rows for the steps up to the second, third or
+// fourth roulette; a photon that survives that one (1 in 100 .. 10^4) is walked
+// to its end by the whole warp and tallied with 64-bit global atomics.
+//
+// A row is hist_cells counts, the weight (times 2^20) its deposits have, and
+// the address just behind the next roulette's row; one more row holds the
+// weight behind the last.  Addresses are shared-memory bytes.
+struct CountTable {
+    uint32_t base, end, stride;
+    uint32_t weight_at;   // of a row's weight; the roulette address follows
+};
+
+__device__ __forceinline__ uint32_t ld_shared(uint32_t addr)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+
+// Add a 128-bit value into a 128-bit global tally.
+__device__ __forceinline__ void flush128(unsigned long long *g_lo, unsigned long long *g_hi, unsigned long long lo,
+                                         unsigned long long hi)
+{
+    if (lo | hi) {
+        const unsigned long long old = atomicAdd(g_lo, lo);
+        hi += old + lo < old ? 1ull : 0ull;
+        if (hi)
+            atomicAdd(g_hi, hi);
+    }
+}
+
+// Add the counts of shells s0, s0 + ds, ... over rows n0, n0 + dn, ... into the
+// global tally; returns the sum of the counts.  EXCHANGE: take and clear them by
+// atomic exchanges while other warps deposit, the last shell's cells included;
+// else shell S-1's first cell holds the sum of its cells.
+template <bool EXCHANGE>
+__device__ __forceinline__ unsigned long long flush_counts(uint32_t *table, uint32_t rows, uint32_t S, uint32_t s0,
+                                                           uint32_t ds, uint32_t n0, uint32_t dn,
+                                                           unsigned long long *g)
+{
+    const uint32_t C = hist_cells(S), stride = C + 2;
+    unsigned long long total = 0;
+    for (uint32_t s = s0; s < S; s += ds) {
+        unsigned long long lo = 0, hi = 0, lo2 = 0, hi2 = 0;
+        for (uint32_t n = n0; n < rows; n += dn) {
+            uint32_t *row = table + n * stride;
+            uint32_t count = 0;
+            if constexpr (EXCHANGE) {
+                for (uint32_t c = s; c < (s + 1 < S ? s + 1 : C); ++c)
+                    count += atomicExch(row + c, 0u);
+            } else {
+                count = row[s];
+            }
+            if (count == 0)
+                continue;
+            total += count;
+            const float weight = __uint_as_float(row[C]);
+            uint32_t l, h;
+            units_split(weight_units(weight), l, h);
+            const unsigned long long u = ((unsigned long long)(h - UNITS_HI_BIAS) << 32) | l;
+            units_split(weight2_units(weight), l, h);
+            const unsigned long long u2 = ((unsigned long long)(h - UNITS_HI_BIAS) << 32) | l;
+            lo += u * count;
+            hi += __umul64hi(u, count) + (lo < u * count ? 1ull : 0ull);
+            lo2 += u2 * count;
+            hi2 += __umul64hi(u2, count) + (lo2 < u2 * count ? 1ull : 0ull);
+        }
+        unsigned long long *gs = g + 4 * (size_t)s;
+        flush128(&gs[0], &gs[1], lo, hi);
+        flush128(&gs[2], &gs[3], lo2, hi2);
+    }
+    return total;
 }
 
 // Per-problem constants of photon.c:8-9 (computed on the host in float,
@@ -708,6 +790,69 @@ struct WeightTally {
     __device__ __forceinline__ uint32_t row_after(uint32_t, uint32_t) const { return 0; }
     __device__ __forceinline__ void resume(LanePhoton &, uint32_t) {}
     __device__ __forceinline__ void whole(uint32_t, uint32_t cell, float weight) { deposit(cell, weight); }
+};
+
+template <class M, int BLOCK>
+struct CountTally {
+    CountTable table;
+    uint32_t last;            // index of the last shell
+    unsigned long long *g;
+    uint32_t row;             // of the photon's next deposit, from table.base
+    uint32_t roulette = 0;    // row behind its next roulette
+    uint32_t steps = 0;       // deposits outside the table
+
+    __device__ __forceinline__ void launched()
+    {
+        row = table.base;
+        roulette = ld_shared(table.base + table.weight_at + 4);
+    }
+    __device__ __forceinline__ void step(LanePhoton &, uint32_t cell)
+    {
+        red_shared_add(row + 4 * cell, 1u);
+        row += table.stride;
+    }
+    __device__ __forceinline__ bool low(const LanePhoton &) const { return row == roulette; }
+    __device__ __forceinline__ void survived(LanePhoton &p)
+    {
+        if (row == table.end)
+            Ring<BLOCK>::set_aside(p);
+        else
+            roulette = ld_shared(row + table.weight_at + 4);
+    }
+    __device__ __forceinline__ void died(LanePhoton &) {}
+    __device__ __forceinline__ float weight(const LanePhoton &) const
+    {
+        return __uint_as_float(ld_shared(row + table.weight_at));
+    }
+    __device__ __forceinline__ uint32_t row_of(const LanePhoton &) const { return row; }
+    __device__ __forceinline__ uint32_t row_after(uint32_t at, uint32_t steps) const
+    {
+        return min(at + steps * table.stride, table.end);
+    }
+    __device__ __forceinline__ void resume(LanePhoton &p, uint32_t at)
+    {
+        row = at;
+        if (p.t > 1.0f)   // the roulette behind its last deposit may be yet to come
+            return;
+        if (at == table.end)
+            Ring<BLOCK>::set_aside(p);
+        else
+            roulette = ld_shared(at + table.weight_at + 4);
+    }
+    __device__ __forceinline__ void whole(uint32_t at, uint32_t cell, float weight)
+    {
+        if (at < table.end) {
+            red_shared_add(at + 4 * cell, 1u);
+            return;
+        }
+        uint32_t lo, hi;
+        unsigned long long *gs = g + 4 * (size_t)min(cell, last);
+        units_split(weight_units(weight), lo, hi);
+        flush128(&gs[0], &gs[1], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
+        units_split(weight2_units(weight), lo, hi);
+        flush128(&gs[2], &gs[3], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
+        ++steps;
+    }
 };
 
 // Walk photons from `src` until it is exhausted and every lane's photon has
