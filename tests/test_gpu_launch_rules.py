@@ -133,3 +133,19 @@ def test_counts_equal_oracle(tmc_mod, oracle_mod):
     got, steps = gpu_fx(tmc_mod, n, seed=12, **PARAMS_H)
     ref, _, ref_steps = oracle_fx(oracle_mod, n, seed=12, **PARAMS_H)
     assert steps == ref_steps and np.array_equal(got, ref)
+
+
+# Shell counts on both sides of the block histogram's limit (1057 / 1058 cells
+# of a 128-thread block, 4513 / 4514 of a 512-thread one) and shell widths on
+# both sides of the split form's reach; the last one deposits everywhere beyond.
+@pytest.mark.parametrize("block", [0, 128, 512])
+@pytest.mark.parametrize("shells,mps", [(1057, 50.0), (1058, 50.0), (1089, 5.0), (4513, 10.0), (4514, 10.0), (4544, 2.0),
+                                        (4545, 0.5), (20000, 5.0), (20000, 0.05), (1 << 20, 0.001)])
+def test_split_and_global_tallies(tmc_mod, oracle_mod, shells, mps, block):
+    optics = dict(shells=shells, microns_per_shell=mps, mu_a=2.0, mu_s=20.0)
+    n = 3001
+    tmc_mod.set_plain_launch(block, 0, 0)
+    got, steps = gpu_fx(tmc_mod, n, seed=3, **optics)
+    tmc_mod.set_plain_launch(0, 0, 0)
+    ref, _, ref_steps = oracle_fx(oracle_mod, n, seed=3, **optics)
+    assert steps == ref_steps and np.array_equal(got, ref)

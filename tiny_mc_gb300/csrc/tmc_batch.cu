@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_batch(const BatchArg
         const uint32_t ps = min(a.probe_shell, S - 1);
         const bool probe = a.item_probe || a.done_ring;
         const uint32_t steps = walk_loop<BLOCK, M, SharedSource<BATCH_CHUNK>, Hist::Block>(
-            pr.c, src, a.keys, smem, g, my, probe ? &sh_probe_acc : nullptr,
+            pr.c, src, a.keys, smem, g, my, 0, probe ? &sh_probe_acc : nullptr,
             probe ? &sh_probe_hi : nullptr, ps);
 
         __syncthreads();

@@ -313,6 +313,23 @@ __device__ __forceinline__ void flush128(unsigned long long *g_lo, unsigned long
     }
 }
 
+// A deposit straight into a shell's 128-bit global tally (four words).  Both
+// sums' low words are added before either carry is looked at, so that one
+// atomic's way to the L2 and back hides the other's.
+__device__ __forceinline__ void deposit_global(unsigned long long *gs, float weight)
+{
+    uint32_t l, h;
+    units_split(weight_units(weight), l, h);
+    const unsigned long long v = ((unsigned long long)(h - UNITS_HI_BIAS) << 32) | l;
+    units_split(weight2_units(weight), l, h);
+    const unsigned long long v2 = ((unsigned long long)(h - UNITS_HI_BIAS) << 32) | l;
+    const unsigned long long old = atomicAdd(&gs[0], v), old2 = atomicAdd(&gs[2], v2);
+    if (old + v < old)
+        atomicAdd(&gs[1], 1ull);
+    if (old2 + v2 < old2)
+        atomicAdd(&gs[3], 1ull);
+}
+
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 {
 #pragma unroll

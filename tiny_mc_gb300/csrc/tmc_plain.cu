@@ -9,10 +9,11 @@
 // end.
 // Short walks over not too many shells (params.h's among them) take
 // walk_counts: one count per (step, shell) and block instead of the sums.
-// Shell counts whose histogram does not fit in shared memory at all
-// (params.h's SHELLS is any size in the reference) take the global form:
-// deposits go straight into the 128-bit global tally with 64-bit atomics.  The
-// sums are the same integers in every form.
+// Shell counts whose histogram leaves no room for the SM's blocks (params.h's
+// SHELLS is any size in the reference) take the split form: a histogram of the
+// shells nearest to the source, and 64-bit atomics on the 128-bit global tally
+// beyond them; or, with shells so thin that most deposits land beyond it, no
+// histogram at all.  The sums are the same integers in every form.
 #include <algorithm>
 #include <cmath>
 
@@ -60,13 +61,25 @@ struct PlainArgs {
     uint32_t rows;               // walk_counts: steps with counts
 };
 
+// Shells of the split form's histogram: what 1024 threads per SM (two blocks of
+// 512) leave of its 228 KB beside the rings and each block's own 1 KB.
+__host__ __device__ constexpr uint32_t split_cells(int block)
+{
+    return ((228 * 1024) / (1024 / block) - 1024 - 4 * SLOTS * block) / 16;
+}
+static_assert(split_cells(512) == 4544 && split_cells(128) % 4 == 0, "whole 16-byte rows of the ring behind it");
+
+// Two blocks of 512 threads per SM, three where every deposit waits for the L2
+// (200000 shells of 0.1 um, 2^20 photons: 2.2 ms with two, 1.32 with three).
 template <int BLOCK, class M, Hist H>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArgs a)
+__global__ void __launch_bounds__(BLOCK, (H == Hist::Global ? 1536 : 1024) / BLOCK) walk_plain(const PlainArgs a)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     constexpr bool PER_WARP = H == Hist::Warp;
     const uint32_t S = a.c.shells;
-    const uint32_t hist = H == Hist::Global ? 0u : 4 * hist_cells(S);   // words per histogram
+    const uint32_t near = min(split_cells(BLOCK), S);   // shells of the split form's histogram
+    // words per histogram
+    const uint32_t hist = 4 * (H == Hist::Split ? split_cells(BLOCK) : H == Hist::Global ? 0 : hist_cells(S));
     const uint32_t words = (PER_WARP ? BLOCK / 32 : 1) * hist;
     for (uint32_t s = threadIdx.x; s < words; s += BLOCK)
         smem[s] = 0;
@@ -80,9 +93,14 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArg
     uint32_t *my = smem + words + threadIdx.x;   // ring slot k: my[k * BLOCK]
     uint32_t *tally = PER_WARP ? smem + (threadIdx.x / 32) * hist : smem;
     const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H>(
-        a.c, src, a.keys, tally, a.tally, my);
+        a.c, src, a.keys, tally, a.tally, my, near);
 
-    if constexpr (PER_WARP) {
+    if constexpr (H == Hist::Split) {
+        __syncthreads();
+        const uint32_t part = (near + BLOCK / 32 - 1) / (BLOCK / 32);
+        const uint32_t first = min(threadIdx.x / 32 * part, near);   // this warp's share of the cells
+        warp_flush_cells<false>(smem + first, min(part, near - first), near, a.tally + 4 * (size_t)first);
+    } else if constexpr (PER_WARP) {
         warp_flush_tally<false>(tally, S, a.tally);
     } else if constexpr (H == Hist::Block) {
         __syncthreads();
@@ -192,7 +210,8 @@ static uint32_t count_rows(const Derived &d, size_t smem_optin)
 
 static size_t plain_smem_bytes(uint32_t shells, int block, Hist h)
 {
-    const size_t hist = h == Hist::Global ? 0 : (size_t)16 * hist_cells(shells) * (h == Hist::Warp ? block / 32 : 1);
+    const size_t cells = h == Hist::Split ? split_cells(block) : h == Hist::Global ? 0 : hist_cells(shells);
+    const size_t hist = 16 * cells * (h == Hist::Warp ? block / 32 : 1);
     return hist + (size_t)4 * SLOTS * block;
 }
 
@@ -287,8 +306,31 @@ static cudaError_t launch_counts(const PlainLaunch &L, const DeviceCtx &ctx, uin
                                      : launch_counts_t<ExactMath, TRIP>(L, ctx, rows, stream);
 }
 
+// The split form pays where its histogram reaches far enough: a walk of k steps
+// of about a mean free path ends about sqrt(k) of them out.  With 4544 shells,
+// 2^20 photons and params.h optics (k = 73): shells of 0.4 um (reach 0.47 sqrt(k))
+// 1.74 ms split, 1.47 global; 0.8 um (0.94) 0.99, 1.59; 5 um 0.56, 3.48.  At
+// albedo 0.09 (k = 3): 0.05 um (0.14) 0.207, 0.146; 0.2 um (0.6) 0.156, 0.150;
+// 0.5 um 0.126, 0.168.
+static bool reaches(uint32_t shells, const Derived &d)
+{
+    const double k = d.albedo > 0.0f ? std::log(0.001) / std::log((double)d.albedo) : 0.0;
+    return shells >= 0.6 * d.spm * std::sqrt(1.0 + k);
+}
+
+template <int BLOCK, class M, Hist H>
+static cudaError_t try_launch(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
+{
+    int per_sm = 0;
+    const cudaError_t e = occupancy<BLOCK, M, H>(ctx, plain_smem_bytes(L.d.shells, BLOCK, H), per_sm);
+    return e == cudaSuccess ? launch_t<BLOCK, M, H>(L, ctx, per_sm, stream) : e;
+}
+
 // Per-warp histograms where they fit at the occupancy a per-block histogram
-// would get, else a per-block histogram where it fits, else the global form.
+// would get, a per-block histogram where it leaves the SM its 1024 threads, else
+// the split form (8000 shells of 12.5 um, 2^21 photons of params.h optics: one
+// block per SM 1.26 ms, split 1.02; 20000 shells of 5 um: 5.25 ms global, 1.02
+// split), else global.
 template <int BLOCK, class M>
 static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
@@ -301,13 +343,10 @@ static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStre
         return e;
     if (warp_sm >= 1 && warp_sm >= block_sm)
         return launch_t<BLOCK, M, Hist::Warp>(L, ctx, warp_sm, stream);
-    if (block_sm >= 1)
+    if (block_sm >= 1024 / BLOCK)
         return launch_t<BLOCK, M, Hist::Block>(L, ctx, block_sm, stream);
-    int global_sm = 0;
-    e = occupancy<BLOCK, M, Hist::Global>(ctx, plain_smem_bytes(S, BLOCK, Hist::Global), global_sm);
-    if (e != cudaSuccess)
-        return e;
-    return launch_t<BLOCK, M, Hist::Global>(L, ctx, global_sm, stream);
+    return reaches(split_cells(BLOCK), L.d) ? try_launch<BLOCK, M, Hist::Split>(L, ctx, stream)
+                                            : try_launch<BLOCK, M, Hist::Global>(L, ctx, stream);
 }
 
 template <int BLOCK>
@@ -322,8 +361,9 @@ static cudaError_t load_kernels()
 {
     const void *kernels[] = {
         (const void *)walk_plain<128, M, Hist::Warp>, (const void *)walk_plain<128, M, Hist::Block>,
-        (const void *)walk_plain<128, M, Hist::Global>, (const void *)walk_plain<512, M, Hist::Warp>,
-        (const void *)walk_plain<512, M, Hist::Block>, (const void *)walk_plain<512, M, Hist::Global>,
+        (const void *)walk_plain<128, M, Hist::Split>, (const void *)walk_plain<128, M, Hist::Global>,
+        (const void *)walk_plain<512, M, Hist::Warp>,  (const void *)walk_plain<512, M, Hist::Block>,
+        (const void *)walk_plain<512, M, Hist::Split>, (const void *)walk_plain<512, M, Hist::Global>,
         (const void *)walk_counts<M, TRIP>, (const void *)walk_counts<M, SHORT_TRIP>};
     for (const void *k : kernels) {
         cudaFuncAttributes attr;

@@ -72,11 +72,13 @@ constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the 
 constexpr int WARP_WALK_MAX = 8;
 
 // Where a walk keeps its tallies.  Warp: one shared histogram per warp.
-// Block: one per block, shared by its warps.  Global: none; every deposit is
-// a 64-bit atomic add into the 128-bit global tally (shell counts whose
-// histogram does not fit in shared memory).  Count: one count per (step, shell)
+// Block: one per block, shared by its warps.  Split: a block's histogram holds
+// the shells nearest to the source, where nearly all deposits of a point source
+// land, and a deposit farther out is a 64-bit atomic add into the 128-bit global
+// tally (shell counts whose histogram does not fit in shared memory).  Global:
+// every deposit is (shells so thin that most land beyond such a histogram).  Count: one count per (step, shell)
 // of a block (CountTable).
-enum class Hist { Warp, Block, Global, Count };
+enum class Hist { Warp, Block, Split, Global, Count };
 
 // A warp adds the shared histogram it deposits into (its own, or its block's
 // of `lanes` lanes) into the global tally and clears it every
@@ -129,15 +131,14 @@ __device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *
 // tally at one flush or the next.  probe_acc / probe_hi (shared, may be
 // null): the 128-bit running sum of the w words taken from shell
 // probe_shell.  Warp-collective.  The last shell's cells are added up first
-// (their total obeys the bound below, so it fits 64 bits).
+// (their total obeys the bound below, so it fits 64 bits).  warp_flush_cells:
+// the first n cells only, of planes of C cells.
 template <bool EXCHANGE>
-__device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g,
+__device__ __forceinline__ void warp_flush_cells(uint32_t *tally, uint32_t n, uint32_t C, unsigned long long *g,
                                                  unsigned long long *probe_acc = nullptr,
                                                  uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
 {
-    const uint32_t C = hist_cells(S), lane = threadIdx.x & 31u;
-    __syncwarp();
-    for (uint32_t s = lane; s < S - 1; s += 32) {
+    for (uint32_t s = threadIdx.x & 31u; s < n; s += 32) {
         const unsigned long long v = take_cell<EXCHANGE>(&tally[s], &tally[C + s]);
         flush128(&g[4 * s + 0], &g[4 * s + 1], v);
         if (EXCHANGE && probe_acc && s == probe_shell && v) {
@@ -147,6 +148,16 @@ __device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, un
         }
         flush128(&g[4 * s + 2], &g[4 * s + 3], take_cell<EXCHANGE>(&tally[2 * C + s], &tally[3 * C + s]));
     }
+}
+
+template <bool EXCHANGE>
+__device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g,
+                                                 unsigned long long *probe_acc = nullptr,
+                                                 uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
+{
+    const uint32_t C = hist_cells(S), lane = threadIdx.x & 31u;
+    __syncwarp();
+    warp_flush_cells<EXCHANGE>(tally, S - 1, C, g, probe_acc, probe_hi, probe_shell);
     __syncwarp();
     const uint32_t s = S - 1 + lane;
     const unsigned long long v = warp_sum_u64(take_cell<EXCHANGE>(&tally[s], &tally[C + s]));
@@ -753,19 +764,16 @@ template <class M, Hist H>
 struct WeightTally {
     uint32_t hist;            // shared address of the histogram
     uint32_t plane;           // bytes between a cell's words
-    unsigned long long *g;    // global tally (H = Global)
+    unsigned long long *g;    // global tally (H = Split)
     float albedo;
+    uint32_t near;            // H = Split: shells of the histogram
     uint32_t steps = 0;
 
     __device__ __forceinline__ void deposit(uint32_t cell, float weight)
     {
         uint32_t lo, hi;
-        if constexpr (H == Hist::Global) {
-            unsigned long long *gs = g + 4 * (size_t)cell;
-            units_split(weight_units(weight), lo, hi);
-            flush128(&gs[0], &gs[1], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
-            units_split(weight2_units(weight), lo, hi);
-            flush128(&gs[2], &gs[3], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
+        if (H == Hist::Global || (H == Hist::Split && cell >= near)) {
+            deposit_global(g + 4 * (size_t)cell, weight);
         } else {
             const uint32_t at = hist + 4 * cell;
             units_split(weight_units(weight), lo, hi);
@@ -845,26 +853,21 @@ struct CountTally {
             red_shared_add(at + 4 * cell, 1u);
             return;
         }
-        uint32_t lo, hi;
-        unsigned long long *gs = g + 4 * (size_t)min(cell, last);
-        units_split(weight_units(weight), lo, hi);
-        flush128(&gs[0], &gs[1], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
-        units_split(weight2_units(weight), lo, hi);
-        flush128(&gs[2], &gs[3], ((unsigned long long)(hi - UNITS_HI_BIAS) << 32) | lo);
+        deposit_global(g + 4 * (size_t)min(cell, last), weight);
         ++steps;
     }
 };
 
 // Walk photons from `src` until it is exhausted and every lane's photon has
 // died.  Warp-collective: all 32 lanes of every warp call it.  flush() empties
-// the shared histogram into the global tally; it is called at the latest every
+// the shared tallies into the global one; it is called at the latest every
 // FLUSH iterations.
 template <int BLOCK, class M, bool COUNTS, uint32_t FLUSH, int TRIP, class Source, class Tally, class Flush>
 __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, Source &src, const PhiloxKeys &keys,
                                              uint32_t *my, Tally &tally, Flush flush)
 {
     using R = Ring<BLOCK>;
-    constexpr uint32_t FLUSH_TRIPS = FLUSH / TRIP;   // 0: never
+    constexpr uint32_t FLUSH_TRIPS = FLUSH / TRIP;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
     char *ring = reinterpret_cast<char *>(my);
@@ -909,7 +912,7 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
             __syncwarp();
             saved.save((int)lane, p, tally.weight(p), tally.row_of(p));
             __syncwarp();
-            while (todo && (FLUSH_TRIPS == 0 || trips < FLUSH_TRIPS)) {
+            while (todo && trips < FLUSH_TRIPS) {
                 const int l = __ffs((int)todo) - 1;
                 todo &= todo - 1;
                 WarpPhoton q = saved.get(l);
@@ -922,9 +925,8 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
                     if (lane < n)
                         tally.whole(tally.row_after(row, lane), cell, weight);
                     row = tally.row_after(row, n);
-                    if constexpr (FLUSH_TRIPS != 0)
-                        ++trips;
-                } while (!over && (FLUSH_TRIPS == 0 || trips < FLUSH_TRIPS));
+                    ++trips;
+                } while (!over && trips < FLUSH_TRIPS);
                 if (over)
                     left &= ~(1u << l);
                 else if ((int)lane == l)   // a flush is due first: back to its lane
@@ -949,13 +951,11 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
             if (left != had)
                 continue;
         }
-        if constexpr (FLUSH_TRIPS != 0) {
-            if (trips == FLUSH_TRIPS) {   // a trip stands for TRIP deposits of a lane at most
-                trips = 0;
-                flush();
-            }
-            ++trips;
+        if (trips == FLUSH_TRIPS) {   // a trip stands for TRIP deposits of a lane at most
+            trips = 0;
+            flush();
         }
+        ++trips;
 #pragma unroll
         for (int k = 0; k < TRIP; ++k) {
             if (k % 2 == 0)
@@ -968,23 +968,27 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
 // walk_photons with a shared histogram of 64-bit sums (H = Warp: this warp's;
 // Block: the block's), 4 * hist_cells words (low and high of sum w, then of sum
 // w^2), flushed into g, the problem's global 128-bit tally [shells][4], every
-// flush_steps iterations (the caller flushes what is left), or with none (H =
-// Global).  probe_acc / probe_hi (Block only, may be null): receive the w sums
-// those flushes take from shell probe_shell.  Returns this thread's photon
-// steps.
+// flush_steps iterations (the caller flushes what is left).  H = Split: a block
+// histogram of 4 * near words for the first `near` shells.  probe_acc /
+// probe_hi (Block only, may be null): receive the w sums those flushes take
+// from shell probe_shell.  Returns this thread's photon steps.
 template <int BLOCK, class M, class Source, Hist H>
 __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               const PhiloxKeys &keys, uint32_t *tally,
-                                              unsigned long long *g, uint32_t *my,
+                                              unsigned long long *g, uint32_t *my, uint32_t near = 0,
                                               unsigned long long *probe_acc = nullptr,
                                               uint32_t *probe_hi = nullptr,
                                               uint32_t probe_shell = 0)
 {
-    constexpr uint32_t FLUSH = H == Hist::Global ? 0u : flush_steps(H == Hist::Warp ? 32u : (uint32_t)BLOCK);
-    const float beyond = H == Hist::Global ? c.last : c.last + (float)(threadIdx.x & 31u);
-    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally), 4 * hist_cells(c.shells), g, c.albedo};
+    constexpr uint32_t FLUSH = flush_steps(H == Hist::Warp ? 32u : (uint32_t)BLOCK);
+    constexpr bool FAR = H == Hist::Split || H == Hist::Global;
+    const float beyond = FAR ? c.last : c.last + (float)(threadIdx.x & 31u);
+    const uint32_t cells = H == Hist::Split ? near : hist_cells(c.shells);
+    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally), 4 * cells, g, c.albedo, near};
     walk_photons<BLOCK, M, false, FLUSH, TRIP>(c, beyond, src, keys, my, t, [&] {
-        if constexpr (H != Hist::Global)
+        if constexpr (H == Hist::Split)
+            warp_flush_cells<true>(tally, near, near, g);
+        else if constexpr (H != Hist::Global)
             warp_flush_tally<H == Hist::Block>(tally, c.shells, g, probe_acc, probe_hi, probe_shell);
     });
     return t.steps;
