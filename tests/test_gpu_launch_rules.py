@@ -149,3 +149,12 @@ def test_split_and_global_tallies(tmc_mod, oracle_mod, shells, mps, block):
     tmc_mod.set_plain_launch(0, 0, 0)
     ref, _, ref_steps = oracle_fx(oracle_mod, n, seed=3, **optics)
     assert steps == ref_steps and np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("n", [152 * 256 - 1, 152 * 256, 152 * 256 + 1])
+def test_block_rule_short_walks(tmc_mod, oracle_mod, n):
+    optics = dict(shells=101, microns_per_shell=50.0, mu_a=10.0, mu_s=1.0)
+    tmc_mod.set_plain_launch(0, 0, 0)
+    got, steps = gpu_fx(tmc_mod, n, seed=5, **optics)
+    ref, _, ref_steps = oracle_fx(oracle_mod, n, seed=5, **optics)
+    assert steps == ref_steps and np.array_equal(got, ref)

@@ -328,9 +328,11 @@ static cudaError_t try_launch(const PlainLaunch &L, const DeviceCtx &ctx, cudaSt
 
 // Per-warp histograms where they fit at the occupancy a per-block histogram
 // would get, a per-block histogram where it leaves the SM its 1024 threads, else
-// the split form (8000 shells of 12.5 um, 2^21 photons of params.h optics: one
-// block per SM 1.26 ms, split 1.02; 20000 shells of 5 um: 5.25 ms global, 1.02
-// split), else global.
+// the split form where it reaches (8000 shells of 12.5 um, 2^21 photons of
+// params.h optics: one block per SM 1.26 ms, split 1.02; 20000 shells of 5 um:
+// 5.25 ms global, 1.02 split), else a per-block histogram at any occupancy
+// (4001 shells of 1 um, 5000 photons: 1.2 ms global, 55 us with three blocks
+// of 128 threads per SM), else global.
 template <int BLOCK, class M>
 static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
@@ -345,8 +347,11 @@ static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStre
         return launch_t<BLOCK, M, Hist::Warp>(L, ctx, warp_sm, stream);
     if (block_sm >= 1024 / BLOCK)
         return launch_t<BLOCK, M, Hist::Block>(L, ctx, block_sm, stream);
-    return reaches(split_cells(BLOCK), L.d) ? try_launch<BLOCK, M, Hist::Split>(L, ctx, stream)
-                                            : try_launch<BLOCK, M, Hist::Global>(L, ctx, stream);
+    if (reaches(split_cells(BLOCK), L.d))
+        return try_launch<BLOCK, M, Hist::Split>(L, ctx, stream);
+    if (block_sm >= 1)
+        return launch_t<BLOCK, M, Hist::Block>(L, ctx, block_sm, stream);
+    return try_launch<BLOCK, M, Hist::Global>(L, ctx, stream);
 }
 
 template <int BLOCK>
@@ -378,8 +383,10 @@ cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_
 {
     // 512 threads by default: 512 measured 0.8% faster than 256.  A launch too
     // small to give every SM a block of 512 takes blocks of 128, which spread
-    // the same warps over four times as many SMs.
-    const bool small = L.n_photons < (unsigned long long)ctx.sms * 512;
+    // the same warps over four times as many SMs (70000 photons at albedo 0.09
+    // are not: 64 us with 128-thread blocks, 38 with the counts below).
+    const bool brief = L.d.albedo < SHORT_ALBEDO;   // walks of a few steps: ending a warp's tally costs more
+    const bool small = L.n_photons < (unsigned long long)ctx.sms * (brief ? 256 : 512);
     // a launch of no photons is a caller's set-up call: it loads every kernel
     // a call of its arithmetic may take
     if (L.n_photons == 0 && !L.block) {
