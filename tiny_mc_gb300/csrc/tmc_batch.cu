@@ -93,14 +93,15 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_batch(const BatchArg
             smem[s] = 0;
         __syncthreads();
 
-        SharedSource<BATCH_CHUNK> src;
+        SharedSource src;
         src.counter = &sh_next;
         src.count = item.count;
         src.first = pr.id_base + item.first;
+        src.chunk = pr.claim ? pr.claim : (uint32_t)BATCH_CHUNK;
         unsigned long long *g = a.tally + 4 * pr.tally_offset;
         const uint32_t ps = min(a.probe_shell, S - 1);
         const bool probe = a.item_probe || a.done_ring;
-        const uint32_t steps = walk_loop<BLOCK, M, SharedSource<BATCH_CHUNK>, Hist::Block>(
+        const uint32_t steps = walk_loop<BLOCK, M, SharedSource, Hist::Block>(
             pr.c, src, a.keys, smem, g, my, 0, probe ? &sh_probe_acc : nullptr,
             probe ? &sh_probe_hi : nullptr, ps);
 
@@ -247,6 +248,7 @@ struct tmc_batch {
     int grid = 0;            // resident blocks for the current config (set by plan)
     size_t smem_optin = 0;
     // device buffers
+    std::vector<BatchProblemDev> dev;    // d_problems' contents
     BatchProblemDev *d_problems = nullptr;
     BatchItemDev *d_items = nullptr;
     uint32_t n_items = 0;
@@ -278,13 +280,76 @@ cudaError_t grid_for(const tmc_batch *b, int *grid)
                          : walk_batch_prepare(b->cfg.block, b->math, b->max_shells, b->sms, grid);
 }
 
-// Split problems into items of about equal estimated photon steps.
+// How a batch uses the device: blocks per SM, and from how many expected steps
+// per photon on a problem's photons are walked one to a warp (walk_batch; see
+// warp_steps) instead of one to a lane.
+struct Spread {
+    int per_sm = 1;
+    double whole = 1e300;
+};
+
+// More warps per scheduler walk more steps a second, but each lane takes longer
+// for its own, and a launch ends no earlier than its longest photons' lanes.  A
+// warp walks one photon an order of magnitude faster, at a fifth of the steps a
+// second.  This picks the pair with the shortest estimate.  Measured with w
+// warps per scheduler (fast arithmetic, 152 SMs): 1.70e11 steps/s with 8, 1.32
+// with 4, 1.17 with 3, 0.88 with 2 (the 4096-problem sweep); about 0.65 us a
+// step of one lane with 8, 0.45 with 4, 0.36 with 2; both fitted below.  One
+// photon to a warp: 2.9e10 steps/s, 43 ns a step alone, 0.12 us with 8.
+// 256 problems up to 5.9e4 steps per photon (3.0e9 in all): 8 per scheduler 63
+// ms, 4 47, 3 40, 2 48; 378 up to 1.5e5 (3.5e9): 93, 88, 77, 68; the sweep
+// (6.9e10, up to 6.6e5): 498, 529, 589, 788.  With the longest problems one
+// photon to a warp: 73 problems (9e7 steps, up to 7e4) 7.7 ms against 41 on
+// lanes, 378 55 ms against 68.
+Spread spread(const std::vector<tmc_problem> &problems, const std::vector<double> &est_steps, int block, int most,
+              int sms, uint32_t math, bool stream)
+{
+    std::vector<std::pair<double, double>> p;   // steps per photon and in all, longest first
+    double total = 0.0;
+    for (size_t i = 0; i < problems.size(); ++i)
+        if (problems[i].n_photons) {
+            p.push_back({est_steps[i], est_steps[i] * (double)problems[i].n_photons});
+            total += p.back().second;
+        }
+    Spread best;
+    best.per_sm = most;
+    if (p.empty())
+        return best;
+    std::sort(p.begin(), p.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
+    const double slow = math == TMC_MATH_FAST ? 1.0 : 1.3, size = sms / 152.0;
+    double best_t = 1e300;
+    for (int k = most; k >= 1; --k) {
+        const double w = k * block / 128.0;
+        const double lane_rate = 2.15e11 * size / slow * w / (w + 2.3), lane_step = (0.29 + 0.045 * w) * 1e-6 * slow;
+        const double warp_rate = 2.6e10 * size * std::min(1.0, w / 5.0), warp_step = std::max(0.043e-6, 0.016e-6 * w);
+        double long_work = 0.0;
+        for (size_t i = 0; i <= p.size(); ++i) {   // the i longest problems' photons one to a warp
+            double t = (total - long_work) / lane_rate + long_work / warp_rate;
+            if (i < p.size())
+                t = std::max(t, p[i].first * lane_step);
+            if (i)
+                t = std::max(t, p[0].first * warp_step);
+            if (t < best_t) {
+                best_t = t;
+                best.per_sm = k;
+                best.whole = i ? p[i - 1].first : 1e300;
+            }
+            if (i == p.size() || stream)
+                break;
+            long_work += p[i].second;
+        }
+    }
+    return best;
+}
+
 // Split problems into work items (photon-id ranges) of about equal
 // estimated photon steps for `grid` resident blocks of `block` threads with
 // `items_per_block` items each, heaviest first.  Host only.
+// Problems of `whole` expected steps per photon and more, walked one photon to a
+// warp, get items a fifth of the size, down to a photon per warp, ahead of all.
 std::vector<BatchItemDev> plan_items(const std::vector<tmc_problem> &problems,
                                      const std::vector<double> &est_steps, int grid, int block,
-                                     int items_per_block)
+                                     int items_per_block, double whole = 1e300)
 {
     double total = 0.0;
     for (size_t i = 0; i < problems.size(); ++i)
@@ -302,10 +367,11 @@ std::vector<BatchItemDev> plan_items(const std::vector<tmc_problem> &problems,
         const unsigned long long n = problems[i].n_photons;
         if (n == 0)
             continue;
+        const bool by_warp = est_steps[i] >= whole;
         const unsigned long long min_item =
-            (unsigned long long)block * (2.0 * est_steps[i] <= lane_steps ? 2 : 1);
+            by_warp ? block / 32 : (unsigned long long)block * (2.0 * est_steps[i] <= lane_steps ? 2 : 1);
         const double work = est_steps[i] * (double)n;
-        unsigned long long k = (unsigned long long)std::ceil(work / target);
+        unsigned long long k = (unsigned long long)std::ceil(by_warp ? 5.0 * work / target : work / target);
         k = std::max(1ull, std::min(k, (n + min_item - 1) / min_item));
         k = std::max(k, (n + 0x3fffffffull) / 0x40000000ull);   // counts stay below 2^30
         const unsigned long long per = n / k, extra = n % k;
@@ -320,8 +386,10 @@ std::vector<BatchItemDev> plan_items(const std::vector<tmc_problem> &problems,
             items.push_back({est_steps[i] * (double)c, it});
         }
     }
-    std::stable_sort(items.begin(), items.end(),
-                     [](const auto &x, const auto &y) { return x.first > y.first; });
+    std::stable_sort(items.begin(), items.end(), [&](const auto &x, const auto &y) {
+        const bool xw = est_steps[x.second.problem] >= whole, yw = est_steps[y.second.problem] >= whole;
+        return xw != yw ? xw : x.first > y.first;
+    });
     std::vector<BatchItemDev> h(items.size());
     for (size_t i = 0; i < items.size(); ++i)
         h[i] = items[i].second;
@@ -334,9 +402,11 @@ int plan(tmc_batch *b)
     cudaError_t e = grid_for(b, &grid);   // also sets the kernel's shared-memory limit
     if (e != cudaSuccess)
         return set_cuda_error(e, "batch kernel config");
+    const Spread use = spread(b->problems, b->est_steps, b->cfg.block, grid / b->sms, b->sms, b->math, b->cfg.stream != 0);
+    grid = b->sms * use.per_sm;
     b->grid = grid;
     const std::vector<BatchItemDev> h =
-        plan_items(b->problems, b->est_steps, grid, b->cfg.block, b->cfg.items_per_block);
+        plan_items(b->problems, b->est_steps, grid, b->cfg.block, b->cfg.items_per_block, use.whole);
     if (h.size() > b->items_cap) {
         if (b->d_items)
             cudaFree(b->d_items);
@@ -351,6 +421,17 @@ int plan(tmc_batch *b)
         e = cudaMemcpy(b->d_items, h.data(), sizeof(BatchItemDev) * h.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess)
             return set_cuda_error(e, "cudaMemcpy(batch items)");
+    }
+    bool claims = false;   // claims that differ from the device's
+    for (size_t i = 0; i < b->dev.size(); ++i) {
+        const uint32_t claim = b->est_steps[i] >= use.whole ? 1 : 0;
+        claims = claims || claim != b->dev[i].claim;
+        b->dev[i].claim = claim;
+    }
+    if (claims) {
+        e = cudaMemcpy(b->d_problems, b->dev.data(), sizeof(BatchProblemDev) * b->dev.size(), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess)
+            return set_cuda_error(e, "cudaMemcpy(batch problems)");
     }
     b->n_items = (uint32_t)h.size();
     if (b->graph) {
@@ -533,6 +614,8 @@ int tmc_batch_create(tmc_batch **out, const tmc_problem *problems, uint32_t n_pr
         hp[i].c.spm = d.spm;
         hp[i].c.last = d.last;
         hp[i].c.shells = d.shells;
+        hp[i].claim = 0;
+        hp[i].reserved = 0;
         hp[i].id_base = q.photon_id_base;
         hp[i].tally_offset = b->offsets[i];
         b->offsets[i + 1] = b->offsets[i] + q.shells;
@@ -551,6 +634,7 @@ int tmc_batch_create(tmc_batch **out, const tmc_problem *problems, uint32_t n_pr
         free_batch(b.release());
         return r;
     }
+    b->dev = std::move(hp);
     *out = b.release();
     return TMC_OK;
 }

@@ -9,13 +9,15 @@
 
 namespace tmc {
 
-constexpr int BATCH_CHUNK = 32;   // photon ids a warp claims from its item at once
+constexpr int BATCH_CHUNK = 32;   // photon ids a warp claims from its item at once, if its problem does not say
 
 // The queue-mode control word (BatchArgs::q_mode), written by the host.
 constexpr unsigned QUEUE_HOLD = 0, QUEUE_DRAIN = 1, QUEUE_STOP = 2;
 
 struct BatchProblemDev {
     WalkConsts c;
+    uint32_t claim;                    // walk_batch: photon ids a warp claims at once (0: BATCH_CHUNK)
+    uint32_t reserved;
     unsigned long long id_base;
     unsigned long long tally_offset;   // in shells
 };
@@ -163,6 +165,7 @@ __device__ __forceinline__ bool queue_try_claim(const BatchArgs &a, BatchItemDev
     pr.c.spm = vp->c.spm;
     pr.c.last = vp->c.last;
     pr.c.shells = vp->c.shells;
+    pr.claim = 0;
     pr.id_base = vp->id_base;
     pr.tally_offset = vp->tally_offset;
     qidx = slot;

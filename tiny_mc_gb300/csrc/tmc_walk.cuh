@@ -313,11 +313,11 @@ struct GlobalSource {
 
 // Photon ids from a shared-memory 32-bit counter over one work item of
 // `count` photons starting at id `first`.
-template <int CHUNK>
 struct SharedSource {
     uint32_t *counter;   // shared memory, zero at the start of the item
     uint32_t count;
     unsigned long long first;
+    uint32_t chunk;      // ids per claim (as GlobalSource's)
     uint32_t cnext = 0, cend = 0;
     bool exhausted = false;
 
@@ -332,14 +332,14 @@ struct SharedSource {
             uint32_t base = 0;
             if (!exhausted) {
                 if (lane == 0)
-                    base = atomicAdd(counter, (uint32_t)CHUNK);
+                    base = atomicAdd(counter, chunk);
                 base = __shfl_sync(FULL_MASK, base, 0);
                 exhausted = base >= count;
             }
             if (exhausted) {
                 cnext = cend;
             } else {
-                cend = min(base + (uint32_t)CHUNK, count);
+                cend = min(base + chunk, count);
                 if (!got) {
                     id = base + (rank - take0);
                     got = id < cend;
