@@ -2,11 +2,9 @@
 //
 // Reference path: tiny_mc.c:47-49 calls photon() (photon.c:6-51) once per
 // photon.  Here a persistent grid walks all n photons with the loop in
-// tmc_walk.cuh.  Deposits go into shared-memory histograms of the problem's
-// shells: one per warp where that fits without costing occupancy, else one
-// per block; each is added into the 128-bit global tally every flush_steps
-// iterations (2^18 for a warp's, 2^23 / threads for a block's) and at the
-// end.
+// tmc_walk.cuh.  Deposits go into a block's shared-memory histogram of the
+// problem's shells, added into the 128-bit global tally every flush_steps
+// iterations (2^23 / threads) and at the end.
 // Short walks over not too many shells (params.h's among them) take
 // walk_counts: one count per (step, shell) and block instead of the sums.
 // Shell counts whose histogram leaves no room for the SM's blocks (params.h's
@@ -75,13 +73,11 @@ template <int BLOCK, class M, Hist H>
 __global__ void __launch_bounds__(BLOCK, (H == Hist::Global ? 1536 : 1024) / BLOCK) walk_plain(const PlainArgs a)
 {
     extern __shared__ __align__(16) uint32_t smem[];
-    constexpr bool PER_WARP = H == Hist::Warp;
     const uint32_t S = a.c.shells;
     const uint32_t near = min(split_cells(BLOCK), S);   // shells of the split form's histogram
     // words per histogram
     const uint32_t hist = 4 * (H == Hist::Split ? split_cells(BLOCK) : H == Hist::Global ? 0 : hist_cells(S));
-    const uint32_t words = (PER_WARP ? BLOCK / 32 : 1) * hist;
-    for (uint32_t s = threadIdx.x; s < words; s += BLOCK)
+    for (uint32_t s = threadIdx.x; s < hist; s += BLOCK)
         smem[s] = 0;
     __syncthreads();
 
@@ -90,18 +86,15 @@ __global__ void __launch_bounds__(BLOCK, (H == Hist::Global ? 1536 : 1024) / BLO
     src.n = a.n_photons;
     src.id_base = a.id_base;
     src.chunk = a.chunk;
-    uint32_t *my = smem + words + threadIdx.x;   // ring slot k: my[k * BLOCK]
-    uint32_t *tally = PER_WARP ? smem + (threadIdx.x / 32) * hist : smem;
+    uint32_t *my = smem + hist + threadIdx.x;   // ring slot k: my[k * BLOCK]
     const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H>(
-        a.c, src, a.keys, tally, a.tally, my, near);
+        a.c, src, a.keys, smem, a.tally, my, near);
 
     if constexpr (H == Hist::Split) {
         __syncthreads();
         const uint32_t part = (near + BLOCK / 32 - 1) / (BLOCK / 32);
         const uint32_t first = min(threadIdx.x / 32 * part, near);   // this warp's share of the cells
         warp_flush_cells<false>(smem + first, min(part, near - first), near, a.tally + 4 * (size_t)first);
-    } else if constexpr (PER_WARP) {
-        warp_flush_tally<false>(tally, S, a.tally);
     } else if constexpr (H == Hist::Block) {
         __syncthreads();
         flush_tally<BLOCK>(smem, S, a.tally);
@@ -211,8 +204,7 @@ static uint32_t count_rows(const Derived &d, size_t smem_optin)
 static size_t plain_smem_bytes(uint32_t shells, int block, Hist h)
 {
     const size_t cells = h == Hist::Split ? split_cells(block) : h == Hist::Global ? 0 : hist_cells(shells);
-    const size_t hist = 16 * cells * (h == Hist::Warp ? block / 32 : 1);
-    return hist + (size_t)4 * SLOTS * block;
+    return 16 * cells + (size_t)4 * SLOTS * block;
 }
 
 template <int BLOCK, class M, Hist H>
@@ -326,25 +318,19 @@ static cudaError_t try_launch(const PlainLaunch &L, const DeviceCtx &ctx, cudaSt
     return e == cudaSuccess ? launch_t<BLOCK, M, H>(L, ctx, per_sm, stream) : e;
 }
 
-// Per-warp histograms where they fit at the occupancy a per-block histogram
-// would get, a per-block histogram where it leaves the SM its 1024 threads, else
-// the split form where it reaches (8000 shells of 12.5 um, 2^21 photons of
-// params.h optics: one block per SM 1.26 ms, split 1.02; 20000 shells of 5 um:
-// 5.25 ms global, 1.02 split), else a per-block histogram at any occupancy
-// (4001 shells of 1 um, 5000 photons: 1.2 ms global, 55 us with three blocks
+// A histogram per block where it leaves the SM its 1024 threads, else the split
+// form where it reaches (8000 shells of 12.5 um, 2^21 photons of params.h
+// optics: one block per SM 1.26 ms, split 1.02; 20000 shells of 5 um: 5.25 ms
+// global, 1.02 split), else a block's histogram at any occupancy (4001 shells of 1 um, 5000 photons: 1.2 ms global, 55 us with three blocks
 // of 128 threads per SM), else global.
 template <int BLOCK, class M>
 static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
     const uint32_t S = L.d.shells;
-    int warp_sm = 0, block_sm = 0;
-    cudaError_t e = occupancy<BLOCK, M, Hist::Warp>(ctx, plain_smem_bytes(S, BLOCK, Hist::Warp), warp_sm);
-    if (e == cudaSuccess)
-        e = occupancy<BLOCK, M, Hist::Block>(ctx, plain_smem_bytes(S, BLOCK, Hist::Block), block_sm);
+    int block_sm = 0;
+    const cudaError_t e = occupancy<BLOCK, M, Hist::Block>(ctx, plain_smem_bytes(S, BLOCK, Hist::Block), block_sm);
     if (e != cudaSuccess)
         return e;
-    if (warp_sm >= 1 && warp_sm >= block_sm)
-        return launch_t<BLOCK, M, Hist::Warp>(L, ctx, warp_sm, stream);
     if (block_sm >= 1024 / BLOCK)
         return launch_t<BLOCK, M, Hist::Block>(L, ctx, block_sm, stream);
     if (reaches(split_cells(BLOCK), L.d))
@@ -365,10 +351,9 @@ template <class M>
 static cudaError_t load_kernels()
 {
     const void *kernels[] = {
-        (const void *)walk_plain<128, M, Hist::Warp>, (const void *)walk_plain<128, M, Hist::Block>,
-        (const void *)walk_plain<128, M, Hist::Split>, (const void *)walk_plain<128, M, Hist::Global>,
-        (const void *)walk_plain<512, M, Hist::Warp>,  (const void *)walk_plain<512, M, Hist::Block>,
-        (const void *)walk_plain<512, M, Hist::Split>, (const void *)walk_plain<512, M, Hist::Global>,
+        (const void *)walk_plain<128, M, Hist::Block>,  (const void *)walk_plain<128, M, Hist::Split>,
+        (const void *)walk_plain<128, M, Hist::Global>, (const void *)walk_plain<512, M, Hist::Block>,
+        (const void *)walk_plain<512, M, Hist::Split>,  (const void *)walk_plain<512, M, Hist::Global>,
         (const void *)walk_counts<M, TRIP>, (const void *)walk_counts<M, SHORT_TRIP>};
     for (const void *k : kernels) {
         cudaFuncAttributes attr;
@@ -381,12 +366,19 @@ static cudaError_t load_kernels()
 
 cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
-    // 512 threads by default: 512 measured 0.8% faster than 256.  A launch too
-    // small to give every SM a block of 512 takes blocks of 128, which spread
-    // the same warps over four times as many SMs (70000 photons at albedo 0.09
-    // are not: 64 us with 128-thread blocks, 38 with the counts below).
-    const bool brief = L.d.albedo < SHORT_ALBEDO;   // walks of a few steps: ending a warp's tally costs more
-    const bool small = L.n_photons < (unsigned long long)ctx.sms * (brief ? 256 : 512);
+    // Counts instead of sums wherever their table fits and the launch fills the
+    // device: 2^24 photons of params.h optics 7.63 -> 6.86 ms, 2^25 in exact
+    // arithmetic 20.0 -> 18.4 ms, 2^22 at albedo 0.09 0.25 -> 0.15 ms.  In smaller
+    // launches setting the table up and adding it costs more: 100000 photons 125
+    // us against 100, 131072 127 against 118, 155000 128 against 130; at albedo
+    // 0.09 70000 photons 38 against 64.
+    const unsigned long long per_sm = L.n_photons / (unsigned)ctx.sms;
+    const bool fill = per_sm >= (L.d.albedo < SHORT_ALBEDO ? 256 : 900);
+    // Sums take blocks of 128 threads where eight histograms fit an SM: they
+    // spread small launches over more SMs (32768 photons on 64 blocks of 512
+    // took 114 us, 84 on 256 of 128) and end one by one (2^18 high-albedo
+    // photons 13.3 -> 12.5 ms).  More shells take them below 512 photons per SM.
+    const bool blocks128 = hist_cells(L.d.shells) <= split_cells(128) || per_sm < 512;
     // a launch of no photons is a caller's set-up call: it loads every kernel
     // a call of its arithmetic may take
     if (L.n_photons == 0 && !L.block) {
@@ -394,17 +386,12 @@ cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_
         if (e != cudaSuccess)
             return e;
     }
-    // Counts instead of sums wherever their table fits: 2^24 photons of params.h
-    // optics 7.63 -> 6.86 ms, 2^25 in exact arithmetic 20.0 -> 18.4 ms, 2^22 at
-    // albedo 0.09 0.25 -> 0.15 ms, 131072 159 -> 126 us.  Not in small launches,
-    // where setting the table up and adding it costs more (32768 photons 98 us
-    // against 83).
-    if (L.block == 0 && !small) {
+    if (L.block == 0 && fill) {
         const uint32_t rows = count_rows(L.d, ctx.smem_optin);
         if (rows)
             return launch_counts(L, ctx, rows, stream);
     }
-    switch (L.block ? L.block : small ? 128 : 512) {
+    switch (L.block ? L.block : blocks128 ? 128 : 512) {
     case 128: return launch_b<128>(L, ctx, stream);
     case 256: return launch_b<256>(L, ctx, stream);
     case 512: return launch_b<512>(L, ctx, stream);

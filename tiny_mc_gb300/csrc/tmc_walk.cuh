@@ -28,10 +28,9 @@
 //  * the two tallies of photon.c:30-31 go into a shared-memory histogram of
 //    64-bit fixed-point sums (sum of w and of w^2, 2^-40 units), each kept as
 //    two 32-bit words updated with native 32-bit shared atomics (a 64-bit
-//    shared atomicAdd is a compare-and-swap loop, 4x slower here).  The
-//    histogram is one per warp (the plain kernel, where that fits) or one per
-//    block; either way a warp adds it into the 128-bit global tally and clears
-//    it every flush_steps iterations, which keeps its 64-bit sums from
+//    shared atomicAdd is a compare-and-swap loop, 4x slower here).  Each warp
+//    adds the block's histogram into the 128-bit global tally and clears it
+//    every flush_steps iterations, which keeps its 64-bit sums from
 //    wrapping, so a deposit needs no wrap check.
 //
 // What bounds it: instruction issue, then the shared-memory pipe.  One photon
@@ -71,18 +70,18 @@ constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the 
 // reduced scale: 788 ms without, 608 (6), 619 (10), 615 (16), 812 ms (24).
 constexpr int WARP_WALK_MAX = 8;
 
-// Where a walk keeps its tallies.  Warp: one shared histogram per warp.
-// Block: one per block, shared by its warps.  Split: a block's histogram holds
+// Where a walk keeps its tallies.  Block: a shared histogram per block (one per
+// warp, which the plain walk once had, measured the same at 2^18 photons and
+// more and costs small launches more flushes: 75000 photons 127 us against 96).  Split: a block's histogram holds
 // the shells nearest to the source, where nearly all deposits of a point source
 // land, and a deposit farther out is a 64-bit atomic add into the 128-bit global
 // tally (shell counts whose histogram does not fit in shared memory).  Global:
 // every deposit is (shells so thin that most land beyond such a histogram).  Count: one count per (step, shell)
 // of a block (CountTable).
-enum class Hist { Warp, Block, Split, Global, Count };
+enum class Hist { Block, Split, Global, Count };
 
-// A warp adds the shared histogram it deposits into (its own, or its block's
-// of `lanes` lanes) into the global tally and clears it every
-// flush_steps(lanes) of its iterations.  A lane deposits at most once per
+// A warp adds its block's histogram, of `lanes` lanes, into the global tally and
+// clears it every flush_steps(lanes) of its iterations.  A lane deposits at most once per
 // iteration, so between two flushes, whichever warps make them, every lane
 // deposits at most flush_steps times (its warp would have flushed).  A deposit
 // adds at most 2^8 + 1 to a high word (w <= 1, plus the low word's carry), so
@@ -93,7 +92,6 @@ __host__ __device__ constexpr uint32_t flush_steps(uint32_t lanes)
     return (1u << 23) / lanes;
 }
 static_assert(512ull * 257ull * ((1ull << 23) / 512 + 1) < (1ull << 32), "high word bound");
-static_assert(32ull * 257ull * ((1ull << 23) / 32 + 1) < (1ull << 32), "high word bound");
 
 // Cells of a shared histogram.  Every photon beyond the last shell deposits
 // into it (photon.c:27-29): in an optically thin problem nearly all lanes of a
@@ -123,9 +121,9 @@ __device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *
 }
 
 // Add a histogram into the 128-bit global tally and clear it.
-// EXCHANGE = false: a warp's own histogram.  EXCHANGE = true: a block's, by one
-// warp while the others keep depositing: every word is taken with an atomic
-// exchange against zero.  Sums stay exact: a deposit's low-word overflow is
+// EXCHANGE = false: after a barrier.  EXCHANGE = true: by one warp while the
+// others keep depositing: every word is taken with an atomic exchange against
+// zero.  Sums stay exact: a deposit's low-word overflow is
 // carried into a high word by the depositing lane, whichever side of an
 // exchange either add lands on, and every word's content reaches the global
 // tally at one flush or the next.  probe_acc / probe_hi (shared, may be
@@ -150,22 +148,21 @@ __device__ __forceinline__ void warp_flush_cells(uint32_t *tally, uint32_t n, ui
     }
 }
 
-template <bool EXCHANGE>
 __device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g,
                                                  unsigned long long *probe_acc = nullptr,
                                                  uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
 {
     const uint32_t C = hist_cells(S), lane = threadIdx.x & 31u;
     __syncwarp();
-    warp_flush_cells<EXCHANGE>(tally, S - 1, C, g, probe_acc, probe_hi, probe_shell);
+    warp_flush_cells<true>(tally, S - 1, C, g, probe_acc, probe_hi, probe_shell);
     __syncwarp();
     const uint32_t s = S - 1 + lane;
-    const unsigned long long v = warp_sum_u64(take_cell<EXCHANGE>(&tally[s], &tally[C + s]));
-    const unsigned long long v2 = warp_sum_u64(take_cell<EXCHANGE>(&tally[2 * C + s], &tally[3 * C + s]));
+    const unsigned long long v = warp_sum_u64(take_cell<true>(&tally[s], &tally[C + s]));
+    const unsigned long long v2 = warp_sum_u64(take_cell<true>(&tally[2 * C + s], &tally[3 * C + s]));
     if (lane == 0) {
         unsigned long long *gl = g + 4 * (size_t)(S - 1);
         flush128(&gl[0], &gl[1], v);
-        if (EXCHANGE && probe_acc && S - 1 == probe_shell && v) {
+        if (probe_acc && S - 1 == probe_shell && v) {
             const unsigned long long old = atomicAdd(probe_acc, v);
             if (old + v < old)
                 atomicAdd(probe_hi, 1u);
@@ -965,8 +962,7 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
     }
 }
 
-// walk_photons with a shared histogram of 64-bit sums (H = Warp: this warp's;
-// Block: the block's), 4 * hist_cells words (low and high of sum w, then of sum
+// walk_photons with a block's histogram of 64-bit sums, 4 * hist_cells words (low and high of sum w, then of sum
 // w^2), flushed into g, the problem's global 128-bit tally [shells][4], every
 // flush_steps iterations (the caller flushes what is left).  H = Split: a block
 // histogram of 4 * near words for the first `near` shells.  probe_acc /
@@ -980,7 +976,7 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               uint32_t *probe_hi = nullptr,
                                               uint32_t probe_shell = 0)
 {
-    constexpr uint32_t FLUSH = flush_steps(H == Hist::Warp ? 32u : (uint32_t)BLOCK);
+    constexpr uint32_t FLUSH = flush_steps((uint32_t)BLOCK);
     constexpr bool FAR = H == Hist::Split || H == Hist::Global;
     const float beyond = FAR ? c.last : c.last + (float)(threadIdx.x & 31u);
     const uint32_t cells = H == Hist::Split ? near : hist_cells(c.shells);
@@ -989,7 +985,7 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
         if constexpr (H == Hist::Split)
             warp_flush_cells<true>(tally, near, near, g);
         else if constexpr (H != Hist::Global)
-            warp_flush_tally<H == Hist::Block>(tally, c.shells, g, probe_acc, probe_hi, probe_shell);
+            warp_flush_tally(tally, c.shells, g, probe_acc, probe_hi, probe_shell);
     });
     return t.steps;
 }
