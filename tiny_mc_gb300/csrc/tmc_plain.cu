@@ -30,18 +30,20 @@ namespace tmc {
 // photons ran on 8 of 152 SMs (695 us against 167).
 //
 // Small launches: one photon, which the whole warp then walks (warp_steps).
-// With k steps to the first roulette that costs about n (k / 32 + 4) rounds
-// of 730 warp-instructions on the launch's schedulers, while on lanes it takes
-// the latency of k iterations whatever n.  Measured, lanes -> whole warps:
-// params.h optics (k = 73) 5000 photons 73 -> 67 us, 12000 75 -> 145 us; high
-// albedo (k = 6905) 4099 photons 4.2 -> 1.0 ms, 12000 4.3 -> 2.3 ms, 24000
-// 4.7 -> 4.7 ms.
+// With k steps to the first roulette that costs about n (k / 32 + 1.4) rounds
+// on the launch's schedulers, while on lanes it takes the latency of k
+// iterations whatever n (exact arithmetic's are the longer).  Measured equal at
+// about 11000 photons of params.h optics (k = 73) in fast arithmetic and 14000
+// in exact, 17500 and 22000 at k = 342, 18000 and 24000 of high albedo (k =
+// 6905); at half of that one to a warp takes 0.7 of the time (6000 photons of
+// params.h optics 45 us against 61, 9000 of high albedo 1.8 ms against 3.1).
 constexpr unsigned MIN_CHUNK = 32, MAX_CHUNK = 256;
 
-static unsigned claim_chunk(unsigned long long n_photons, unsigned long long warps, int sms, float albedo)
+static unsigned claim_chunk(unsigned long long n_photons, unsigned long long warps, int sms, float albedo,
+                            bool exact)
 {
     const double k = albedo > 0.0f ? std::log(0.001) / std::log((double)albedo) : 0.0;
-    if ((double)n_photons < 28.0 * 4 * sms * k / (k + 128.0))
+    if ((double)n_photons < (exact ? 38.0 : 30.0) * 4 * sms * k / (k + 45.0))
         return 1;
     const unsigned long long share = n_photons / (4 * warps) / MIN_CHUNK * MIN_CHUNK;
     return (unsigned)std::max<unsigned long long>(MIN_CHUNK, std::min<unsigned long long>(MAX_CHUNK, share));
@@ -235,7 +237,7 @@ static unsigned plain_args(const PlainLaunch &L, const DeviceCtx &ctx, int block
         per_sm = std::min(per_sm, L.blocks_per_sm);
     unsigned long long grid = (unsigned long long)ctx.sms * per_sm;
     // no more blocks than there are photon chunks to hand out
-    a.chunk = claim_chunk(L.n_photons, grid * (block / 32), ctx.sms, L.d.albedo);
+    a.chunk = claim_chunk(L.n_photons, grid * (block / 32), ctx.sms, L.d.albedo, L.p->math == TMC_MATH_EXACT);
     const unsigned long long warps_needed = (L.n_photons + a.chunk - 1) / a.chunk;
     const unsigned long long blocks_needed = (warps_needed + block / 32 - 1) / (block / 32);
     grid = std::max(1ull, std::min(grid, blocks_needed));
