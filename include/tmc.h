@@ -16,7 +16,7 @@
  * Thread safety: like photon() (global rand, unsynchronised +=), the library
  * is meant to be driven by one host thread at a time per process; calls are
  * serialised by an internal lock so concurrent calls are safe but not
- * concurrent.  Device scratch the library owns is ordered on the GPU as well:
+ * concurrent.  Device scratch the library shares is ordered on the GPU as well:
  * an asynchronous call that uses it (tmc_photon_batch_device with no
  * workspace) finishes on the GPU before any later call touches it.
  */
@@ -110,10 +110,10 @@ size_t tmc_workspace_bytes(void);
  * Device-resident form: d_tally is DEVICE memory [p->shells] and is added to
  * (+=).  d_steps (device, may be NULL) += photon steps.  d_workspace is
  * device scratch of tmc_workspace_bytes() bytes, or NULL to use a buffer the
- * library allocates once per device.  That shared buffer is also the one the
- * host-array calls use: every use of it, on any stream, first waits on the
- * GPU for the previous use to end, so calls with NULL on different streams
- * run one after another (bring a workspace per stream to overlap them).
+ * library allocates once per device.  Every use of that buffer, on any stream,
+ * first waits on the GPU for the previous use to end, so calls with NULL on
+ * different streams run one after another (bring a workspace per stream to
+ * overlap them).
  * Under stream capture that ordering is not recorded: pass a workspace when
  * capturing.  stream is a cudaStream_t (NULL = legacy default stream).
  * Asynchronous: returns after the launch.

@@ -1,9 +1,10 @@
 // tmc_api.cu — the C ABI (include/tmc.h): validation, per-device resources,
 // the drop-in photon_batch entry points and the FP64 finalisation kernel.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
-#include <vector>
 
 #include "tmc_device.cuh"
 #include "tmc_internal.h"
@@ -141,29 +142,54 @@ cudaError_t ws_release(DeviceCtx &c, cudaStream_t stream)
     return cudaEventRecord(c.ws_done, stream);
 }
 
-static int ensure_buffers(DeviceCtx &c, uint32_t shells)
+cudaError_t CallBuffers::device(size_t bytes, size_t keep)
 {
-    if (c.tally_cap < shells) {
-        if (c.tally)
-            cudaFree(c.tally);
-        c.tally = nullptr;
-        c.tally_cap = 0;
-        cudaError_t e = cudaMalloc(&c.tally, sizeof(tmc_tally) * shells);
-        if (e != cudaSuccess)
-            return set_cuda_error(e, "cudaMalloc(tally)");
-        c.tally_cap = shells;
+    if (bytes > keep) {
+        const cudaError_t e = cudaMalloc(&dev, bytes);
+        own_dev = e == cudaSuccess;
+        return e;
     }
-    if (c.out_cap < shells) {
-        if (c.heat_out)
-            cudaFree(c.heat_out);
-        c.heat_out = nullptr;
-        c.out_cap = 0;
-        cudaError_t e = cudaMalloc(&c.heat_out, sizeof(double) * 2 * shells);
+    if (bytes > ctx.scratch_cap) {
+        cudaFree(ctx.scratch);   // waits for earlier work
+        ctx.scratch = nullptr;
+        ctx.scratch_cap = 0;
+        const size_t want = std::min(keep, std::max<size_t>(bytes + bytes / 2, 16384));
+        const cudaError_t e = cudaMalloc(&ctx.scratch, want);
         if (e != cudaSuccess)
-            return set_cuda_error(e, "cudaMalloc(heat)");
-        c.out_cap = shells;
+            return e;
+        ctx.scratch_cap = want;
     }
-    return TMC_OK;
+    dev = static_cast<char *>(ctx.scratch);
+    return cudaSuccess;
+}
+
+cudaError_t CallBuffers::host(size_t bytes)
+{
+    if (bytes > PINNED_KEEP) {
+        pin = static_cast<char *>(std::malloc(bytes));
+        own_pin = pin != nullptr;
+        return pin ? cudaSuccess : cudaErrorMemoryAllocation;
+    }
+    if (bytes > ctx.pinned_cap) {
+        cudaFreeHost(ctx.pinned);
+        ctx.pinned = nullptr;
+        ctx.pinned_cap = 0;
+        const size_t want = std::min(PINNED_KEEP, std::max<size_t>(bytes + bytes / 2, 16384));
+        const cudaError_t e = cudaMallocHost(&ctx.pinned, want);
+        if (e != cudaSuccess)
+            return e;
+        ctx.pinned_cap = want;
+    }
+    pin = static_cast<char *>(ctx.pinned);
+    return cudaSuccess;
+}
+
+CallBuffers::~CallBuffers()
+{
+    if (own_dev)
+        cudaFree(dev);   // waits for the call's work
+    if (own_pin)
+        std::free(pin);
 }
 
 __global__ void tally_to_heat_kernel(const tmc_tally *t, uint32_t shells, double c, double *heat,
@@ -219,18 +245,28 @@ cudaError_t launch_tally_to_heat(const tmc_tally *d_tally, uint32_t shells, doub
     return cudaGetLastError();
 }
 
-// Shared part of the host-array entry points: walk into ctx.tally.
-static int run_into_ctx_tally(DeviceCtx &c, uint64_t n, const tmc_params *p, const Derived &d,
-                              unsigned long long *d_steps)
+// Shared part of the host-array entry points.  Device scratch: claim and step
+// counters (WORKSPACE_BYTES), the tallies, then FP64 heat and heat2; the walk
+// fills the tallies and the step counter.
+struct HostWalk {
+    tmc_tally *tally;
+    unsigned long long *steps;
+    double *heat;
+};
+
+static int walk_into(CallBuffers &buf, DeviceCtx &c, uint64_t n, const tmc_params *p, const Derived &d, bool steps,
+                     size_t pinned, HostWalk &w)
 {
-    int st = ensure_buffers(c, p->shells);
-    if (st)
-        return st;
-    cudaError_t e = cudaMemsetAsync(c.tally, 0, sizeof(tmc_tally) * p->shells, c.stream);
+    const size_t S = p->shells;
+    cudaError_t e = buf.device(WORKSPACE_BYTES + (sizeof(tmc_tally) + 2 * sizeof(double)) * S, WALK_KEEP);
     if (e == cudaSuccess)
-        e = ws_acquire(c, c.stream);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(c.workspace, 0, WORKSPACE_BYTES, c.stream);
+        e = buf.host(pinned);
+    if (e != cudaSuccess)
+        return set_cuda_error(e, "host-array call's buffers");
+    w.tally = reinterpret_cast<tmc_tally *>(buf.dev + WORKSPACE_BYTES);
+    w.steps = reinterpret_cast<unsigned long long *>(buf.dev) + 1;
+    w.heat = reinterpret_cast<double *>(buf.dev + WORKSPACE_BYTES + sizeof(tmc_tally) * S);
+    e = cudaMemsetAsync(buf.dev, 0, WORKSPACE_BYTES + sizeof(tmc_tally) * S, c.stream);
     if (e != cudaSuccess)
         return set_cuda_error(e, "cudaMemsetAsync");
     if (n == 0)
@@ -239,9 +275,9 @@ static int run_into_ctx_tally(DeviceCtx &c, uint64_t n, const tmc_params *p, con
     L.p = p;
     L.d = d;
     L.n_photons = n;
-    L.d_tally = c.tally;
-    L.d_work = reinterpret_cast<unsigned long long *>(c.workspace);
-    L.d_steps = d_steps;
+    L.d_tally = w.tally;
+    L.d_work = reinterpret_cast<unsigned long long *>(buf.dev);
+    L.d_steps = steps ? w.steps : nullptr;
     L.block = g_plain_block;
     L.blocks_per_sm = g_plain_blocks_per_sm;
     L.max_blocks = g_plain_max_blocks;
@@ -249,13 +285,6 @@ static int run_into_ctx_tally(DeviceCtx &c, uint64_t n, const tmc_params *p, con
     if (e != cudaSuccess)
         return set_cuda_error(e, "walk_plain launch");
     return TMC_OK;
-}
-
-// After the host-array calls' reads of the step counter.
-static int release_ctx_workspace(DeviceCtx &c)
-{
-    const cudaError_t e = ws_release(c, c.stream);
-    return e == cudaSuccess ? TMC_OK : set_cuda_error(e, "cudaEventRecord(workspace)");
 }
 
 static int check_sizes(uint64_t n, const tmc_params *p)
@@ -317,21 +346,21 @@ int tmc_photon_batch_fx(tmc_tally *tally, uint64_t n_photons, const tmc_params *
     if ((st = check_sizes(n_photons, p)))
         return st;
     const Derived d = derive(p->mu_a, p->mu_s, p->microns_per_shell, p->shells);
-    unsigned long long *d_steps = reinterpret_cast<unsigned long long *>(c->workspace) + 1;
-    if ((st = run_into_ctx_tally(*c, n_photons, p, d, d_steps)))
+    // results in pinned memory: the step count, then the tallies
+    const size_t bytes = sizeof(tmc_tally) * (size_t)p->shells;
+    CallBuffers buf(*c);
+    HostWalk w{};
+    if ((st = walk_into(buf, *c, n_photons, p, d, true, 64 + bytes, w)))
         return st;
-    std::vector<tmc_tally> h(p->shells);
-    unsigned long long steps = 0;
-    cudaError_t e = cudaMemcpyAsync(h.data(), c->tally, sizeof(tmc_tally) * p->shells,
-                                    cudaMemcpyDeviceToHost, c->stream);
+    const tmc_tally *h = reinterpret_cast<const tmc_tally *>(buf.pin + 64);
+    cudaError_t e = cudaMemcpyAsync(buf.pin + 64, w.tally, bytes, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&steps, d_steps, sizeof steps, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess && (st = release_ctx_workspace(*c)))
-        return st;
+        e = cudaMemcpyAsync(buf.pin, w.steps, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess)
         return set_cuda_error(e, "tmc_photon_batch_fx");
+    const uint64_t steps = *reinterpret_cast<const uint64_t *>(buf.pin);
     for (uint32_t s = 0; s < p->shells; ++s) {
         unsigned __int128 a = ((unsigned __int128)tally[s].w_hi << 64) | tally[s].w_lo;
         unsigned __int128 b = ((unsigned __int128)tally[s].w2_hi << 64) | tally[s].w2_lo;
@@ -362,17 +391,16 @@ int tmc_photon_batch(float *heat, float *heat2, uint64_t n_photons, const tmc_pa
     if ((st = check_sizes(n_photons, p)))
         return st;
     const Derived d = derive(p->mu_a, p->mu_s, p->microns_per_shell, p->shells);
-    if ((st = run_into_ctx_tally(*c, n_photons, p, d, nullptr)))
-        return st;
-    if ((st = release_ctx_workspace(*c)))
-        return st;
     const uint32_t S = p->shells;
-    cudaError_t e = launch_tally_to_heat(c->tally, S, (double)d.c, c->heat_out, c->heat_out + S,
-                                         c->stream);
-    std::vector<double> h(2 * (size_t)S);
+    const size_t bytes = 2 * sizeof(double) * (size_t)S;
+    CallBuffers buf(*c);
+    HostWalk w{};
+    if ((st = walk_into(buf, *c, n_photons, p, d, false, bytes, w)))
+        return st;
+    const double *h = reinterpret_cast<const double *>(buf.pin);
+    cudaError_t e = launch_tally_to_heat(w.tally, S, (double)d.c, w.heat, w.heat + S, c->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(h.data(), c->heat_out, sizeof(double) * 2 * S, cudaMemcpyDeviceToHost,
-                            c->stream);
+        e = cudaMemcpyAsync(buf.pin, w.heat, bytes, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess)
@@ -452,25 +480,24 @@ int tmc_report_fp64(const tmc_tally *tally, const tmc_params *p, uint64_t photon
     DeviceCtx *c = current_ctx(&st);
     if (!c)
         return st;
-    if ((st = ensure_buffers(*c, p->shells)))
-        return st;
     const uint32_t S = p->shells;
-    double *d_out = nullptr;
-    cudaError_t e = cudaMallocAsync(&d_out, sizeof(double) * (2 * S + 1), c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->tally, tally, sizeof(tmc_tally) * S, cudaMemcpyHostToDevice, c->stream);
+    CallBuffers buf(*c);
+    cudaError_t e = buf.device(sizeof(tmc_tally) * (size_t)S + sizeof(double) * (2 * (size_t)S + 1), WALK_KEEP);
+    if (e != cudaSuccess)
+        return set_cuda_error(e, "tmc_report_fp64");
+    tmc_tally *d_tally = reinterpret_cast<tmc_tally *>(buf.dev);
+    double *d_out = reinterpret_cast<double *>(buf.dev + sizeof(tmc_tally) * (size_t)S);
+    e = cudaMemcpyAsync(d_tally, tally, sizeof(tmc_tally) * S, cudaMemcpyHostToDevice, c->stream);
     const Derived d = derive(p->mu_a, p->mu_s, p->microns_per_shell, S);
     if (e == cudaSuccess)
-        e = launch_report_fp64(c->tally, S, (double)d.c, (double)p->microns_per_shell, (double)photons,
-                               d_out, c->stream);
+        e = launch_report_fp64(d_tally, S, (double)d.c, (double)p->microns_per_shell, (double)photons, d_out,
+                               c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(density, d_out, sizeof(double) * (S - 1), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(error, d_out + S, sizeof(double) * (S - 1), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(extra, d_out + 2 * S, sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    if (d_out)
-        cudaFreeAsync(d_out, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
     return e == cudaSuccess ? TMC_OK : set_cuda_error(e, "tmc_report_fp64");

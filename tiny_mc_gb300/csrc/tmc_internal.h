@@ -42,10 +42,14 @@ struct DeviceCtx {
     int cc_major = 0, cc_minor = 0;
     size_t smem_optin = 0;
     void *workspace = nullptr;          // tmc_workspace_bytes()
-    tmc_tally *tally = nullptr;         // tally_cap shells
-    size_t tally_cap = 0;
-    double *heat_out = nullptr;         // 2 * out_cap doubles
-    size_t out_cap = 0;
+    // The host-array calls' own buffers, used under the library's lock on
+    // `stream` and finished when a call returns: device scratch, grown to the
+    // largest call so far, and pinned host memory for results, each up to a
+    // bound (a larger call's is its own).
+    void *scratch = nullptr;
+    size_t scratch_cap = 0;
+    void *pinned = nullptr;
+    size_t pinned_cap = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ws_done = nullptr;      // recorded after the last use of workspace
 };
@@ -59,9 +63,29 @@ void set_error_text(const std::string &s);
 
 constexpr size_t WORKSPACE_BYTES = 256;
 
+// Device scratch and pinned memory for the length of one host-array call.  Kept
+// by the context up to a bound: allocating and freeing them in each call took
+// 140 us of a colour map's 205 (800 x 800) and 6 of a 20-photon call's 39 (stream-ordered
+// memory goes back to the driver at every synchronisation).
+// Bounds: the tallies and results of the largest walk (2^24 shells), images of
+// 64 MB, 4 MB of pinned memory (results beyond come through pageable memory).
+constexpr size_t WALK_KEEP = 1u << 30, IMAGE_KEEP = 64u << 20, PINNED_KEEP = 4u << 20;
+struct CallBuffers {
+    explicit CallBuffers(DeviceCtx &c) : ctx(c) {}
+    ~CallBuffers();
+    CallBuffers(const CallBuffers &) = delete;
+    CallBuffers &operator=(const CallBuffers &) = delete;
+    cudaError_t device(size_t bytes, size_t keep);   // once; sets dev
+    cudaError_t host(size_t bytes);                  // once; sets pin
+    DeviceCtx &ctx;
+    char *dev = nullptr;
+    char *pin = nullptr;
+    bool own_dev = false, own_pin = false;
+};
+
 // The context's workspace (photon claim counter, step counter) is shared by
-// the host-array calls and by device-form calls that bring no workspace of
-// their own, on whatever stream each uses.  ws_acquire makes `stream` wait on
+// device-form calls that bring no workspace of their own, on whatever stream
+// each uses.  ws_acquire makes `stream` wait on
 // the GPU until the previous use has finished; ws_release marks the end of
 // this use.  A stream under capture is left alone (the ordering would not be
 // part of the graph; callers that capture pass their own workspace).

@@ -144,27 +144,22 @@ int tmc_colormap_host(const float *heats, uint32_t shells, uint32_t width, uint3
     DeviceCtx *c = current_ctx(&st);
     if (!c)
         return st;
+    // device scratch: the image as floats, as RGBA, and the heats
     const size_t px = (size_t)width * height;
-    float *d_h = nullptr, *d_red = nullptr;
-    uint8_t *d_rgba = nullptr;
-    cudaError_t e = cudaMallocAsync(&d_h, sizeof(float) * shells, c->stream);
-    if (e == cudaSuccess && red)
-        e = cudaMallocAsync(&d_red, sizeof(float) * px, c->stream);
-    if (e == cudaSuccess && rgba)
-        e = cudaMallocAsync(&d_rgba, 4 * px, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(d_h, heats, sizeof(float) * shells, cudaMemcpyHostToDevice, c->stream);
+    CallBuffers buf(*c);
+    cudaError_t e = buf.device((red ? 4 * px : 0) + (rgba ? 4 * px : 0) + sizeof(float) * (size_t)shells, IMAGE_KEEP);
+    if (e != cudaSuccess)
+        return set_cuda_error(e, "tmc_colormap_host");
+    float *d_red = red ? reinterpret_cast<float *>(buf.dev) : nullptr;
+    uint8_t *d_rgba = rgba ? reinterpret_cast<uint8_t *>(buf.dev + (red ? 4 * px : 0)) : nullptr;
+    float *d_h = reinterpret_cast<float *>(buf.dev + (red ? 4 * px : 0) + (rgba ? 4 * px : 0));
+    e = cudaMemcpyAsync(d_h, heats, sizeof(float) * shells, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess)
         e = launch_colormap(d_h, shells, width, height, d_red, d_rgba, c->stream);
     if (e == cudaSuccess && red)
         e = cudaMemcpyAsync(red, d_red, sizeof(float) * px, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess && rgba)
         e = cudaMemcpyAsync(rgba, d_rgba, 4 * px, cudaMemcpyDeviceToHost, c->stream);
-    cudaFreeAsync(d_h, c->stream);
-    if (d_red)
-        cudaFreeAsync(d_red, c->stream);
-    if (d_rgba)
-        cudaFreeAsync(d_rgba, c->stream);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(c->stream);
     return e == cudaSuccess ? TMC_OK : set_cuda_error(e, "tmc_colormap_host");
