@@ -281,11 +281,12 @@ cudaError_t grid_for(const tmc_batch *b, int *grid)
 }
 
 // How a batch uses the device: blocks per SM, and from how many expected steps
-// per photon on a problem's photons are walked one to a warp (walk_batch; see
-// warp_steps) instead of one to a lane.
+// per photon on a problem's photons are walked one to a warp (see warp_steps)
+// instead of one to a lane.
 struct Spread {
     int per_sm = 1;
     double whole = 1e300;
+    double finish = 1e300;   // from here on, walk_stream's photons past a roulette are the whole warp's
 };
 
 // More warps per scheduler walk more steps a second, but each lane takes longer
@@ -302,7 +303,7 @@ struct Spread {
 // photon to a warp: 73 problems (9e7 steps, up to 7e4) 7.7 ms against 41 on
 // lanes, 378 55 ms against 68.
 Spread spread(const std::vector<tmc_problem> &problems, const std::vector<double> &est_steps, int block, int most,
-              int sms, uint32_t math, bool stream)
+              int sms, uint32_t math)
 {
     std::vector<std::pair<double, double>> p;   // steps per photon and in all, longest first
     double total = 0.0;
@@ -333,8 +334,9 @@ Spread spread(const std::vector<tmc_problem> &problems, const std::vector<double
                 best_t = t;
                 best.per_sm = k;
                 best.whole = i ? p[i - 1].first : 1e300;
+                best.finish = 0.4 * t / lane_step;
             }
-            if (i == p.size() || stream)
+            if (i == p.size())
                 break;
             long_work += p[i].second;
         }
@@ -402,7 +404,7 @@ int plan(tmc_batch *b)
     cudaError_t e = grid_for(b, &grid);   // also sets the kernel's shared-memory limit
     if (e != cudaSuccess)
         return set_cuda_error(e, "batch kernel config");
-    const Spread use = spread(b->problems, b->est_steps, b->cfg.block, grid / b->sms, b->sms, b->math, b->cfg.stream != 0);
+    const Spread use = spread(b->problems, b->est_steps, b->cfg.block, grid / b->sms, b->sms, b->math);
     grid = b->sms * use.per_sm;
     b->grid = grid;
     const std::vector<BatchItemDev> h =
@@ -424,9 +426,10 @@ int plan(tmc_batch *b)
     }
     bool claims = false;   // claims that differ from the device's
     for (size_t i = 0; i < b->dev.size(); ++i) {
-        const uint32_t claim = b->est_steps[i] >= use.whole ? 1 : 0;
-        claims = claims || claim != b->dev[i].claim;
+        const uint32_t claim = b->est_steps[i] >= use.whole ? 1 : 0, finish = b->est_steps[i] >= use.finish ? 1 : 0;
+        claims = claims || claim != b->dev[i].claim || finish != b->dev[i].finish;
         b->dev[i].claim = claim;
+        b->dev[i].finish = finish;
     }
     if (claims) {
         e = cudaMemcpy(b->d_problems, b->dev.data(), sizeof(BatchProblemDev) * b->dev.size(), cudaMemcpyHostToDevice);
@@ -615,7 +618,7 @@ int tmc_batch_create(tmc_batch **out, const tmc_problem *problems, uint32_t n_pr
         hp[i].c.last = d.last;
         hp[i].c.shells = d.shells;
         hp[i].claim = 0;
-        hp[i].reserved = 0;
+        hp[i].finish = 0;
         hp[i].id_base = q.photon_id_base;
         hp[i].tally_offset = b->offsets[i];
         b->offsets[i + 1] = b->offsets[i] + q.shells;

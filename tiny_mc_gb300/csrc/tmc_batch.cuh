@@ -17,7 +17,8 @@ constexpr unsigned QUEUE_HOLD = 0, QUEUE_DRAIN = 1, QUEUE_STOP = 2;
 struct BatchProblemDev {
     WalkConsts c;
     uint32_t claim;                    // walk_batch: photon ids a warp claims at once (0: BATCH_CHUNK)
-    uint32_t reserved;
+    // walk_stream: photons that survive a roulette are walked on by the whole warp
+    uint32_t finish;
     unsigned long long id_base;
     unsigned long long tally_offset;   // in shells
 };
@@ -166,6 +167,7 @@ __device__ __forceinline__ bool queue_try_claim(const BatchArgs &a, BatchItemDev
     pr.c.last = vp->c.last;
     pr.c.shells = vp->c.shells;
     pr.claim = 0;
+    pr.finish = 0;
     pr.id_base = vp->id_base;
     pr.tally_offset = vp->tally_offset;
     qidx = slot;

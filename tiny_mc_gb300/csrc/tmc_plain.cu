@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(COUNT_BLOCK, 2) walk_counts(const PlainArgs a)
     src.n = a.n_photons;
     src.id_base = a.id_base;
     src.chunk = a.chunk;
+    const float beyond = a.c.last + (float)(threadIdx.x & 31u);
     CountTally<M, COUNT_BLOCK> tally{table, S - 1, a.tally, table.base};
     auto add_steps = [&](unsigned long long n) {
         if (a.steps) {
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(COUNT_BLOCK, 2) walk_counts(const PlainArgs a)
     };
     // a warp adds at most 2^27 to a count between its flushes: 2^31 for a block
     walk_photons<COUNT_BLOCK, M, true, (1u << 22), TRIP>(
-        a.c, a.c.last + (float)(threadIdx.x & 31u), src, a.keys, smem + words + threadIdx.x, tally, [&] {
+        a.c, beyond, src, a.keys, smem + words + threadIdx.x, tally, [&] {
             add_steps(flush_counts<true>(smem, rows, S, threadIdx.x & 31u, 32, 0, 1, a.tally));
         });
 

@@ -851,7 +851,7 @@ int tmc_server_submit(tmc_server *s, const tmc_request *r, uint64_t *id)
     pd.c.last = q.d.last;
     pd.c.shells = q.d.shells;
     pd.claim = 0;
-    pd.reserved = 0;
+    pd.finish = 0;
     pd.id_base = r->photon_id_base;
     pd.tally_offset = (unsigned long long)q.slot * s->cfg.max_shells;
     cudaError_t e = cudaSuccess;

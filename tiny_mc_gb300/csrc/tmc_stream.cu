@@ -65,6 +65,8 @@ struct __align__(16) OpenItem {    // per buffer, in shared memory
     uint32_t problem;              // the item's problem
     uint32_t item;                 // global item index, or END_ITEM
     uint32_t count;                // photons in the item
+    uint32_t claim;                // photon ids per claim; 1: the whole warp walks each
+    uint32_t finish;               // the whole warp walks photons past a roulette
     uint32_t ps;                   // probe shell, clamped to the problem
     uint32_t next;                 // photon counter within the item
     uint32_t done;                 // warps that reported the item
@@ -81,6 +83,8 @@ __device__ __forceinline__ void fill_item(const BatchArgs &a, OpenItem *o, const
     o->g = a.tally + 4 * pr.tally_offset;
     o->id_first = pr.id_base + itm.first;
     o->count = itm.count;
+    o->finish = pr.finish;
+    o->claim = pr.claim ? pr.claim : (uint32_t)BATCH_CHUNK;
     o->problem = itm.problem;
     o->ps = min(a.probe_shell, pr.c.shells - 1);
     o->next = 0;
@@ -128,45 +132,78 @@ __device__ __forceinline__ bool open_item(const BatchArgs &a, OpenItem *o)
     return false;
 }
 
-// step_photon's tally of a lane: its photon's item's histogram and record.
-template <class M>
+// step_photon's tally of a lane (its photon's item's histogram and record), and
+// walk_whole's of a warp (the record of the photon it walks).
+template <int BLOCK, class M>
 struct StreamTally {
-    uint32_t *hist;
-    uint32_t cells, last, probe;
-    float albedo;
+    uint32_t *smem;     // the two histograms
+    uint32_t HS;        // words of one
+    uint32_t spread;
+    OpenItem *open;
+    uint32_t lane, lb;  // buffer of this lane's photon
+    // the item of this lane's photon; in walk_whole, of the photon walked
+    WalkConsts c;
     unsigned long long *g;
-    OpenItem *item;
-    uint32_t &steps;   // of this lane's photon
+    uint32_t probe, buf;
+    bool finish;        // of this lane's photon's item
+    uint32_t &steps;    // of this lane's photon
     bool &want;
 
+    __device__ __forceinline__ void deposit(uint32_t cell, float weight)
+    {
+        const uint32_t shell = min(cell, c.shells - 1), cells = c.shells + spread;
+        uint32_t *t0 = smem + buf * HS + cell;
+        uint32_t lo, hi;
+        units_split(weight_units(weight), lo, hi);
+        tally_add(t0, t0 + cells, &g[4 * shell + 1], lo, hi, shell == probe ? &open[buf].wraps : nullptr);
+        units_split(weight2_units(weight), lo, hi);
+        tally_add(t0 + 2 * cells, t0 + 3 * cells, &g[4 * shell + 3], lo, hi);
+    }
     __device__ __forceinline__ void step(LanePhoton &p, uint32_t cell)
     {
-        const uint32_t shell = min(cell, last);
-        uint32_t *t0 = hist + cell;
-        uint32_t lo, hi;
-        units_split(weight_units(p.weight), lo, hi);
-        tally_add(t0, t0 + cells, &g[4 * shell + 1], lo, hi, shell == probe ? &item->wraps : nullptr);
-        units_split(weight2_units(p.weight), lo, hi);
-        tally_add(t0 + 2 * cells, t0 + 3 * cells, &g[4 * shell + 3], lo, hi);
-        p.weight = M::mul(p.weight, albedo);
+        deposit(cell, p.weight);
+        p.weight = M::mul(p.weight, c.albedo);
         ++steps;
     }
     __device__ __forceinline__ bool low(const LanePhoton &p) const { return p.weight < 0.001f * WEIGHT_ONE; }
-    __device__ __forceinline__ void survived(LanePhoton &p) { p.weight = __fdiv_rn(p.weight, 0.1f); }
+    __device__ __forceinline__ void survived(LanePhoton &p)
+    {
+        p.weight = __fdiv_rn(p.weight, 0.1f);
+        if (finish)
+            Ring<BLOCK>::set_aside(p);
+    }
     __device__ __forceinline__ void died(LanePhoton &)
     {
         want = true;
         // the photon's steps into its item's 64-bit count
-        const uint32_t old = atomicAdd(&item->steps_lo, steps);
+        const uint32_t old = atomicAdd(&open[lb].steps_lo, steps);
         if (old + steps < old)
-            atomicAdd(&item->steps_hi, 1u);
+            atomicAdd(&open[lb].steps_hi, 1u);
+    }
+    __device__ __forceinline__ float weight(const LanePhoton &p) const { return p.weight; }
+    __device__ __forceinline__ uint32_t row_of(const LanePhoton &) const { return 0; }
+    __device__ __forceinline__ uint32_t row_after(uint32_t, uint32_t) const { return 0; }
+    __device__ __forceinline__ void resume(LanePhoton &, uint32_t) {}
+    __device__ __forceinline__ Optics optics(int l)
+    {
+        buf = __shfl_sync(FULL_MASK, lb, l);
+        c = open[buf].c;
+        g = open[buf].g;
+        probe = open[buf].ps;
+        return Optics{c, c.last + (float)(lane & spread)};
+    }
+    __device__ __forceinline__ void whole(uint32_t, uint32_t cell, float weight) { deposit(cell, weight); }
+    __device__ __forceinline__ void walked(int l, uint32_t n)
+    {
+        if ((int)lane == l)
+            steps += n;
     }
 };
 
 }  // namespace
 
 template <int BLOCK, class M, bool QUEUE>
-__global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_stream(const BatchArgs a)
 {
     constexpr unsigned NWARPS = BLOCK / 32;
     extern __shared__ __align__(16) uint32_t smem[];
@@ -220,9 +257,16 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
     WalkConsts pc{};
     unsigned long long *pg = nullptr;
     uint32_t pps = 0;
+    bool pfin = false;
     unsigned long long wait_start = 0;
 
     for (;;) {
+        // photons set aside for the whole warp
+        const bool aside = R::aside(p);
+        if (aside)
+            p.cur -= R::ASIDE;
+        unsigned todo = __ballot_sync(FULL_MASK, aside);
+
         // -------- report items this warp is finished with (oldest first)
         for (;;) {
             if (rep > jc || (rep == jc && !exh))
@@ -311,7 +355,7 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
                 if (k == 0) {
                     uint32_t base = 0;
                     if (lane == 0)
-                        base = atomicAdd((unsigned *)&open[cb].next, (uint32_t)BATCH_CHUNK);
+                        base = atomicAdd((unsigned *)&open[cb].next, open[cb].claim);
                     base = __shfl_sync(FULL_MASK, base, 0);
                     const uint32_t count = open[cb].count;
                     if (base >= count) {
@@ -319,7 +363,7 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
                         continue;
                     }
                     cn = base;
-                    ce = min(base + (uint32_t)BATCH_CHUNK, count);
+                    ce = min(base + open[cb].claim, count);
                     k = min((uint32_t)n_need, ce - cn);
                 }
                 const bool mine = ((need >> lane) & 1u) && rank < k;
@@ -332,8 +376,13 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
                     pc = open[cb].c;
                     pg = open[cb].g;
                     pps = open[cb].ps;
+                    pfin = open[cb].finish != 0;
                 }
                 cn += k;
+                if (open[cb].claim == 1) {   // one photon at a time
+                    todo |= __ballot_sync(FULL_MASK, mine);
+                    break;
+                }
                 need = __ballot_sync(FULL_MASK, want);
                 continue;
             }
@@ -366,8 +415,8 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
             want = false;
         }
 
-        const bool any_alive = __any_sync(FULL_MASK, R::walking(p));
-        if (!any_alive) {
+        const unsigned alive = __ballot_sync(FULL_MASK, R::walking(p));
+        if (!alive) {
             if (it_c == END_ITEM && rep >= jc)
                 break;   // all photons walked, all items reported
             // nothing to walk until the block frees a buffer: sleep about an
@@ -386,9 +435,27 @@ __global__ void __launch_bounds__(BLOCK) walk_stream(const BatchArgs a)
         }
         wait_start = 0;
 
-        StreamTally<M> tally{smem + lb * HS, pc.shells + spread, pc.shells - 1, pps, pc.albedo, pg, &open[lb], steps, want};
+        StreamTally<BLOCK, M> tally{smem, HS, spread, open, lane, lb, pc, pg, pps, lb, pfin, steps, want};
+        // no more items and few photons left: the whole warp walks them (one
+        // whose direction is still sought waits for the lane loop)
+        if (it_c == END_ITEM && __popc(alive) <= WARP_WALK_MAX)
+            todo |= __ballot_sync(FULL_MASK, R::walking(p) && !(p.t > 1.0f));
+        if (todo) {
+            uint32_t trips = 0;
+            const unsigned ended = walk_whole<BLOCK, M, 0>(p, todo, trips, ring, a.keys, tally,
+                                                               [&](int l) { return tally.optics(l); });
+            pc = open[lb].c;
+            pg = open[lb].g;
+            pps = open[lb].ps;
+            if (ended)
+                continue;
+        }
+        tally.c = pc;
+        tally.g = pg;
+        tally.probe = pps;
+        tally.buf = lb;
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < 4; ++k) {
             if (k % 2 == 0)
                 R::refill(p, ring, a.keys);
             step_photon<BLOCK, M>(p, ring, pc.spm, pc.last, pc.last + (float)(lane & spread), tally);

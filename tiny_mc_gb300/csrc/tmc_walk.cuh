@@ -757,6 +757,11 @@ struct SavedPhotons {
 
 // Tally objects of step_photon: `whole` deposits a step of a photon that the
 // whole warp walks.
+struct Optics {
+    WalkConsts c;
+    float beyond;   // cell of a radius beyond the last shell, this lane's
+};
+
 template <class M, Hist H>
 struct WeightTally {
     uint32_t hist;            // shared address of the histogram
@@ -795,6 +800,7 @@ struct WeightTally {
     __device__ __forceinline__ uint32_t row_after(uint32_t, uint32_t) const { return 0; }
     __device__ __forceinline__ void resume(LanePhoton &, uint32_t) {}
     __device__ __forceinline__ void whole(uint32_t, uint32_t cell, float weight) { deposit(cell, weight); }
+    __device__ __forceinline__ void walked(int, uint32_t) {}
 };
 
 template <class M, int BLOCK>
@@ -829,6 +835,7 @@ struct CountTally {
     {
         return __uint_as_float(ld_shared(row + table.weight_at));
     }
+    __device__ __forceinline__ void walked(int, uint32_t) {}
     __device__ __forceinline__ uint32_t row_of(const LanePhoton &) const { return row; }
     __device__ __forceinline__ uint32_t row_after(uint32_t at, uint32_t steps) const
     {
@@ -854,6 +861,68 @@ struct CountTally {
         ++steps;
     }
 };
+
+// The whole warp walks the photons of the lanes in `todo` one by one to their
+// ends, or until `trips`, counted up once per round, reaches MAX_TRIPS (0: no
+// bound).  Every lane's ring is used as scratch and filled again.  Returns the
+// lanes whose photons ended.  optics(l) gives the constants of lane l's
+// photon, tally.whole(..) deposits a step of it, tally.walked(l, n) counts n,
+// tally.died is called on lane l at its end.
+template <int BLOCK, class M, uint32_t MAX_TRIPS, class Tally, class Of>
+__device__ __forceinline__ unsigned walk_whole(LanePhoton &p, unsigned todo, uint32_t &trips, char *ring,
+                                               const PhiloxKeys &keys, Tally &tally, Of optics)
+{
+    using R = Ring<BLOCK>;
+    const unsigned lane = threadIdx.x & 31u;
+    const WarpScratch sc{ring - 4 * lane, R::W};
+    unsigned left = __ballot_sync(FULL_MASK, R::walking(p));   // lanes with a photon
+    const unsigned had = left;
+    const SavedPhotons<BLOCK> saved{sc.rows};
+    __syncwarp();
+    saved.save((int)lane, p, tally.weight(p), tally.row_of(p));
+    __syncwarp();
+    while (todo && (MAX_TRIPS == 0 || trips < MAX_TRIPS)) {
+        const int l = __ffs((int)todo) - 1;
+        todo &= todo - 1;
+        const Optics o = optics(l);
+        WarpPhoton q = saved.get(l);
+        uint32_t row = saved.word(l, S_ROW);
+        bool over = false;
+        do {
+            uint32_t cell;
+            float weight;
+            const uint32_t n = warp_steps<M>(q, over, sc, o.c, keys, o.beyond, cell, weight);
+            if (lane < n)
+                tally.whole(tally.row_after(row, lane), cell, weight);
+            row = tally.row_after(row, n);
+            tally.walked(l, n);
+            ++trips;
+        } while (!over && (MAX_TRIPS == 0 || trips < MAX_TRIPS));
+        if (over)
+            left &= ~(1u << l);
+        else if ((int)lane == l)   // a flush is due first: back to its lane
+            saved.put_walk(l, q, row);
+    }
+    // back to the lanes, with fresh rings
+    __syncwarp();
+    const WarpPhoton q = saved.get((int)lane);
+    const uint32_t row = saved.word((int)lane, S_ROW);
+    p.t = saved.real((int)lane, S_T);
+    __syncwarp();
+    p.key = q.key;
+    p.x = q.x; p.y = q.y; p.z = q.z;
+    p.u = q.u; p.v = q.v; p.w = q.w;
+    p.weight = q.weight;
+    if ((left >> lane) & 1u) {
+        R::restart(p, q.block, q.rest, ring, keys);
+        tally.resume(p, row);
+    } else {
+        R::drop(p);
+        if ((had >> lane) & 1u)
+            tally.died(p);
+    }
+    return had & ~left;
+}
 
 // Walk photons from `src` until it is exhausted and every lane's photon has
 // died.  Warp-collective: all 32 lanes of every warp call it.  flush() empties
@@ -900,52 +969,10 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
             todo |= __ballot_sync(FULL_MASK, R::walking(p) && !(p.t > 1.0f));
         }
         if (todo) {
-            const WarpScratch sc{ring - 4 * lane, R::W};
             if (COUNTS && R::aside(p))
                 p.cur -= R::ASIDE;
-            unsigned left = __ballot_sync(FULL_MASK, R::walking(p));   // lanes with a photon
-            const unsigned had = left;
-            const SavedPhotons<BLOCK> saved{sc.rows};
-            __syncwarp();
-            saved.save((int)lane, p, tally.weight(p), tally.row_of(p));
-            __syncwarp();
-            while (todo && trips < FLUSH_TRIPS) {
-                const int l = __ffs((int)todo) - 1;
-                todo &= todo - 1;
-                WarpPhoton q = saved.get(l);
-                uint32_t row = saved.word(l, S_ROW);
-                bool over = false;
-                do {
-                    uint32_t cell;
-                    float weight;
-                    const uint32_t n = warp_steps<M>(q, over, sc, c, keys, beyond, cell, weight);
-                    if (lane < n)
-                        tally.whole(tally.row_after(row, lane), cell, weight);
-                    row = tally.row_after(row, n);
-                    ++trips;
-                } while (!over && trips < FLUSH_TRIPS);
-                if (over)
-                    left &= ~(1u << l);
-                else if ((int)lane == l)   // a flush is due first: back to its lane
-                    saved.put_walk(l, q, row);
-            }
-            // back to the lanes, with fresh rings
-            __syncwarp();
-            const WarpPhoton q = saved.get((int)lane);
-            const uint32_t row = saved.word((int)lane, S_ROW);
-            p.t = saved.real((int)lane, S_T);
-            __syncwarp();
-            p.key = q.key;
-            p.x = q.x; p.y = q.y; p.z = q.z;
-            p.u = q.u; p.v = q.v; p.w = q.w;
-            p.weight = q.weight;
-            if ((left >> lane) & 1u) {
-                R::restart(p, q.block, q.rest, ring, keys);
-                tally.resume(p, row);
-            } else {
-                R::drop(p);
-            }
-            if (left != had)
+            if (walk_whole<BLOCK, M, FLUSH_TRIPS>(p, todo, trips, ring, keys, tally,
+                                                  [&](int) { return Optics{c, beyond}; }))
                 continue;
         }
         if (trips == FLUSH_TRIPS) {   // a trip stands for TRIP deposits of a lane at most
