@@ -75,6 +75,7 @@ struct Req {
     double est_steps = 0.0;         // expected photon steps per photon
     uint64_t max_batches = 0;
     uint64_t issued = 0, done = 0;  // work items
+    uint64_t done_photons = 0;      // of finished pieces (a wave may walk an item in several)
     uint64_t next_decision = 0;     // in batches
     std::vector<unsigned long long> probe;   // per item: 128-bit sum of w in the probe shell
                                              // (2^-40 units), lo and hi
@@ -86,8 +87,8 @@ struct Wave {
     cudaEvent_t done = nullptr;
     BatchItemDev *d_items = nullptr;
     unsigned long long *d_counter = nullptr;   // item counter, error flag, ring tail
-    BatchItemDev *h_items = nullptr;           // pinned
-    unsigned long long *h_ring = nullptr;      // mapped: completion ring [items][4]
+    BatchItemDev *h_items = nullptr;           // pinned: the wave's pieces
+    unsigned long long *h_ring = nullptr;      // mapped: completion ring [pieces][4]
     unsigned long long *d_ring = nullptr;      // its device address
     unsigned long long *h_err = nullptr;       // pinned: the wave's error flag
     uint32_t n_items = 0;
@@ -348,9 +349,11 @@ int harvest(tmc_server *s, Wave &w, bool ended)
         }
         Req &q = f->second;
         const uint64_t g = it.first / q.item_photons;
-        q.probe[2 * g] = e[0];
-        q.probe[2 * g + 1] = e[1];
-        ++q.done;
+        const unsigned long long lo = q.probe[2 * g] + e[0];   // an item's pieces add up, 128-bit
+        q.probe[2 * g + 1] += e[1] + (lo < e[0] ? 1 : 0);
+        q.probe[2 * g] = lo;
+        q.done_photons += it.count;
+        q.done = q.done_photons / q.item_photons;   // all issued ones are in when it equals issued
         --s->inflight;
         touched.push_back(id);
         ++w.head;
@@ -416,6 +419,42 @@ uint32_t take_pending(tmc_server *s, uint64_t cap_n, uint64_t quota_base, Put pu
     return n;
 }
 
+// Where the launches in flight leave blocks idle, cut a wave's n items into equal
+// pieces for them, as many as the wave has room for, of two photons per thread
+// or more (the kernel's smallest item), or one where a photon is 4096 steps or
+// longer; the pieces with the longest walks of a lane go first.  An item is about
+// 8e6 photon steps, 30 ms of one block; 48 requests of 16 such batches on 1216
+// blocks take 34 ms whole and 23 ms in pieces.  Not with a bound on the items
+// in flight, which counts items.  Returns the number of pieces.
+uint32_t split_items(const tmc_server *s, Wave &w, uint32_t n)
+{
+    uint64_t k = 1;
+    while (2 * k * n <= s->wave_cap && s->inflight + k * n < 4ull * (uint64_t)s->grid)
+        k *= 2;
+    if (k == 1 || s->cfg.inflight_items)
+        return n;
+    std::vector<std::pair<double, BatchItemDev>> pieces;
+    for (uint32_t i = 0; i < n; ++i) {
+        const BatchItemDev &it = w.h_items[i];
+        const double est = s->active.find(s->slot_req[it.problem])->second.est_steps;
+        const uint32_t per_thread = est < 4096.0 ? 2 : 1;
+        const uint32_t lo = s->cfg.stream ? (uint32_t)BATCH_CHUNK : per_thread * s->cfg.block;
+        uint32_t parts = 1;   // item sizes are powers of two
+        while (parts < k && it.count / (2 * parts) >= lo)
+            parts *= 2;
+        BatchItemDev piece = it;
+        piece.count = it.count / parts;
+        const double chain = est * std::max(1.0, (double)piece.count / s->cfg.block);
+        for (uint32_t j = 0; j < parts; ++j, piece.first += piece.count)
+            pieces.push_back({chain, piece});
+    }
+    std::stable_sort(pieces.begin(), pieces.end(),
+                     [](const auto &x, const auto &y) { return x.first > y.first; });
+    for (size_t i = 0; i < pieces.size(); ++i)
+        w.h_items[i] = pieces[i].second;
+    return (uint32_t)pieces.size();
+}
+
 // Fill a wave with pending items (take_pending's order) and launch it.
 int launch_wave(tmc_server *s, Wave &w)
 {
@@ -429,6 +468,7 @@ int launch_wave(tmc_server *s, Wave &w)
                  [&](const BatchItemDev &it, uint64_t, uint64_t) { w.h_items[n++] = it; });
     if (n == 0)
         return TMC_OK;
+    n = split_items(s, w, n);
     w.n_items = n;
     w.head = 0;
     s->inflight += n;
