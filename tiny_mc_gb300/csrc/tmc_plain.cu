@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(COUNT_BLOCK, 2) walk_counts(const PlainArgs a)
     // a warp adds at most 2^27 to a count between its flushes: 2^31 for a block
     walk_photons<COUNT_BLOCK, M, true, (1u << 22), TRIP>(
         a.c, beyond, src, a.keys, smem + words + threadIdx.x, tally, [&] {
-            add_steps(flush_counts<true>(smem, rows, S, threadIdx.x & 31u, 32, 0, 1, a.tally));
+            const unsigned long long n = flush_counts<true>(smem, rows, S, threadIdx.x & 31u, 32, 0, 1, a.tally);
+            add_steps(n + ((threadIdx.x & 31u) == 0 ? atomicExch(smem + rows * stride, 0u) : 0u));
         });
 
     __syncthreads();
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(COUNT_BLOCK, 2) walk_counts(const PlainArgs a)
     }
     __syncthreads();
     const uint32_t across = min((S + 31) / 32 * 32, (uint32_t)COUNT_BLOCK), groups = COUNT_BLOCK / across;
-    unsigned long long counted = tally.steps;
+    unsigned long long counted = threadIdx.x == 0 ? smem[rows * stride] : 0u;
     if (threadIdx.x < groups * across)
         counted += flush_counts<false>(smem, rows, S, threadIdx.x % across, across, threadIdx.x / across, groups,
                                        a.tally);
