@@ -63,18 +63,18 @@ REF_SECONDS_PER_STEP = 3.0    # each reference-arm step: every core walks ~3 s
 # marks the figures "stale" when they differ (the kernel changed since the
 # capture), in which case they must not be read as this build's.
 NCU_WALK = {
-    "capture": "profiles/walk_plain_fast_2p25photons_ncu_full.txt",
+    "capture": "profiles/walk_counts_fast_2p25photons_ncu_full.txt",
     "sources": ["tiny_mc_gb300/csrc/tmc_device.cuh", "tiny_mc_gb300/csrc/tmc_walk.cuh",
                 "tiny_mc_gb300/csrc/tmc_plain.cu"],
-    "sources_sha256": "ea19d338f68d330bf85235a1a34dc1fde124bf73e8b6288c8c512f1da601432c",
+    "sources_sha256": "a2f658ccba6d4ff1a4a3b6568480be7dae807b38030cf626e146ef28dc000ca1",
     # thread-instructions (predicated on) per photon step
-    "thread_instr_per_step": 226.5,
+    "thread_instr_per_step": 136.3,
     # busy fraction of each pipe
-    "pipes_busy": {"issue_slots": 0.827, "alu": 0.550, "fma": 0.340, "xu_sfu": 0.134,
-                   "shared_wavefronts": 0.541, "dram": 0.0},
-    # DRAM bytes read + written by one launch (constant and code fetch plus the
-    # warps' 101-shell histogram flushes; not proportional to the photon count)
-    "dram_bytes_per_launch": 178944,
+    "pipes_busy": {"issue_slots": 0.746, "alu": 0.527, "fma": 0.391, "xu_sfu": 0.094,
+                   "shared_wavefronts": 0.339, "dram": 0.0},
+    # DRAM bytes read + written by one launch (constant and code fetch; the
+    # 101-shell tally stays in L2; not proportional to the photon count)
+    "dram_bytes_per_launch": 61184,
 }
 
 

@@ -16,6 +16,8 @@
 //    flush_steps(BLOCK) steps swaps the histogram into the problem's global
 //    tally), then adds what is left to the problem's 128-bit global tally and
 //    takes the next item;
+//  * an estimate of the launch's end (spread) picks the blocks per SM and the
+//    problems whose photons are walked one to a warp instead of one to a lane;
 //  * results are integer tallies keyed by photon id, so each problem's tally
 //    is bit-identical to the plain kernel's for the same photons, whatever
 //    the item split, block size or order;

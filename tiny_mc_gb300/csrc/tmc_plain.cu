@@ -278,7 +278,8 @@ template <class M, int TRIP>
 static cudaError_t launch_counts_t(const PlainLaunch &L, const DeviceCtx &ctx, uint32_t rows, cudaStream_t stream)
 {
     const size_t smem = 4 * (size_t)(count_words(rows, L.d.shells) + SLOTS * COUNT_BLOCK);
-    cudaError_t e = cudaFuncSetAttribute(walk_counts<M, TRIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(walk_counts<M, TRIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per_sm = 0;
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, walk_counts<M, TRIP>, COUNT_BLOCK, smem);
@@ -325,8 +326,9 @@ static cudaError_t try_launch(const PlainLaunch &L, const DeviceCtx &ctx, cudaSt
 // A histogram per block where it leaves the SM its 1024 threads, else the split
 // form where it reaches (8000 shells of 12.5 um, 2^21 photons of params.h
 // optics: one block per SM 1.26 ms, split 1.02; 20000 shells of 5 um: 5.25 ms
-// global, 1.02 split), else a block's histogram at any occupancy (4001 shells of 1 um, 5000 photons: 1.2 ms global, 55 us with three blocks
-// of 128 threads per SM), else global.
+// global, 1.02 split), else a block's histogram at any occupancy (4001 shells of
+// 1 um, 5000 photons: 1.2 ms global, 55 us with three blocks of 128 threads per
+// SM), else global.
 template <int BLOCK, class M>
 static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
@@ -371,8 +373,8 @@ static cudaError_t load_kernels()
 cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
     // Counts instead of sums wherever their table fits and the launch fills the
-    // device: 2^24 photons of params.h optics 7.63 -> 6.86 ms, 2^25 in exact
-    // arithmetic 20.0 -> 18.4 ms, 2^22 at albedo 0.09 0.25 -> 0.15 ms.  In smaller
+    // device: 2^24 photons of params.h optics 7.63 -> 6.72 ms, 2^25 in exact
+    // arithmetic 20.0 -> 18.2 ms, 2^22 at albedo 0.09 0.25 -> 0.15 ms.  In smaller
     // launches setting the table up and adding it costs more: 100000 photons 125
     // us against 100, 131072 127 against 118, 155000 128 against 130; at albedo
     // 0.09 70000 photons 38 against 64.

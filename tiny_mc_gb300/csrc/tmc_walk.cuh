@@ -28,21 +28,26 @@
 //  * the two tallies of photon.c:30-31 go into a shared-memory histogram of
 //    64-bit fixed-point sums (sum of w and of w^2, 2^-40 units), each kept as
 //    two 32-bit words updated with native 32-bit shared atomics (a 64-bit
-//    shared atomicAdd is a compare-and-swap loop, 4x slower here).  Each warp
-//    adds the block's histogram into the 128-bit global tally and clears it
-//    every flush_steps iterations, which keeps its 64-bit sums from
-//    wrapping, so a deposit needs no wrap check.
+//    shared atomicAdd is a compare-and-swap loop, 4x slower here), or, for
+//    short walks over not too many shells, into one 32-bit count per step
+//    number and shell (CountTable).  A warp adds the block's histogram into the
+//    128-bit global tally and clears it every flush_steps iterations, which
+//    keeps the sums from wrapping, so a deposit needs no wrap check;
+//  * the last few photons of a warp, whose lanes would each take a step in
+//    turns that nobody else shares, are walked by all 32 lanes (warp_steps).
 //
-// What bounds it: instruction issue, then the shared-memory pipe.  One photon
-// step takes 5.86 warp-instructions (8.34 before the loop took this form) at
-// 3.03 per clock per SM, shared-memory wavefronts 69% of peak (2^25 photons
-// of params.h optics, fast arithmetic).  2^26 such photons: 41.1 ms with voted
-// single-block refills, 35.1 with one unvoted block per iteration, 33.8 with
-// the loop body unrolled twice, 32.1 with two blocks every second iteration
-// (which share the round-key loads), 31.2 with four iterations per check for
-// finished photons.  Six and eight iterations gain under 1% more there and
-// leave lanes of short walks idle longer.  Occupancy does not matter at this
-// point: 48 warps per SM (40 registers) measured the same as 32.
+// What bounds it: instruction issue.  2^25 photons of params.h optics in fast
+// arithmetic: 226 thread-instructions per photon step before the loop took this
+// form (8.34 warp-instructions, 3.28 per clock per SM), 159 with sums (5.86,
+// 3.03), 136 with counts (4.89, 2.97); shared-memory wavefronts 69% of peak
+// with sums, 34% with counts; ALU pipe 53%, heavy FMA pipe (Philox multiplies)
+// 42%.  Exact arithmetic 194 (6.97, 3.13).  What the loop's parts were worth, 2^26 such
+// photons with sums: 41.1 ms with voted single-block refills, 35.1 with one
+// unvoted block per iteration, 33.8 with the loop body unrolled twice, 32.1 with
+// two blocks every second iteration (which share the round-key loads), 31.2
+// with four iterations per check for finished photons; with counts and eight
+// iterations 26.9.  Occupancy does not matter at this point: 48 warps per SM
+// (40 registers) measured the same as 32.
 #pragma once
 
 #include "tmc_device.cuh"
@@ -71,14 +76,14 @@ constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the 
 constexpr int WARP_WALK_MAX = 8;
 
 // Where a walk keeps its tallies.  Block: a shared histogram per block (one per
-// warp, which the plain walk once had, measured the same at 2^18 photons and
-// more and costs small launches more flushes: 75000 photons 127 us against 96).  Split: a block's histogram holds
+// warp measured the same from 2^18 photons on and costs small launches more
+// flushes: 75000 photons 127 us against 96).  Split: a block's histogram holds
 // the shells nearest to the source, where nearly all deposits of a point source
 // land, and a deposit farther out is a 64-bit atomic add into the 128-bit global
 // tally (shell counts whose histogram does not fit in shared memory).  Global:
-// every deposit is (shells so thin that most land beyond such a histogram).  Count: one count per (step, shell)
-// of a block (CountTable).
-enum class Hist { Block, Split, Global, Count };
+// every deposit is (shells so thin that most land beyond such a histogram).
+// Counts have a tally of their own (CountTally).
+enum class Hist { Block, Split, Global };
 
 // A warp adds its block's histogram, of `lanes` lanes, into the global tally and
 // clears it every flush_steps(lanes) of its iterations.  A lane deposits at most once per
@@ -990,12 +995,13 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
     }
 }
 
-// walk_photons with a block's histogram of 64-bit sums, 4 * hist_cells words (low and high of sum w, then of sum
-// w^2), flushed into g, the problem's global 128-bit tally [shells][4], every
-// flush_steps iterations (the caller flushes what is left).  H = Split: a block
-// histogram of 4 * near words for the first `near` shells.  probe_acc /
-// probe_hi (Block only, may be null): receive the w sums those flushes take
-// from shell probe_shell.  Returns this thread's photon steps.
+// walk_photons with a block's histogram of 64-bit sums, 4 * hist_cells words
+// (low and high of sum w, then of sum w^2), flushed into g, the problem's global
+// 128-bit tally [shells][4], every flush_steps iterations (the caller flushes
+// what is left).  H = Split: a block histogram of 4 * near words for the first
+// `near` shells; H = Global: none.  probe_acc / probe_hi (Block only, may be
+// null): receive the w sums those flushes take from shell probe_shell.  Returns
+// this thread's photon steps.
 template <int BLOCK, class M, class Source, Hist H>
 __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               const PhiloxKeys &keys, uint32_t *tally,
