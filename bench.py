@@ -57,7 +57,7 @@ SFU_OPS_PER_STEP = 4          # log, sqrt (radius), divide + sqrt (direction)
 CPU_SECONDS_PER_PROC = 10.5   # each CPU-baseline process runs at least 10 s
 REF_SECONDS_PER_STEP = 3.0    # each reference-arm step: every core walks ~3 s
 
-# Figures from one ncu capture of walk_plain<512, FastMath> at params.h optics
+# Figures from one ncu capture of walk_counts<FastMath, 8> at params.h optics
 # (one 2^25-photon launch).  They describe the kernel built from the sources
 # whose SHA-256 is recorded here; bench.py hashes the current sources and
 # marks the figures "stale" when they differ (the kernel changed since the
@@ -153,7 +153,7 @@ def workload_config(args, world):
         "mu_s_per_cm": o["mu_s"],
         "rng": "Philox-4x32-10 keyed by photon id, seed 1",
         "math": args.math,
-        "tallies": "u64 shared / u128 global fixed point (2^-40)",
+        "tallies": "u32 counts or u64 sums shared / u128 global fixed point (2^-40)",
         "l2": "flushed between timed steps (256 MiB write); inputs are only parameters",
         "parallelism": f"replicas x{world} (photon-id ranges)",
     }
