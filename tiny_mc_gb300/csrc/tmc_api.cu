@@ -142,19 +142,22 @@ cudaError_t ws_release(DeviceCtx &c, cudaStream_t stream)
     return cudaEventRecord(c.ws_done, stream);
 }
 
+// All of a context's calls use its one stream, so its memory is ordered by that
+// stream and growing or freeing it waits for no other work on the device.
 cudaError_t CallBuffers::device(size_t bytes, size_t keep)
 {
     if (bytes > keep) {
-        const cudaError_t e = cudaMalloc(&dev, bytes);
+        const cudaError_t e = cudaMallocAsync(&dev, bytes, ctx.stream);
         own_dev = e == cudaSuccess;
         return e;
     }
     if (bytes > ctx.scratch_cap) {
-        cudaFree(ctx.scratch);   // waits for earlier work
+        if (ctx.scratch)
+            cudaFreeAsync(ctx.scratch, ctx.stream);
         ctx.scratch = nullptr;
         ctx.scratch_cap = 0;
         const size_t want = std::min(keep, std::max<size_t>(bytes + bytes / 2, 16384));
-        const cudaError_t e = cudaMalloc(&ctx.scratch, want);
+        const cudaError_t e = cudaMallocAsync(&ctx.scratch, want, ctx.stream);
         if (e != cudaSuccess)
             return e;
         ctx.scratch_cap = want;
@@ -187,7 +190,7 @@ cudaError_t CallBuffers::host(size_t bytes)
 CallBuffers::~CallBuffers()
 {
     if (own_dev)
-        cudaFree(dev);   // waits for the call's work
+        cudaFreeAsync(dev, ctx.stream);
     if (own_pin)
         std::free(pin);
 }
