@@ -152,7 +152,7 @@ static cudaError_t walk_batch_config(int sms, size_t smem, int *grid)
         return e;
     if (per_sm < 1)
         return cudaErrorInvalidConfiguration;
-    *grid = sms * per_sm;
+    *grid = sms * (QUEUE ? queue_blocks(per_sm) : per_sm);
     return cudaSuccess;
 }
 
