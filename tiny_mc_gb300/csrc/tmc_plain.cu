@@ -9,8 +9,8 @@
 // walk_counts: one count per (step, shell) and block instead of the sums.
 // Shell counts whose histogram leaves no room for the SM's blocks (params.h's
 // SHELLS is any size in the reference) take the split form: a histogram of the
-// shells nearest to the source, and 64-bit atomics on the 128-bit global tally
-// beyond them; or, with shells so thin that most deposits land beyond it, no
+// shells nearest to the source and of the last one, and 64-bit atomics on the
+// 128-bit global tally between them; or, with shells so thin that most deposits land beyond it, no
 // histogram at all.  The sums are the same integers in every form.
 #include <algorithm>
 #include <cmath>
@@ -61,11 +61,15 @@ struct PlainArgs {
     uint32_t rows;               // walk_counts: steps with counts
 };
 
-// Shells of the split form's histogram: what 1024 threads per SM (two blocks of
+// Cells of the split form's histogram: what 1024 threads per SM (two blocks of
 // 512) leave of its 228 KB beside the rings and each block's own 1 KB.
 __host__ __device__ constexpr uint32_t split_cells(int block)
 {
     return ((228 * 1024) / (1024 / block) - 1024 - 4 * SLOTS * block) / 16;
+}
+__host__ __device__ constexpr uint32_t split_near(int block, uint32_t shells)   // shells nearest to the source in it
+{
+    return split_cells(block) - LAST_CELLS < shells - 1 ? split_cells(block) - LAST_CELLS : shells - 1;
 }
 static_assert(split_cells(512) == 4544 && split_cells(128) % 4 == 0, "whole 16-byte rows of the ring behind it");
 
@@ -76,7 +80,7 @@ __global__ void __launch_bounds__(BLOCK, (H == Hist::Global ? 1536 : 1024) / BLO
 {
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t S = a.c.shells;
-    const uint32_t near = min(split_cells(BLOCK), S);   // shells of the split form's histogram
+    const uint32_t near = H == Hist::Split ? split_near(BLOCK, S) : S - 1;
     // words per histogram
     const uint32_t hist = 4 * (H == Hist::Split ? split_cells(BLOCK) : H == Hist::Global ? 0 : hist_cells(S));
     for (uint32_t s = threadIdx.x; s < hist; s += BLOCK)
@@ -92,14 +96,9 @@ __global__ void __launch_bounds__(BLOCK, (H == Hist::Global ? 1536 : 1024) / BLO
     const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H>(
         a.c, src, a.keys, smem, a.tally, my, near);
 
-    if constexpr (H == Hist::Split) {
+    if constexpr (H != Hist::Global) {
         __syncthreads();
-        const uint32_t part = (near + BLOCK / 32 - 1) / (BLOCK / 32);
-        const uint32_t first = min(threadIdx.x / 32 * part, near);   // this warp's share of the cells
-        warp_flush_cells<false>(smem + first, min(part, near - first), near, a.tally + 4 * (size_t)first);
-    } else if constexpr (H == Hist::Block) {
-        __syncthreads();
-        flush_tally<BLOCK>(smem, S, a.tally);
+        flush_tally<BLOCK>(smem, near, S, a.tally);
     }
     if (a.steps) {
         const unsigned long long tot = warp_sum_u64(steps);
@@ -339,7 +338,7 @@ static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStre
         return e;
     if (block_sm >= 1024 / BLOCK)
         return launch_t<BLOCK, M, Hist::Block>(L, ctx, block_sm, stream);
-    if (reaches(split_cells(BLOCK), L.d))
+    if (reaches(split_near(BLOCK, S), L.d))
         return try_launch<BLOCK, M, Hist::Split>(L, ctx, stream);
     if (block_sm >= 1)
         return launch_t<BLOCK, M, Hist::Block>(L, ctx, block_sm, stream);

@@ -79,8 +79,9 @@ constexpr int WARP_WALK_MAX = 8;
 // warp measured the same from 2^18 photons on and costs small launches more
 // flushes: 75000 photons 127 us against 96).  Split: a block's histogram holds
 // the shells nearest to the source, where nearly all deposits of a point source
-// land, and a deposit farther out is a 64-bit atomic add into the 128-bit global
-// tally (shell counts whose histogram does not fit in shared memory).  Global:
+// land, and the last one, and a deposit between them is a 64-bit atomic add into
+// the 128-bit global tally (shell counts whose histogram does not fit in shared
+// memory).  Global:
 // every deposit is (shells so thin that most land beyond such a histogram).
 // Counts have a tally of their own (CountTally).
 enum class Hist { Block, Split, Global };
@@ -103,30 +104,21 @@ static_assert(512ull * 257ull * ((1ull << 23) / 512 + 1) < (1ull << 32), "high w
 // warp at once, and shared atomics on one word take their turns.  So the last
 // shell has 32 cells, one per lane, which the flushes add up.  2^20 high-albedo
 // photons (1001 shells of 10 um, many walks leave): 46.8 -> 44.8 ms; the reduced
-// 4096-problem sweep 609 -> 555 ms.
+// 4096-problem sweep 609 -> 555 ms.  In the split form, where they would be
+// global atomics on one address, 2^21 photons of params.h optics over 4600 shells
+// of 0.53 um: 128.7 ms without the cells, 1.18 with them.
 constexpr uint32_t LAST_CELLS = 32;
 __host__ __device__ constexpr uint32_t hist_cells(uint32_t shells) { return shells + LAST_CELLS - 1; }
 
-// Take the 64-bit sum of cell s: `clear` by plain loads and stores, else by
-// atomic exchanges against zero while other warps deposit.
-template <bool EXCHANGE>
+// Take the 64-bit sum of a cell, by atomic exchanges against zero.
 __device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *hi)
 {
-    uint32_t l, h;
-    if constexpr (EXCHANGE) {
-        l = atomicExch(lo, 0u);
-        h = atomicExch(hi, 0u);
-    } else {
-        l = *lo;
-        h = *hi;
-        *lo = 0;
-        *hi = 0;
-    }
+    const uint32_t l = atomicExch(lo, 0u), h = atomicExch(hi, 0u);
     return ((unsigned long long)h << 32) | l;
 }
 
-// Add a histogram into the 128-bit global tally and clear it.
-// EXCHANGE = false: after a barrier.  EXCHANGE = true: by one warp while the
+// Add a histogram of the first `near` shells and the last of S into the 128-bit
+// global tally and clear it (near = S - 1: all shells), by one warp while the
 // others keep depositing: every word is taken with an atomic exchange against
 // zero.  Sums stay exact: a deposit's low-word overflow is
 // carried into a high word by the depositing lane, whichever side of an
@@ -134,36 +126,27 @@ __device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *
 // tally at one flush or the next.  probe_acc / probe_hi (shared, may be
 // null): the 128-bit running sum of the w words taken from shell
 // probe_shell.  Warp-collective.  The last shell's cells are added up first
-// (their total obeys the bound below, so it fits 64 bits).  warp_flush_cells:
-// the first n cells only, of planes of C cells.
-template <bool EXCHANGE>
-__device__ __forceinline__ void warp_flush_cells(uint32_t *tally, uint32_t n, uint32_t C, unsigned long long *g,
+// (their total obeys the bound below, so it fits 64 bits).
+__device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t near, uint32_t S, unsigned long long *g,
                                                  unsigned long long *probe_acc = nullptr,
                                                  uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
 {
-    for (uint32_t s = threadIdx.x & 31u; s < n; s += 32) {
-        const unsigned long long v = take_cell<EXCHANGE>(&tally[s], &tally[C + s]);
+    const uint32_t C = hist_cells(near + 1), lane = threadIdx.x & 31u;
+    __syncwarp();
+    for (uint32_t s = lane; s < near; s += 32) {
+        const unsigned long long v = take_cell(&tally[s], &tally[C + s]);
         flush128(&g[4 * s + 0], &g[4 * s + 1], v);
-        if (EXCHANGE && probe_acc && s == probe_shell && v) {
+        if (probe_acc && s == probe_shell && v) {
             const unsigned long long old = atomicAdd(probe_acc, v);
             if (old + v < old)
                 atomicAdd(probe_hi, 1u);
         }
-        flush128(&g[4 * s + 2], &g[4 * s + 3], take_cell<EXCHANGE>(&tally[2 * C + s], &tally[3 * C + s]));
+        flush128(&g[4 * s + 2], &g[4 * s + 3], take_cell(&tally[2 * C + s], &tally[3 * C + s]));
     }
-}
-
-__device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g,
-                                                 unsigned long long *probe_acc = nullptr,
-                                                 uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
-{
-    const uint32_t C = hist_cells(S), lane = threadIdx.x & 31u;
     __syncwarp();
-    warp_flush_cells<true>(tally, S - 1, C, g, probe_acc, probe_hi, probe_shell);
-    __syncwarp();
-    const uint32_t s = S - 1 + lane;
-    const unsigned long long v = warp_sum_u64(take_cell<true>(&tally[s], &tally[C + s]));
-    const unsigned long long v2 = warp_sum_u64(take_cell<true>(&tally[2 * C + s], &tally[3 * C + s]));
+    const uint32_t s = near + lane;
+    const unsigned long long v = warp_sum_u64(take_cell(&tally[s], &tally[C + s]));
+    const unsigned long long v2 = warp_sum_u64(take_cell(&tally[2 * C + s], &tally[3 * C + s]));
     if (lane == 0) {
         unsigned long long *gl = g + 4 * (size_t)(S - 1);
         flush128(&gl[0], &gl[1], v);
@@ -773,17 +756,20 @@ template <class M, Hist H>
 struct WeightTally {
     uint32_t hist;            // shared address of the histogram
     uint32_t plane;           // bytes between a cell's words
-    unsigned long long *g;    // global tally (H = Split)
+    unsigned long long *g;    // global tally (H = Split, Global)
     float albedo;
-    uint32_t near;            // H = Split: shells of the histogram
+    uint32_t near;            // H = Split: shells nearest to the source in the histogram,
+    uint32_t last;            // and the index of the last, behind them
     uint32_t steps = 0;
 
     __device__ __forceinline__ void deposit(uint32_t cell, float weight)
     {
         uint32_t lo, hi;
-        if (H == Hist::Global || (H == Hist::Split && cell >= near)) {
+        if (H == Hist::Global || (H == Hist::Split && cell >= near && cell < last)) {
             deposit_global(g + 4 * (size_t)cell, weight);
         } else {
+            if (H == Hist::Split && cell >= near)
+                cell = near + (threadIdx.x & 31u);
             const uint32_t at = hist + 4 * cell;
             units_split(weight_units(weight), lo, hi);
             tally_add_nowrap(at, at + plane, lo, hi);
@@ -998,10 +984,10 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
 // walk_photons with a block's histogram of 64-bit sums, 4 * hist_cells words
 // (low and high of sum w, then of sum w^2), flushed into g, the problem's global
 // 128-bit tally [shells][4], every flush_steps iterations (the caller flushes
-// what is left).  H = Split: a block histogram of 4 * near words for the first
-// `near` shells; H = Global: none.  probe_acc / probe_hi (Block only, may be
-// null): receive the w sums those flushes take from shell probe_shell.  Returns
-// this thread's photon steps.
+// what is left).  H = Split: of 4 * hist_cells(near + 1) words, for the first
+// `near` shells and the last; H = Global: none.  probe_acc / probe_hi (Block
+// only, may be null): receive the w sums those flushes take from shell
+// probe_shell.  Returns this thread's photon steps.
 template <int BLOCK, class M, class Source, Hist H>
 __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               const PhiloxKeys &keys, uint32_t *tally,
@@ -1013,29 +999,30 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
     constexpr uint32_t FLUSH = flush_steps((uint32_t)BLOCK);
     constexpr bool FAR = H == Hist::Split || H == Hist::Global;
     const float beyond = FAR ? c.last : c.last + (float)(threadIdx.x & 31u);
-    const uint32_t cells = H == Hist::Split ? near : hist_cells(c.shells);
-    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally), 4 * cells, g, c.albedo, near};
+    if constexpr (H == Hist::Block)
+        near = c.shells - 1;
+    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally), 4 * hist_cells(near + 1), g, c.albedo, near,
+                        c.shells - 1};
     walk_photons<BLOCK, M, false, FLUSH, TRIP>(c, beyond, src, keys, my, t, [&] {
-        if constexpr (H == Hist::Split)
-            warp_flush_cells<true>(tally, near, near, g);
-        else if constexpr (H != Hist::Global)
-            warp_flush_tally(tally, c.shells, g, probe_acc, probe_hi, probe_shell);
+        if constexpr (H != Hist::Global)
+            warp_flush_tally(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
     });
     return t.steps;
 }
 
-// Add what is left in a block's histogram to a 128-bit global tally
-// [shells][4], after a barrier.  Block-collective.
+// Add what is left in a block's histogram (of the first `near` shells and the
+// last of S) to a 128-bit global tally [shells][4], after a barrier.
+// Block-collective.
 template <int BLOCK>
-__device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t S, unsigned long long *g)
+__device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t near, uint32_t S, unsigned long long *g)
 {
-    const uint32_t C = hist_cells(S);
-    for (uint32_t s = threadIdx.x; s < S - 1; s += BLOCK) {
+    const uint32_t C = hist_cells(near + 1);
+    for (uint32_t s = threadIdx.x; s < near; s += BLOCK) {
         flush128(&g[4 * s + 0], &g[4 * s + 1], ((unsigned long long)tally[C + s] << 32) | tally[s]);
         flush128(&g[4 * s + 2], &g[4 * s + 3], ((unsigned long long)tally[3 * C + s] << 32) | tally[2 * C + s]);
     }
     if (threadIdx.x < 32) {
-        const uint32_t s = S - 1 + threadIdx.x;
+        const uint32_t s = near + threadIdx.x;
         const unsigned long long v = warp_sum_u64(((unsigned long long)tally[C + s] << 32) | tally[s]);
         const unsigned long long v2 = warp_sum_u64(((unsigned long long)tally[3 * C + s] << 32) | tally[2 * C + s]);
         if (threadIdx.x == 0) {
