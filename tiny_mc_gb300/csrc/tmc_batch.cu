@@ -40,7 +40,8 @@ namespace tmc {
 // thread 0 claims each item from the ring in mapped host memory, waiting with
 // back-off while nothing is published (bounded: see queue_idle_verdict), and
 // each finished item's completion is appended to the completion ring.
-template <int BLOCK, class M, bool QUEUE>
+// BODY: iterations between the walk's checks for finished photons.
+template <int BLOCK, class M, bool QUEUE, int BODY = TRIP>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_batch(const BatchArgs a)
 {
     constexpr uint32_t END = 0xffffffffu;
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_batch(const BatchArg
         unsigned long long *g = a.tally + 4 * pr.tally_offset;
         const uint32_t ps = min(a.probe_shell, S - 1);
         const bool probe = a.item_probe || a.done_ring;
-        const uint32_t steps = walk_loop<BLOCK, M, SharedSource, Hist::Block>(
+        const uint32_t steps = walk_loop<BLOCK, M, SharedSource, Hist::Block, BODY>(
             pr.c, src, a.keys, smem, g, my, 0, probe ? &sh_probe_acc : nullptr,
             probe ? &sh_probe_hi : nullptr, ps);
 
@@ -144,6 +145,9 @@ static cudaError_t walk_batch_config(int sms, size_t smem, int *grid)
 {
     auto kern = walk_batch<BLOCK, M, QUEUE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && !QUEUE)
+        e = cudaFuncSetAttribute(walk_batch<BLOCK, M, false, SHORT_TRIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
     if (e != cudaSuccess)
         return e;
     int per_sm = 0;
@@ -183,26 +187,29 @@ cudaError_t walk_batch_prepare(int block, uint32_t math, uint32_t max_shells, in
                  : batch_prepare<false>(block, fast, smem, sms, grid);
 }
 
-template <int BLOCK>
-static void batch_launch_b(const BatchArgs &a, bool fast, int grid, size_t smem, cudaStream_t s)
+template <int BLOCK, class M>
+static void batch_launch_m(const BatchArgs &a, bool brief, int grid, size_t smem, cudaStream_t s)
 {
-    if (a.q_items) {
-        if (fast) walk_batch<BLOCK, FastMath, true><<<grid, BLOCK, smem, s>>>(a);
-        else walk_batch<BLOCK, ExactMath, true><<<grid, BLOCK, smem, s>>>(a);
-    } else {
-        if (fast) walk_batch<BLOCK, FastMath, false><<<grid, BLOCK, smem, s>>>(a);
-        else walk_batch<BLOCK, ExactMath, false><<<grid, BLOCK, smem, s>>>(a);
-    }
+    if (a.q_items) walk_batch<BLOCK, M, true><<<grid, BLOCK, smem, s>>>(a);
+    else if (brief) walk_batch<BLOCK, M, false, SHORT_TRIP><<<grid, BLOCK, smem, s>>>(a);
+    else walk_batch<BLOCK, M, false><<<grid, BLOCK, smem, s>>>(a);
 }
 
-cudaError_t walk_batch_launch(const BatchArgs &a, int block, uint32_t math, int grid, cudaStream_t s)
+template <int BLOCK>
+static void batch_launch_b(const BatchArgs &a, bool fast, bool brief, int grid, size_t smem, cudaStream_t s)
+{
+    if (fast) batch_launch_m<BLOCK, FastMath>(a, brief, grid, smem, s);
+    else batch_launch_m<BLOCK, ExactMath>(a, brief, grid, smem, s);
+}
+
+cudaError_t walk_batch_launch(const BatchArgs &a, int block, uint32_t math, int grid, cudaStream_t s, bool brief)
 {
     const size_t smem = walk_batch_smem(a.max_shells, block);
     const bool fast = math == TMC_MATH_FAST;
     switch (block) {
-    case 128: batch_launch_b<128>(a, fast, grid, smem, s); break;
-    case 256: batch_launch_b<256>(a, fast, grid, smem, s); break;
-    case 512: batch_launch_b<512>(a, fast, grid, smem, s); break;
+    case 128: batch_launch_b<128>(a, fast, brief, grid, smem, s); break;
+    case 256: batch_launch_b<256>(a, fast, brief, grid, smem, s); break;
+    case 512: batch_launch_b<512>(a, fast, brief, grid, smem, s); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -248,6 +255,7 @@ struct tmc_batch {
     int device = -1;
     int sms = 0;
     int grid = 0;            // resident blocks for the current config (set by plan)
+    bool brief = false;      // most photon steps are of short walks
     size_t smem_optin = 0;
     // device buffers
     std::vector<BatchProblemDev> dev;    // d_problems' contents
@@ -481,7 +489,7 @@ cudaError_t enqueue(const tmc_batch *b, cudaStream_t s)
         return walk_stream_launch(a, b->cfg.block, b->math, grid, s);
     }
     const int grid = std::max(1, std::min<int>(b->grid, (int)b->n_items));
-    return walk_batch_launch(a, b->cfg.block, b->math, grid, s);
+    return walk_batch_launch(a, b->cfg.block, b->math, grid, s, b->brief);
 }
 
 int check_batch_device(const tmc_batch *b)
@@ -609,12 +617,16 @@ int tmc_batch_create(tmc_batch **out, const tmc_problem *problems, uint32_t n_pr
     }
     b->offsets.resize(n_problems + 1);
     std::vector<BatchProblemDev> hp(n_problems);
+    double steps = 0.0, brief_steps = 0.0;
     b->offsets[0] = 0;
     for (uint32_t i = 0; i < n_problems; ++i) {
         const tmc_problem &q = problems[i];
         const Derived d = derive(q.mu_a, q.mu_s, q.microns_per_shell, q.shells);
         b->derived.push_back(d);
         b->est_steps.push_back(expected_steps(d.albedo));
+        const double work = b->est_steps.back() * (double)q.n_photons;
+        steps += work;
+        brief_steps += d.albedo < SHORT_ALBEDO ? work : 0.0;
         hp[i].c.albedo = d.albedo;
         hp[i].c.spm = d.spm;
         hp[i].c.last = d.last;
@@ -640,6 +652,7 @@ int tmc_batch_create(tmc_batch **out, const tmc_problem *problems, uint32_t n_pr
         return r;
     }
     b->dev = std::move(hp);
+    b->brief = 2.0 * brief_steps > steps;
     *out = b.release();
     return TMC_OK;
 }

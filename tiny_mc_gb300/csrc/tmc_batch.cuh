@@ -221,7 +221,9 @@ size_t walk_batch_smem(uint32_t max_shells, int block);
 cudaError_t walk_batch_prepare(int block, uint32_t math, uint32_t max_shells, int sms, int *grid,
                                bool queue = false);
 // Launch only (capturable); walk_batch_prepare must have run for this shape.
-cudaError_t walk_batch_launch(const BatchArgs &a, int block, uint32_t math, int grid, cudaStream_t s);
+// brief: the kernel for short walks (list form), where they are most of the steps.
+cudaError_t walk_batch_launch(const BatchArgs &a, int block, uint32_t math, int grid, cudaStream_t s,
+                              bool brief = false);
 
 // The barrier-free variant (tmc_stream.cu): up to two items open per block.
 size_t walk_stream_smem(uint32_t max_shells, int block);

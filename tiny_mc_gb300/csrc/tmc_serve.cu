@@ -469,6 +469,12 @@ int launch_wave(tmc_server *s, Wave &w)
     if (n == 0)
         return TMC_OK;
     n = split_items(s, w, n);
+    double steps = 0.0, brief_steps = 0.0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const Req &q = s->active.find(s->slot_req[w.h_items[i].problem])->second;
+        steps += w.h_items[i].count * q.est_steps;
+        brief_steps += q.d.albedo < SHORT_ALBEDO ? w.h_items[i].count * q.est_steps : 0.0;
+    }
     w.n_items = n;
     w.head = 0;
     s->inflight += n;
@@ -499,7 +505,7 @@ int launch_wave(tmc_server *s, Wave &w)
                                    std::max(1, std::min<int>(s->grid, (int)n)), w.stream);
         else
             e = walk_batch_launch(a, (int)s->cfg.block, s->cfg.math,
-                                  std::max(1, std::min<int>(s->grid, (int)n)), w.stream);
+                                  std::max(1, std::min<int>(s->grid, (int)n)), w.stream, 2.0 * brief_steps > steps);
     }
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(w.h_err, w.d_counter + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost,

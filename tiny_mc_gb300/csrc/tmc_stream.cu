@@ -67,6 +67,7 @@ struct __align__(16) OpenItem {    // per buffer, in shared memory
     uint32_t count;                // photons in the item
     uint32_t claim;                // photon ids per claim; 1: the whole warp walks each
     uint32_t finish;               // the whole warp walks photons past a roulette
+    uint32_t few;                  // the whole warp walks its last photons from here on
     uint32_t ps;                   // probe shell, clamped to the problem
     uint32_t next;                 // photon counter within the item
     uint32_t done;                 // warps that reported the item
@@ -84,6 +85,7 @@ __device__ __forceinline__ void fill_item(const BatchArgs &a, OpenItem *o, const
     o->id_first = pr.id_base + itm.first;
     o->count = itm.count;
     o->finish = pr.finish;
+    o->few = warp_walk_most(pr.c.albedo);
     o->claim = pr.claim ? pr.claim : (uint32_t)BATCH_CHUNK;
     o->problem = itm.problem;
     o->ps = min(a.probe_shell, pr.c.shells - 1);
@@ -438,7 +440,8 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_stream(const BatchAr
         StreamTally<BLOCK, M> tally{smem, HS, spread, open, lane, lb, pc, pg, pps, lb, pfin, steps, want};
         // no more items and few photons left: the whole warp walks them (one
         // whose direction is still sought waits for the lane loop)
-        if (it_c == END_ITEM && __popc(alive) <= WARP_WALK_MAX)
+        if (it_c == END_ITEM && __popc(alive) <= WARP_WALK_MAX &&
+            __popc(alive) <= __reduce_min_sync(FULL_MASK, R::walking(p) ? open[lb].few : WARP_WALK_MAX))
             todo |= __ballot_sync(FULL_MASK, R::walking(p) && !(p.t > 1.0f));
         if (todo) {
             uint32_t trips = 0;

@@ -65,6 +65,8 @@ constexpr int SLOTS = RING + MIRROR;
 // photons of params.h optics: 27.8 ms with 4, 27.3 with 6, 26.9 with 8; 2^20
 // high-albedo 44.1, 42.5, 42.3; 2^22 photons of three steps (albedo 0.09)
 // 0.152, 0.169, 0.175 ms.  (Two passes through a body of 4 per check: 27.9.)
+// walk_counts and walk_batch have a kernel of each length.  (Both loops in one
+// kernel, or one that leaves a body of 8 in its middle: 1.5% slower for long walks.)
 constexpr int TRIP = 8, SHORT_TRIP = 4;
 constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the first roulette
 
@@ -73,7 +75,22 @@ constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the 
 // ~190 warp-instructions however few lanes walk, a photon's step by the whole
 // warp ~23, so 8 is where the issue slots break even.  4096-problem sweep at a
 // reduced scale: 788 ms without, 608 (6), 619 (10), 615 (16), 812 ms (24).
-constexpr int WARP_WALK_MAX = 8;
+// A round of the whole warp costs the same however few of its 32 steps are walked,
+// so short walks, whose last photons have about k / 2 steps to go (k to the first
+// roulette), go on in lanes: one photon per 8 steps of k.  Batches of short walks
+// (albedo 0.01, exact arithmetic), with four iterations per check as well: 4000
+// problems of 200 photons 260 -> 115 us in 512-thread blocks, 500 of 100000 2.34 ->
+// 1.47 ms.  The kernels for long walks keep the constant: read from a register it
+// costs them 1%.
+constexpr uint32_t WARP_WALK_MAX = 8;
+__device__ __forceinline__ uint32_t warp_walk_most(float albedo)
+{
+    const float a2 = albedo * albedo, a4 = a2 * a2, a8 = a4 * a4;   // the weight after 8 steps
+    uint32_t most = 0;
+    for (float weight = a8; most < WARP_WALK_MAX && weight >= 0.001f; weight *= a8)
+        ++most;
+    return most;
+}
 
 // Where a walk keeps its tallies.  Block: a shared histogram per block (one per
 // warp measured the same from 2^18 photons on and costs small launches more
@@ -928,6 +945,7 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
     constexpr uint32_t FLUSH_TRIPS = FLUSH / TRIP;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
+    const uint32_t few = TRIP == SHORT_TRIP ? warp_walk_most(c.albedo) : WARP_WALK_MAX;
     char *ring = reinterpret_cast<char *>(my);
 
     LanePhoton p{};
@@ -956,7 +974,7 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
             }
         }
         // -------- few photons left: the whole warp walks them one by one
-        if (idle && 32 - __popc(idle) <= WARP_WALK_MAX) {
+        if (idle && 32 - __popc(idle) <= few) {
             // (a photon whose direction is still sought waits for the lane loop)
             todo |= __ballot_sync(FULL_MASK, R::walking(p) && !(p.t > 1.0f));
         }
@@ -988,7 +1006,7 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
 // `near` shells and the last; H = Global: none.  probe_acc / probe_hi (Block
 // only, may be null): receive the w sums those flushes take from shell
 // probe_shell.  Returns this thread's photon steps.
-template <int BLOCK, class M, class Source, Hist H>
+template <int BLOCK, class M, class Source, Hist H, int BODY = TRIP>
 __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               const PhiloxKeys &keys, uint32_t *tally,
                                               unsigned long long *g, uint32_t *my, uint32_t near = 0,
@@ -1003,7 +1021,7 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
         near = c.shells - 1;
     WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally), 4 * hist_cells(near + 1), g, c.albedo, near,
                         c.shells - 1};
-    walk_photons<BLOCK, M, false, FLUSH, TRIP>(c, beyond, src, keys, my, t, [&] {
+    walk_photons<BLOCK, M, false, FLUSH, BODY>(c, beyond, src, keys, my, t, [&] {
         if constexpr (H != Hist::Global)
             warp_flush_tally(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
     });
