@@ -80,3 +80,28 @@ def test_walks_of_one_step_cost_less_than_of_ten(tmc_mod, math):
     walks of ten; a whole-warp round costs as much for either."""
     one, ten = (ms(tmc_mod, problems(4000, 200, 10.0, m), math, 512, False) for m in (0.1, 10.0))
     assert one < 0.65 * ten, (one, ten)
+
+
+@pytest.mark.parametrize("math", ["exact", "fast"])
+def test_small_batch_is_one_turn_of_lanes(tmc_mod, math):
+    """100 problems of 300 photons of three steps: a plan that gave short photons
+    to whole warps, and a launch fewer blocks than items, took walk_stream 52 us
+    where walk_batch took 24 (both about 20 us in one turn)."""
+    pr = problems(100, 300, 10.0, 1.0)
+    assert ms(tmc_mod, pr, math, 256, True) < 1.6 * ms(tmc_mod, pr, math, 256, False)
+
+
+@pytest.mark.parametrize("math", ["exact", "fast"])
+def test_equal_problems_take_one_route(tmc_mod, math):
+    """300 equal problems of long walks, one photon to a lane: the plan takes all or
+    none of them one photon to a warp, and as many blocks as there are items."""
+    pr = problems(300, 200, 0.1, 100.0)
+    assert ms(tmc_mod, pr, math, 512, False) < 1.25 * ms(tmc_mod, pr, math, 256, False)
+    b = tmc_mod.Batch(pr, seed=31, math=math)
+    b.set_config(512, 8, False, False)
+    b.run()
+    t, s = b.read()
+    b.close()
+    for i in (0, 1, 299):
+        ref, ref_steps = plain_tally(tmc_mod, pr[i], 31, math)
+        assert int(s[i]) == ref_steps and np.array_equal(as_array(b.tally_of(t, i)), ref)

@@ -312,15 +312,33 @@ struct Spread {
 // (6.9e10, up to 6.6e5): 498, 529, 589, 788.  With the longest problems one
 // photon to a warp: 73 problems (9e7 steps, up to 7e4) 7.7 ms against 41 on
 // lanes, 378 55 ms against 68.
+//
+// A warp's round is 32 steps however few of them a photon takes, so a photon's
+// last round counts whole.  An item is a photon per thread at least, so a
+// launch takes as many turns as such items fill the blocks (walk_stream's walk two
+// at a time where both fit their threads).  Without either, 100 problems of 300
+// photons of 3 steps in 256-thread blocks: 52 us in walk_stream against 23, 24 in
+// walk_batch against 19; 300 of 200 high-albedo ones in 512: 6.7 ms against 4.9.
+//
+// finish: photons past their first roulette, a tenth of all, get the whole warp
+// where lanes would take more than 0.4 of the launch for one.  256 problems in
+// walk_stream: the same from 0.1 to 0.4, 1.15 of the time at 0.8, 1.56 with it off;
+// the sweep at reduced scales the same within 5% at any.  Walks of under 64 steps,
+// a round or two behind that roulette, stay on lanes.
+constexpr double PART_ROUND = 32.0, FINISH_LEAST = 64.0;
 Spread spread(const std::vector<tmc_problem> &problems, const std::vector<double> &est_steps, int block, int most,
-              int sms, uint32_t math)
+              int sms, uint32_t math, bool stream)
 {
     std::vector<std::pair<double, double>> p;   // steps per photon and in all, longest first
-    double total = 0.0;
+    double total = 0.0, photons = 0.0, least_items = 0.0;
     for (size_t i = 0; i < problems.size(); ++i)
         if (problems[i].n_photons) {
             p.push_back({est_steps[i], est_steps[i] * (double)problems[i].n_photons});
             total += p.back().second;
+            photons += (double)problems[i].n_photons;
+            const double items = std::ceil((double)problems[i].n_photons / block);
+            const bool two = stream && 2.0 * std::ceil((double)problems[i].n_photons / items) <= block;
+            least_items += two ? items / 2.0 : items;
         }
     Spread best;
     best.per_sm = most;
@@ -333,22 +351,27 @@ Spread spread(const std::vector<tmc_problem> &problems, const std::vector<double
         const double w = k * block / 128.0;
         const double lane_rate = 2.15e11 * size / slow * w / (w + 2.3), lane_step = (0.29 + 0.045 * w) * 1e-6 * slow;
         const double warp_rate = 2.6e10 * size * std::min(1.0, w / 5.0), warp_step = std::max(0.043e-6, 0.016e-6 * w);
-        double long_work = 0.0;
+        const double turns = std::ceil(least_items / ((double)k * sms)) * total / photons * lane_step;
+        double long_work = 0.0, long_rounds = 0.0;   // steps of those problems, and 32 for every round a warp takes
         for (size_t i = 0; i <= p.size(); ++i) {   // the i longest problems' photons one to a warp
-            double t = (total - long_work) / lane_rate + long_work / warp_rate;
+            double t = (total - long_work) / lane_rate + long_rounds / warp_rate;
             if (i < p.size())
                 t = std::max(t, p[i].first * lane_step);
-            if (i)
-                t = std::max(t, p[0].first * warp_step);
-            if (t < best_t) {
+            if (i == 0)
+                t = std::max(t, turns);
+            else
+                t = std::max(t, (p[0].first + PART_ROUND) * warp_step);
+            const bool tie = i && i < p.size() && p[i].first == p[i - 1].first;   // all or none of equal lengths
+            if (t < best_t && !tie) {
                 best_t = t;
                 best.per_sm = k;
                 best.whole = i ? p[i - 1].first : 1e300;
-                best.finish = 0.4 * t / lane_step;
+                best.finish = std::max(FINISH_LEAST, 0.4 * t / lane_step);
             }
             if (i == p.size())
                 break;
             long_work += p[i].second;
+            long_rounds += p[i].second * (1.0 + PART_ROUND / p[i].first);
         }
     }
     return best;
@@ -414,7 +437,8 @@ int plan(tmc_batch *b)
     cudaError_t e = grid_for(b, &grid);   // also sets the kernel's shared-memory limit
     if (e != cudaSuccess)
         return set_cuda_error(e, "batch kernel config");
-    const Spread use = spread(b->problems, b->est_steps, b->cfg.block, grid / b->sms, b->sms, b->math);
+    const Spread use = spread(b->problems, b->est_steps, b->cfg.block, grid / b->sms, b->sms, b->math,
+                              b->cfg.stream != 0);
     grid = b->sms * use.per_sm;
     b->grid = grid;
     const std::vector<BatchItemDev> h =
