@@ -67,7 +67,7 @@ struct __align__(16) OpenItem {    // per buffer, in shared memory
     uint32_t count;                // photons in the item
     uint32_t claim;                // photon ids per claim; 1: the whole warp walks each
     uint32_t finish;               // the whole warp walks photons past a roulette
-    uint32_t few;                  // the whole warp walks its last photons from here on
+    int few;                       // the whole warp walks its last photons from here on
     uint32_t ps;                   // probe shell, clamped to the problem
     uint32_t next;                 // photon counter within the item
     uint32_t done;                 // warps that reported the item

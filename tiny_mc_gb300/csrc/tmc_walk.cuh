@@ -82,11 +82,11 @@ constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the 
 // problems of 200 photons 260 -> 115 us in 512-thread blocks, 500 of 100000 2.34 ->
 // 1.47 ms.  The kernels for long walks keep the constant: read from a register it
 // costs them 1%.
-constexpr uint32_t WARP_WALK_MAX = 8;
-__device__ __forceinline__ uint32_t warp_walk_most(float albedo)
+constexpr int WARP_WALK_MAX = 8;
+__device__ __forceinline__ int warp_walk_most(float albedo)
 {
     const float a2 = albedo * albedo, a4 = a2 * a2, a8 = a4 * a4;   // the weight after 8 steps
-    uint32_t most = 0;
+    int most = 0;
     for (float weight = a8; most < WARP_WALK_MAX && weight >= 0.001f; weight *= a8)
         ++most;
     return most;
@@ -116,14 +116,18 @@ __host__ __device__ constexpr uint32_t flush_steps(uint32_t lanes)
 }
 static_assert(512ull * 257ull * ((1ull << 23) / 512 + 1) < (1ull << 32), "high word bound");
 
-// Cells of a shared histogram.  Every photon beyond the last shell deposits
+// Cells of a shared histogram or row of counts.  Every photon beyond the last shell deposits
 // into it (photon.c:27-29): in an optically thin problem nearly all lanes of a
 // warp at once, and shared atomics on one word take their turns.  So the last
 // shell has 32 cells, one per lane, which the flushes add up.  2^20 high-albedo
 // photons (1001 shells of 10 um, many walks leave): 46.8 -> 44.8 ms; the reduced
-// 4096-problem sweep 609 -> 555 ms.  In the split form, where they would be
-// global atomics on one address, 2^21 photons of params.h optics over 4600 shells
-// of 0.53 um: 128.7 ms without the cells, 1.18 with them.
+// 4096-problem sweep 609 -> 555 ms.  A histogram of sums has them before shell 0, lane
+// l's at -1 - l; counts have them in the last shell's place.
+// The split form uses the one at -1 alone: as global atomics on one address 2^21
+// photons of params.h optics over 4600 shells of 0.53 um took 128.7 ms, 1.65 so, 1.16
+// with a cell per lane; but where few photons leave (2000003 photons, 20000 shells of
+// 5 um) 1.007 ms so, 1.023 with a lane's own constant held through the loop, 1.045
+// with the cells behind the near shells (a second compare and a branch's join).
 constexpr uint32_t LAST_CELLS = 32;
 __host__ __device__ constexpr uint32_t hist_cells(uint32_t shells) { return shells + LAST_CELLS - 1; }
 
@@ -150,20 +154,20 @@ __device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t near,
 {
     const uint32_t C = hist_cells(near + 1), lane = threadIdx.x & 31u;
     __syncwarp();
+    uint32_t *const first = tally + LAST_CELLS;
     for (uint32_t s = lane; s < near; s += 32) {
-        const unsigned long long v = take_cell(&tally[s], &tally[C + s]);
+        const unsigned long long v = take_cell(&first[s], &first[C + s]);
         flush128(&g[4 * s + 0], &g[4 * s + 1], v);
         if (probe_acc && s == probe_shell && v) {
             const unsigned long long old = atomicAdd(probe_acc, v);
             if (old + v < old)
                 atomicAdd(probe_hi, 1u);
         }
-        flush128(&g[4 * s + 2], &g[4 * s + 3], take_cell(&tally[2 * C + s], &tally[3 * C + s]));
+        flush128(&g[4 * s + 2], &g[4 * s + 3], take_cell(&first[2 * C + s], &first[3 * C + s]));
     }
     __syncwarp();
-    const uint32_t s = near + lane;
-    const unsigned long long v = warp_sum_u64(take_cell(&tally[s], &tally[C + s]));
-    const unsigned long long v2 = warp_sum_u64(take_cell(&tally[2 * C + s], &tally[3 * C + s]));
+    const unsigned long long v = warp_sum_u64(take_cell(&tally[lane], &tally[C + lane]));
+    const unsigned long long v2 = warp_sum_u64(take_cell(&tally[2 * C + lane], &tally[3 * C + lane]));
     if (lane == 0) {
         unsigned long long *gl = g + 4 * (size_t)(S - 1);
         flush128(&gl[0], &gl[1], v);
@@ -458,7 +462,7 @@ __device__ __forceinline__ void launch_photon(LanePhoton &p, unsigned long long 
 // for the next refill): move, deposit and decay unless its direction is still
 // sought, then two tries for the next direction and the roulette.
 // A radius below `last` shells goes to its shell's cell, any other (NaN too) to
-// cell `beyond`.  The tally keeps the photon's weight: step(p, cell) deposits
+// cell `beyond`, which may be negative.  The tally keeps the photon's weight: step(p, cell) deposits
 // and decays it, low(p) says whether it is below the roulette's threshold,
 // survived(p) and died(p) are the roulette's outcomes.
 template <int BLOCK, class M, class Tally>
@@ -478,7 +482,7 @@ __device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, flo
         // absorb, photon.c:26-32 (clamp in float: same shell for every radius
         // below 2^32 shells)
         const float r = M::radius_shells(p.x, p.y, p.z, spm);
-        tally.step(p, __float2uint_rz(r < last ? r : beyond));
+        tally.step(p, (uint32_t)__float2int_rz(r < last ? r : beyond));
     }
     // the next two tries of the rejection method, photon.c:36-40; the second
     // one's words are consumed only if the first is rejected
@@ -685,7 +689,7 @@ __device__ __forceinline__ uint32_t warp_steps(WarpPhoton &p, bool &dead, const 
     if (low)
         n = __ffs((int)low);   // the steps up to the first roulette
     const float radius = M::radius_shells(x, y, z, c.spm);
-    cell_out = __float2uint_rz(radius < c.last ? radius : beyond);
+    cell_out = (uint32_t)__float2int_rz(radius < c.last ? radius : beyond);
     weight_out = weight;
 
     const int l = (int)n - 1;
@@ -771,22 +775,19 @@ struct Optics {
 
 template <class M, Hist H>
 struct WeightTally {
-    uint32_t hist;            // shared address of the histogram
+    uint32_t hist;            // shared address of the histogram's shell 0
     uint32_t plane;           // bytes between a cell's words
     unsigned long long *g;    // global tally (H = Split, Global)
     float albedo;
-    uint32_t near;            // H = Split: shells nearest to the source in the histogram,
-    uint32_t last;            // and the index of the last, behind them
+    int near;                 // H = Split: shells nearest to the source in the histogram
     uint32_t steps = 0;
 
-    __device__ __forceinline__ void deposit(uint32_t cell, float weight)
+    __device__ __forceinline__ void deposit(int cell, float weight)
     {
         uint32_t lo, hi;
-        if (H == Hist::Global || (H == Hist::Split && cell >= near && cell < last)) {
+        if (H == Hist::Global || (H == Hist::Split && cell >= near)) {
             deposit_global(g + 4 * (size_t)cell, weight);
         } else {
-            if (H == Hist::Split && cell >= near)
-                cell = near + (threadIdx.x & 31u);
             const uint32_t at = hist + 4 * cell;
             units_split(weight_units(weight), lo, hi);
             tally_add_nowrap(at, at + plane, lo, hi);
@@ -798,7 +799,7 @@ struct WeightTally {
     __device__ __forceinline__ void launched() {}
     __device__ __forceinline__ void step(LanePhoton &p, uint32_t cell)
     {
-        deposit(cell, p.weight);
+        deposit((int)cell, p.weight);
         p.weight = M::mul(p.weight, albedo);
     }
     __device__ __forceinline__ bool low(const LanePhoton &p) const { return p.weight < 0.001f * WEIGHT_ONE; }
@@ -809,7 +810,7 @@ struct WeightTally {
     __device__ __forceinline__ uint32_t row_of(const LanePhoton &) const { return 0; }
     __device__ __forceinline__ uint32_t row_after(uint32_t, uint32_t) const { return 0; }
     __device__ __forceinline__ void resume(LanePhoton &, uint32_t) {}
-    __device__ __forceinline__ void whole(uint32_t, uint32_t cell, float weight) { deposit(cell, weight); }
+    __device__ __forceinline__ void whole(uint32_t, uint32_t cell, float weight) { deposit((int)cell, weight); }
     __device__ __forceinline__ void walked(int, uint32_t) {}
 };
 
@@ -945,7 +946,7 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
     constexpr uint32_t FLUSH_TRIPS = FLUSH / TRIP;
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lt_mask = (1u << lane) - 1u;
-    const uint32_t few = TRIP == SHORT_TRIP ? warp_walk_most(c.albedo) : WARP_WALK_MAX;
+    const int few = TRIP == SHORT_TRIP ? warp_walk_most(c.albedo) : WARP_WALK_MAX;
     char *ring = reinterpret_cast<char *>(my);
 
     LanePhoton p{};
@@ -1015,12 +1016,11 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               uint32_t probe_shell = 0)
 {
     constexpr uint32_t FLUSH = flush_steps((uint32_t)BLOCK);
-    constexpr bool FAR = H == Hist::Split || H == Hist::Global;
-    const float beyond = FAR ? c.last : c.last + (float)(threadIdx.x & 31u);
+    const float beyond = H == Hist::Global ? c.last : H == Hist::Split ? -1.0f : -1.0f - (float)(threadIdx.x & 31u);
     if constexpr (H == Hist::Block)
         near = c.shells - 1;
-    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally), 4 * hist_cells(near + 1), g, c.albedo, near,
-                        c.shells - 1};
+    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally + LAST_CELLS), 4 * hist_cells(near + 1), g, c.albedo,
+                        (int)near};
     walk_photons<BLOCK, M, false, FLUSH, BODY>(c, beyond, src, keys, my, t, [&] {
         if constexpr (H != Hist::Global)
             warp_flush_tally(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
@@ -1035,12 +1035,13 @@ template <int BLOCK>
 __device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t near, uint32_t S, unsigned long long *g)
 {
     const uint32_t C = hist_cells(near + 1);
+    const uint32_t *const first = tally + LAST_CELLS;
     for (uint32_t s = threadIdx.x; s < near; s += BLOCK) {
-        flush128(&g[4 * s + 0], &g[4 * s + 1], ((unsigned long long)tally[C + s] << 32) | tally[s]);
-        flush128(&g[4 * s + 2], &g[4 * s + 3], ((unsigned long long)tally[3 * C + s] << 32) | tally[2 * C + s]);
+        flush128(&g[4 * s + 0], &g[4 * s + 1], ((unsigned long long)first[C + s] << 32) | first[s]);
+        flush128(&g[4 * s + 2], &g[4 * s + 3], ((unsigned long long)first[3 * C + s] << 32) | first[2 * C + s]);
     }
     if (threadIdx.x < 32) {
-        const uint32_t s = near + threadIdx.x;
+        const uint32_t s = threadIdx.x;
         const unsigned long long v = warp_sum_u64(((unsigned long long)tally[C + s] << 32) | tally[s]);
         const unsigned long long v2 = warp_sum_u64(((unsigned long long)tally[3 * C + s] << 32) | tally[2 * C + s]);
         if (threadIdx.x == 0) {
@@ -1055,9 +1056,9 @@ __device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t near, uint
 __device__ __forceinline__ unsigned long long shell_sum(const uint32_t *tally, uint32_t S, uint32_t s)
 {
     const uint32_t C = hist_cells(S);
+    const uint32_t at = s + 1 < S ? LAST_CELLS + s : threadIdx.x & 31u;
     if (s + 1 < S)
-        return ((unsigned long long)tally[C + s] << 32) | tally[s];
-    const uint32_t at = s + (threadIdx.x & 31u);
+        return ((unsigned long long)tally[C + at] << 32) | tally[at];
     return warp_sum_u64(((unsigned long long)tally[C + at] << 32) | tally[at]);
 }
 
