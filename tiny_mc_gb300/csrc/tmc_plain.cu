@@ -382,8 +382,19 @@ cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_
     // Sums take blocks of 128 threads where eight histograms fit an SM: they
     // spread small launches over more SMs (32768 photons on 64 blocks of 512
     // took 114 us, 84 on 256 of 128) and end one by one (2^18 high-albedo
-    // photons 13.3 -> 12.5 ms).  More shells take them below 512 photons per SM.
-    const bool blocks128 = hist_cells(L.d.shells) <= split_cells(128) || per_sm < 512;
+    // photons 13.3 -> 12.5 ms).  More shells take them below 512 photons per SM:
+    // with walks of 73 steps, of the time of 512-thread blocks, 0.8 - 1.1 at 1100 ..
+    // 2500 shells and 100 - 300 photons per SM, 1.2 - 1.3 at 500; past 2900 shells,
+    // where fewer than four blocks fit an SM, they lose (4000 shells 1.0 - 1.4, 7000
+    // 1.0 - 2), but from 11810 on only they have room for a histogram (12000 shells
+    // of 0.1 um, 60000 photons 0.20 ms against 5.2).  Short walks take 512 at any
+    // size that has a histogram there: setting a small block's up and adding it is
+    // most of their time (75000 photons at 10/cm and 1/cm: 7000 shells 61 us against
+    // 29, 12000 of 0.3 um 83 against 29).
+    const bool hist512 = plain_smem_bytes(L.d.shells, 512, Hist::Block) <= ctx.smem_optin ||
+                         reaches(split_near(512, L.d.shells), L.d);
+    const bool blocks128 = hist_cells(L.d.shells) <= split_cells(128) ||
+                           (per_sm < 512 && !(L.d.albedo < SHORT_ALBEDO && hist512));
     // a launch of no photons is a caller's set-up call: it loads every kernel
     // a call of its arithmetic may take
     if (L.n_photons == 0 && !L.block) {
