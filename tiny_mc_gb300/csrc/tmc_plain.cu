@@ -10,8 +10,8 @@
 // Shell counts whose histogram leaves no room for the SM's blocks (params.h's
 // SHELLS is any size in the reference) take the split form: a histogram of the
 // shells nearest to the source and of the last one, and 64-bit atomics on the
-// 128-bit global tally between them; or, with shells so thin that most deposits land beyond it, no
-// histogram at all.  The sums are the same integers in every form.
+// 128-bit global tally between them; or, with shells so thin that most deposits
+// land beyond it, of the last one alone.  The sums are the same integers in every form.
 #include <algorithm>
 #include <cmath>
 
@@ -73,16 +73,17 @@ __host__ __device__ constexpr uint32_t split_near(int block, uint32_t shells)   
 }
 static_assert(split_cells(512) == 4544 && split_cells(128) % 4 == 0, "whole 16-byte rows of the ring behind it");
 
-// Two blocks of 512 threads per SM, three where every deposit waits for the L2
-// (200000 shells of 0.1 um, 2^20 photons: 2.2 ms with two, 1.32 with three).
+// 1024 threads per SM.  Where each deposit waits for the L2 (200000 shells of 0.1
+// um) 1536 at 40 registers spill in the whole warp's walk: 2^20 photons 1.31 ms
+// against 1.21, 2^24 19.43 against 18.10.
 template <int BLOCK, class M, Hist H>
-__global__ void __launch_bounds__(BLOCK, (H == Hist::Global ? 1536 : 1024) / BLOCK) walk_plain(const PlainArgs a)
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArgs a)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t S = a.c.shells;
-    const uint32_t near = H == Hist::Split ? split_near(BLOCK, S) : S - 1;
+    const uint32_t near = H == Hist::Split ? split_near(BLOCK, S) : H == Hist::Far ? 0 : S - 1;
     // words per histogram
-    const uint32_t hist = 4 * (H == Hist::Split ? split_cells(BLOCK) : H == Hist::Global ? 0 : hist_cells(S));
+    const uint32_t hist = 4 * (H == Hist::Split ? split_cells(BLOCK) : hist_cells(near + 1));
     for (uint32_t s = threadIdx.x; s < hist; s += BLOCK)
         smem[s] = 0;
     __syncthreads();
@@ -93,13 +94,13 @@ __global__ void __launch_bounds__(BLOCK, (H == Hist::Global ? 1536 : 1024) / BLO
     src.id_base = a.id_base;
     src.chunk = a.chunk;
     uint32_t *my = smem + hist + threadIdx.x;   // ring slot k: my[k * BLOCK]
-    const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H>(
+    // (a body of four iterations where each deposit waits: 2^24 photons of three steps
+    // over 200000 shells, exact arithmetic, 0.97 ms with eight, 0.81 with four)
+    const uint32_t steps = walk_loop<BLOCK, M, GlobalSource, H, H == Hist::Far ? SHORT_TRIP : TRIP>(
         a.c, src, a.keys, smem, a.tally, my, near);
 
-    if constexpr (H != Hist::Global) {
-        __syncthreads();
-        flush_tally<BLOCK>(smem, near, S, a.tally);
-    }
+    __syncthreads();
+    flush_tally<BLOCK>(smem, near, S, a.tally);
     if (a.steps) {
         const unsigned long long tot = warp_sum_u64(steps);
         if ((threadIdx.x & 31u) == 0 && tot)
@@ -206,8 +207,8 @@ static uint32_t count_rows(const Derived &d, size_t smem_optin)
 
 static size_t plain_smem_bytes(uint32_t shells, int block, Hist h)
 {
-    const size_t cells = h == Hist::Split ? split_cells(block) : h == Hist::Global ? 0 : hist_cells(shells);
-    return 16 * cells + (size_t)4 * SLOTS * block;
+    const uint32_t cells = h == Hist::Split ? split_cells(block) : hist_cells(h == Hist::Far ? 1 : shells);
+    return (size_t)16 * cells + (size_t)4 * SLOTS * block;
 }
 
 template <int BLOCK, class M, Hist H>
@@ -303,11 +304,11 @@ static cudaError_t launch_counts(const PlainLaunch &L, const DeviceCtx &ctx, uin
 }
 
 // The split form pays where its histogram reaches far enough: a walk of k steps
-// of about a mean free path ends about sqrt(k) of them out.  With 4544 shells,
-// 2^20 photons and params.h optics (k = 73): shells of 0.4 um (reach 0.47 sqrt(k))
-// 1.74 ms split, 1.47 global; 0.8 um (0.94) 0.99, 1.59; 5 um 0.56, 3.48.  At
-// albedo 0.09 (k = 3): 0.05 um (0.14) 0.207, 0.146; 0.2 um (0.6) 0.156, 0.150;
-// 0.5 um 0.126, 0.168.
+// of about a mean free path ends about sqrt(k) of them out.  512-thread blocks (4512
+// shells), 2^20 photons over 20000 shells at params.h optics (k = 73): 0.34 um (a
+// reach of 0.4) 1.70 ms split, 1.22 far; 0.52 um (0.6) 1.49, 1.34; 0.60 um (0.7)
+// 1.33, 1.46; 0.86 um (1.0) 0.93, 1.55; 1.7 um 0.65, 1.67.  At albedo 0.09 (k = 3)
+// either within 20%: 0.24 um (0.6) 0.088, 0.074; 0.8 um (2.0) 0.078, 0.091.
 static bool reaches(uint32_t shells, const Derived &d)
 {
     const double k = d.albedo > 0.0f ? std::log(0.001) / std::log((double)d.albedo) : 0.0;
@@ -324,10 +325,9 @@ static cudaError_t try_launch(const PlainLaunch &L, const DeviceCtx &ctx, cudaSt
 
 // A histogram per block where it leaves the SM its 1024 threads, else the split
 // form where it reaches (8000 shells of 12.5 um, 2^21 photons of params.h
-// optics: one block per SM 1.26 ms, split 1.02; 20000 shells of 5 um: 5.25 ms
-// global, 1.02 split), else a block's histogram at any occupancy (4001 shells of
-// 1 um, 5000 photons: 1.2 ms global, 55 us with three blocks of 128 threads per
-// SM), else global.
+// optics: one block per SM 1.26 ms, split 1.02; but of 0.86 um, 2^20 photons, 0.66
+// and 0.90), else a block's histogram at any occupancy (8000 shells of 0.35 um: one
+// block per SM 0.66 ms, far 1.13), else far.
 template <int BLOCK, class M>
 static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_t stream)
 {
@@ -342,7 +342,7 @@ static cudaError_t launch_m(const PlainLaunch &L, const DeviceCtx &ctx, cudaStre
         return try_launch<BLOCK, M, Hist::Split>(L, ctx, stream);
     if (block_sm >= 1)
         return launch_t<BLOCK, M, Hist::Block>(L, ctx, block_sm, stream);
-    return try_launch<BLOCK, M, Hist::Global>(L, ctx, stream);
+    return try_launch<BLOCK, M, Hist::Far>(L, ctx, stream);
 }
 
 template <int BLOCK>
@@ -356,9 +356,9 @@ template <class M>
 static cudaError_t load_kernels()
 {
     const void *kernels[] = {
-        (const void *)walk_plain<128, M, Hist::Block>,  (const void *)walk_plain<128, M, Hist::Split>,
-        (const void *)walk_plain<128, M, Hist::Global>, (const void *)walk_plain<512, M, Hist::Block>,
-        (const void *)walk_plain<512, M, Hist::Split>,  (const void *)walk_plain<512, M, Hist::Global>,
+        (const void *)walk_plain<128, M, Hist::Block>, (const void *)walk_plain<128, M, Hist::Split>,
+        (const void *)walk_plain<128, M, Hist::Far>,   (const void *)walk_plain<512, M, Hist::Block>,
+        (const void *)walk_plain<512, M, Hist::Split>, (const void *)walk_plain<512, M, Hist::Far>,
         (const void *)walk_counts<M, TRIP>, (const void *)walk_counts<M, SHORT_TRIP>};
     for (const void *k : kernels) {
         cudaFuncAttributes attr;
@@ -384,17 +384,12 @@ cudaError_t launch_plain(const PlainLaunch &L, const DeviceCtx &ctx, cudaStream_
     // took 114 us, 84 on 256 of 128) and end one by one (2^18 high-albedo
     // photons 13.3 -> 12.5 ms).  More shells take them below 512 photons per SM:
     // with walks of 73 steps, of the time of 512-thread blocks, 0.8 - 1.1 at 1100 ..
-    // 2500 shells and 100 - 300 photons per SM, 1.2 - 1.3 at 500; past 2900 shells,
-    // where fewer than four blocks fit an SM, they lose (4000 shells 1.0 - 1.4, 7000
-    // 1.0 - 2), but from 11810 on only they have room for a histogram (12000 shells
-    // of 0.1 um, 60000 photons 0.20 ms against 5.2).  Short walks take 512 at any
-    // size that has a histogram there: setting a small block's up and adding it is
-    // most of their time (75000 photons at 10/cm and 1/cm: 7000 shells 61 us against
-    // 29, 12000 of 0.3 um 83 against 29).
-    const bool hist512 = plain_smem_bytes(L.d.shells, 512, Hist::Block) <= ctx.smem_optin ||
-                         reaches(split_near(512, L.d.shells), L.d);
+    // 2500 shells and 100 - 300 photons per SM, 1.2 - 1.3 at 500 (past 2900 shells,
+    // where fewer than four blocks fit an SM, 1.0 - 2).  Short walks take 512: setting
+    // a small block's histogram up and adding it is most of their time (75000 photons
+    // at 10/cm and 1/cm: 7000 shells 61 us against 29, 12000 of 0.3 um 83 against 29).
     const bool blocks128 = hist_cells(L.d.shells) <= split_cells(128) ||
-                           (per_sm < 512 && !(L.d.albedo < SHORT_ALBEDO && hist512));
+                           (per_sm < 512 && L.d.albedo >= SHORT_ALBEDO);
     // a launch of no photons is a caller's set-up call: it loads every kernel
     // a call of its arithmetic may take
     if (L.n_photons == 0 && !L.block) {

@@ -98,10 +98,9 @@ __device__ __forceinline__ int warp_walk_most(float albedo)
 // the shells nearest to the source, where nearly all deposits of a point source
 // land, and the last one, and a deposit between them is a 64-bit atomic add into
 // the 128-bit global tally (shell counts whose histogram does not fit in shared
-// memory).  Global:
-// every deposit is (shells so thin that most land beyond such a histogram).
-// Counts have a tally of their own (CountTally).
-enum class Hist { Block, Split, Global };
+// memory).  Far: the last one alone (shells so thin that most deposits land beyond
+// such a histogram).  Counts have a tally of their own (CountTally).
+enum class Hist { Block, Split, Far };
 
 // A warp adds its block's histogram, of `lanes` lanes, into the global tally and
 // clears it every flush_steps(lanes) of its iterations.  A lane deposits at most once per
@@ -777,7 +776,7 @@ template <class M, Hist H>
 struct WeightTally {
     uint32_t hist;            // shared address of the histogram's shell 0
     uint32_t plane;           // bytes between a cell's words
-    unsigned long long *g;    // global tally (H = Split, Global)
+    unsigned long long *g;    // global tally (H = Split, Far)
     float albedo;
     int near;                 // H = Split: shells nearest to the source in the histogram
     uint32_t steps = 0;
@@ -785,7 +784,7 @@ struct WeightTally {
     __device__ __forceinline__ void deposit(int cell, float weight)
     {
         uint32_t lo, hi;
-        if (H == Hist::Global || (H == Hist::Split && cell >= near)) {
+        if (H != Hist::Block && cell >= (H == Hist::Far ? 0 : near)) {
             deposit_global(g + 4 * (size_t)cell, weight);
         } else {
             const uint32_t at = hist + 4 * cell;
@@ -1003,9 +1002,9 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
 // walk_photons with a block's histogram of 64-bit sums, 4 * hist_cells words
 // (low and high of sum w, then of sum w^2), flushed into g, the problem's global
 // 128-bit tally [shells][4], every flush_steps iterations (the caller flushes
-// what is left).  H = Split: of 4 * hist_cells(near + 1) words, for the first
-// `near` shells and the last; H = Global: none.  probe_acc / probe_hi (Block
-// only, may be null): receive the w sums those flushes take from shell
+// what is left).  H = Split, Far: of 4 * hist_cells(near + 1) words, for the first
+// `near` (Far: no) shells and the last.  probe_acc / probe_hi (Block only, may be null):
+// receive the w sums those flushes take from shell
 // probe_shell.  Returns this thread's photon steps.
 template <int BLOCK, class M, class Source, Hist H, int BODY = TRIP>
 __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
@@ -1016,14 +1015,13 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               uint32_t probe_shell = 0)
 {
     constexpr uint32_t FLUSH = flush_steps((uint32_t)BLOCK);
-    const float beyond = H == Hist::Global ? c.last : H == Hist::Split ? -1.0f : -1.0f - (float)(threadIdx.x & 31u);
+    const float beyond = H != Hist::Block ? -1.0f : -1.0f - (float)(threadIdx.x & 31u);
     if constexpr (H == Hist::Block)
         near = c.shells - 1;
     WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally + LAST_CELLS), 4 * hist_cells(near + 1), g, c.albedo,
                         (int)near};
     walk_photons<BLOCK, M, false, FLUSH, BODY>(c, beyond, src, keys, my, t, [&] {
-        if constexpr (H != Hist::Global)
-            warp_flush_tally(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
+        warp_flush_tally(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
     });
     return t.steps;
 }
