@@ -341,8 +341,12 @@ typedef struct tmc_server_config {
                                        end once none are (waves does not apply).  Higher
                                        capacity and lower latency than waves, but while
                                        requests are active it holds the SMs: other work on
-                                       the GPU waits for it (the default, 0, leaves room
-                                       between launches) */
+                                       the GPU waits for it, but for kernels of up to 256
+                                       threads a block and 32 registers without shared
+                                       memory (the colour map, the FP64 report), which it
+                                       leaves room for unless one block's histograms take
+                                       an SM's whole shared memory (the default, 0, leaves
+                                       room between launches) */
 } tmc_server_config;
 
 typedef struct tmc_server tmc_server;

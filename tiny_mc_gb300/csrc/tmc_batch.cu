@@ -42,7 +42,7 @@ namespace tmc {
 // each finished item's completion is appended to the completion ring.
 // BODY: iterations between the walk's checks for finished photons.
 template <int BLOCK, class M, bool QUEUE, int BODY = TRIP>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_batch(const BatchArgs a)
+__global__ void __launch_bounds__(bound_threads(BLOCK, QUEUE), 1024 / BLOCK) walk_batch(const BatchArgs a)
 {
     constexpr uint32_t END = 0xffffffffu;
     extern __shared__ __align__(16) uint32_t smem[];
@@ -140,6 +140,31 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_batch(const BatchArg
         queue_block_end(a);
 }
 
+cudaError_t queue_blocks(const void *kernel, int block, size_t smem, int &per_sm)
+{
+    cudaFuncAttributes attr;
+    int dev = 0, regs = 0, threads = 0, shared = 0;
+    cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
+    if (e == cudaSuccess)
+        e = cudaGetDevice(&dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&threads, cudaDevAttrMaxThreadsPerMultiProcessor, dev);
+    if (e == cudaSuccess)
+        e = cudaDeviceGetAttribute(&shared, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+    if (e != cudaSuccess)
+        return e;
+    const size_t own = 1024;   // shared memory the system takes per block
+    auto room = [&](int n) {   // beside n blocks
+        return regs - n * block * ((attr.numRegs + 7) / 8 * 8) >= BESIDE_THREADS * BESIDE_REGS &&
+               threads - n * block >= BESIDE_THREADS && (size_t)n * (smem + attr.sharedSizeBytes + own) + own <= (size_t)shared;
+    };
+    while (per_sm > 1 && !room(per_sm))
+        --per_sm;
+    return cudaSuccess;
+}
+
 template <int BLOCK, class M, bool QUEUE>
 static cudaError_t walk_batch_config(int sms, size_t smem, int *grid)
 {
@@ -156,8 +181,10 @@ static cudaError_t walk_batch_config(int sms, size_t smem, int *grid)
         return e;
     if (per_sm < 1)
         return cudaErrorInvalidConfiguration;
-    *grid = sms * (QUEUE ? queue_blocks(per_sm) : per_sm);
-    return cudaSuccess;
+    if (QUEUE)
+        e = queue_blocks((const void *)kern, BLOCK, smem, per_sm);
+    *grid = sms * per_sm;
+    return e;
 }
 
 size_t walk_batch_smem(uint32_t max_shells, int block)

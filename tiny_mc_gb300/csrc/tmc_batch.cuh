@@ -117,13 +117,23 @@ __device__ __forceinline__ void publish_item_at(const BatchArgs &a, unsigned lon
 // -------------------------------------------- queue mode (persistent server)
 constexpr unsigned long long QUEUE_DEFAULT_WAIT_LIMIT_NS = 120ull * 1000000000ull;
 
-// Blocks per SM of a persistent launch.  Eight blocks of 128 threads take every
-// register of an SM, and as the launch waits for the host between items, a colour
-// map or a report that the host waits for would never start.  One block less
-// leaves 8192, enough for a block of either (256 threads of 24 and 32 registers).
-// Saturated stream: 1.767e11 photon steps/s with eight, 1.746 with seven; p50 at
-// 70% load 64 and 49 ms.
-inline int queue_blocks(int per_sm) { return per_sm >= 8 ? 7 : per_sm; }
+// A persistent launch waits for the host between items, so a colour map or a
+// report that the host waits for must find room beside it: a block of 256 threads
+// of up to 32 registers, with no shared memory but the 1 KB of every block.  1024
+// threads of 64 registers take all of an SM's.  Blocks of 128 threads leave room by
+// being seven instead of eight; a block less of larger ones would idle a quarter or
+// half of the SM, so the queue forms for those are held to 56 registers (by launch
+// bounds of a ninth more threads).  Saturated server, 1e11 photon steps/s, fast and
+// exact arithmetic: 128 threads 1.60 and 1.15 with seven blocks of 64, 1.58 and 1.18
+// with eight of 56; 256 1.65 and 1.19 with three, 1.62 and 1.21 with four of 56; 512
+// 1.47 and 1.07 with one, 1.59 and 1.20 with two of 56 (walk_stream: 1.27 and 1.04,
+// 1.15 and 0.97; 1.26 and 1.05, 1.30 and 1.08; 1.21 and 0.92, 1.33 and 1.09).
+constexpr int BESIDE_THREADS = 256, BESIDE_REGS = 32;
+constexpr int bound_threads(int block, bool queue) { return queue && block > 128 ? block + block / 8 : block; }
+
+// Blocks per SM of a persistent launch, given those that fit an empty SM: as many
+// as leave that room (one at least).
+cudaError_t queue_blocks(const void *kernel, int block, size_t smem, int &per_sm);
 
 __device__ __forceinline__ unsigned long long global_ns()
 {

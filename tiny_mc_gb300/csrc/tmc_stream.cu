@@ -205,7 +205,7 @@ struct StreamTally {
 }  // namespace
 
 template <int BLOCK, class M, bool QUEUE>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_stream(const BatchArgs a)
+__global__ void __launch_bounds__(bound_threads(BLOCK, QUEUE), 1024 / BLOCK) walk_stream(const BatchArgs a)
 {
     constexpr unsigned NWARPS = BLOCK / 32;
     extern __shared__ __align__(16) uint32_t smem[];
@@ -488,8 +488,10 @@ static cudaError_t stream_config(int sms, size_t smem, int *grid)
         return e;
     if (per_sm < 1)
         return cudaErrorInvalidConfiguration;
-    *grid = sms * (QUEUE ? queue_blocks(per_sm) : per_sm);
-    return cudaSuccess;
+    if (QUEUE)
+        e = queue_blocks((const void *)kern, BLOCK, smem, per_sm);
+    *grid = sms * per_sm;
+    return e;
 }
 
 template <bool QUEUE>
