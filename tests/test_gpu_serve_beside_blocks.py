@@ -44,3 +44,34 @@ def test_small_calls_beside_any_block_size(tmc_mod, block, stream, math, max_she
     assert took < 20.0
     assert same(before, beside)
     assert all(r["photons"] for _, r in out.values())
+
+
+@pytest.mark.parametrize("stream", [0, 1])
+@pytest.mark.parametrize("block", [128, 512])
+def test_small_calls_beside_a_relaunch(tmc_mod, block, stream):
+    """Requests that arrive right after the server has run dry (its blocks wait 20
+    ms before they end): the next launch does not share the SMs with the last one."""
+    from tiny_mc_gb300.serve import Server
+    p = tmc_mod.params(seed=1)
+    tally, _ = tmc_mod.photon_batch_fx(2000, p)
+    before = small_calls(tmc_mod, tally, p)
+    s = Server(slots=8, persistent=1, block=block, stream=stream)
+    for k in range(3):
+        short = req(2.0, 20.0, 101, 0.05, cap=1 << 18, base=(9 + k) << 32)
+        rid = s.submit(short)
+        assert s.run({rid: 101})[rid][1]["photons"]
+        s.progress()                                     # nothing active: drain
+        ids = {s.submit(r): int(r["shells"]) for r in LONG}
+        launches = s.stats()[2] + 1
+        t0 = time.monotonic()
+        while s.stats()[2] < launches and time.monotonic() - t0 < 5.0:
+            in_flight, _ = s.progress()
+        assert in_flight == 1                            # the last launch has ended
+        beside = small_calls(tmc_mod, tally, p)
+        took = time.monotonic() - t0
+        out = s.run(ids)
+        assert took < 20.0
+        assert same(before, beside)
+        assert all(r["photons"] for _, r in out.values())
+        assert s.stats()[2] == launches
+    s.close()

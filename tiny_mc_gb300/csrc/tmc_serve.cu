@@ -37,7 +37,7 @@
 //    appended to a completion ring the host reads from its head.  The blocks
 //    wait for more work
 //    while requests are active and end once none are; the next admission
-//    launches the kernel again.
+//    launches the kernel again, after the last launch has ended.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -653,27 +653,25 @@ int progress_persistent(tmc_server *s)
     int st = harvest_queue(s);
     if (st)
         return st;
-    // blocks wait for work while requests are active, and end once none are
-    const unsigned mode = s->active.empty() ? QUEUE_DRAIN : QUEUE_HOLD;
+    // blocks wait for work while requests are active, and end once none are.  A
+    // launch that was told to drain may have lost blocks by now, and a second one
+    // beside what is left of it would fill the room it leaves for small kernels
+    // (queue_blocks): it is told to end, tens of microseconds with nothing published,
+    // before the next work is published and launched
+    const unsigned mode = s->active.empty() ? QUEUE_DRAIN : Q.drained && running ? QUEUE_STOP : QUEUE_HOLD;
     if (mode != Q.mode) {
         Q.mode = mode;
         __atomic_store_n(Q.h_mode, mode, __ATOMIC_RELEASE);
         if (mode == QUEUE_DRAIN)
             Q.drained = true;
     }
+    if (mode == QUEUE_STOP)
+        return TMC_OK;
     publish_queue(s);
-    // a launch is needed when work is queued and no launch runs, or when the
-    // running ones may be ending (the mode was DRAIN since they started)
-    if (s->inflight > 0 && (running == 0 || (Q.drained && mode == QUEUE_HOLD))) {
-        const uint32_t cap = s->cfg.waves ? s->cfg.waves : DEFAULT_WAVES;
-        for (Wave &w : s->waves) {
-            if (running >= cap)
-                break;
-            if (w.busy)
-                continue;
-            return launch_persistent(s, w);
-        }
-    }
+    if (s->inflight > 0 && running == 0)
+        for (Wave &w : s->waves)
+            if (!w.busy)
+                return launch_persistent(s, w);
     return TMC_OK;
 }
 
