@@ -3,7 +3,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 
 #include "tmc_device.cuh"
@@ -106,6 +105,11 @@ DeviceCtx *current_ctx(int *status)
             *status = set_cuda_error(e, "cudaMalloc(workspace)");
             return nullptr;
         }
+        e = cudaMallocHost(&c.pinned, PINNED_BYTES);
+        if (e != cudaSuccess) {
+            *status = set_cuda_error(e, "cudaMallocHost");
+            return nullptr;
+        }
         e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
         if (e != cudaSuccess) {
             *status = set_cuda_error(e, "cudaStreamCreate");
@@ -142,8 +146,8 @@ cudaError_t ws_release(DeviceCtx &c, cudaStream_t stream)
     return cudaEventRecord(c.ws_done, stream);
 }
 
-// All of a context's calls use its one stream, so its memory is ordered by that
-// stream and growing or freeing it waits for no other work on the device.
+// All of a context's calls use its one stream, so its device scratch is ordered by
+// that stream and growing or freeing it waits for no other work on the device.
 cudaError_t CallBuffers::device(size_t bytes, size_t keep)
 {
     if (bytes > keep) {
@@ -166,33 +170,37 @@ cudaError_t CallBuffers::device(size_t bytes, size_t keep)
     return cudaSuccess;
 }
 
-cudaError_t CallBuffers::host(size_t bytes)
-{
-    if (bytes > PINNED_KEEP) {
-        pin = static_cast<char *>(std::malloc(bytes));
-        own_pin = pin != nullptr;
-        return pin ? cudaSuccess : cudaErrorMemoryAllocation;
-    }
-    if (bytes > ctx.pinned_cap) {
-        cudaFreeHost(ctx.pinned);
-        ctx.pinned = nullptr;
-        ctx.pinned_cap = 0;
-        const size_t want = std::min(PINNED_KEEP, std::max<size_t>(bytes + bytes / 2, 16384));
-        const cudaError_t e = cudaMallocHost(&ctx.pinned, want);
-        if (e != cudaSuccess)
-            return e;
-        ctx.pinned_cap = want;
-    }
-    pin = static_cast<char *>(ctx.pinned);
-    return cudaSuccess;
-}
-
 CallBuffers::~CallBuffers()
 {
     if (own_dev)
         cudaFreeAsync(dev, ctx.stream);
-    if (own_pin)
-        std::free(pin);
+}
+
+// n results from device memory through pinned memory, from its byte 64 on, in
+// pieces of which one is copied while the one before is taken: take(first, count,
+// data).  The stream's earlier work has ended before the first is taken.
+template <class T, class Take>
+static cudaError_t read_back(DeviceCtx &c, const T *d, size_t n, Take take)
+{
+    size_t piece = (PINNED_BYTES - 64) / sizeof(T);
+    if (n > piece)
+        piece /= 2;
+    T *const half[2] = {reinterpret_cast<T *>(c.pinned + 64), reinterpret_cast<T *>(c.pinned + 64) + piece};
+    auto copy = [&](size_t at, int h) {
+        return cudaMemcpyAsync(half[h], d + at, sizeof(T) * std::min(piece, n - at), cudaMemcpyDeviceToHost, c.stream);
+    };
+    cudaError_t e = copy(0, 0);
+    int h = 0;
+    for (size_t at = 0; at < n; at += piece, h ^= 1) {
+        if (e == cudaSuccess)
+            e = cudaStreamSynchronize(c.stream);
+        if (e == cudaSuccess && at + piece < n)
+            e = copy(at + piece, h ^ 1);
+        if (e != cudaSuccess)
+            return e;
+        take(at, std::min(piece, n - at), half[h]);
+    }
+    return e;
 }
 
 __global__ void tally_to_heat_kernel(const tmc_tally *t, uint32_t shells, double c, double *heat,
@@ -258,14 +266,12 @@ struct HostWalk {
 };
 
 static int walk_into(CallBuffers &buf, DeviceCtx &c, uint64_t n, const tmc_params *p, const Derived &d, bool steps,
-                     size_t pinned, HostWalk &w)
+                     HostWalk &w)
 {
     const size_t S = p->shells;
     cudaError_t e = buf.device(WORKSPACE_BYTES + (sizeof(tmc_tally) + 2 * sizeof(double)) * S, WALK_KEEP);
-    if (e == cudaSuccess)
-        e = buf.host(pinned);
     if (e != cudaSuccess)
-        return set_cuda_error(e, "host-array call's buffers");
+        return set_cuda_error(e, "host-array call's scratch");
     w.tally = reinterpret_cast<tmc_tally *>(buf.dev + WORKSPACE_BYTES);
     w.steps = reinterpret_cast<unsigned long long *>(buf.dev) + 1;
     w.heat = reinterpret_cast<double *>(buf.dev + WORKSPACE_BYTES + sizeof(tmc_tally) * S);
@@ -349,33 +355,29 @@ int tmc_photon_batch_fx(tmc_tally *tally, uint64_t n_photons, const tmc_params *
     if ((st = check_sizes(n_photons, p)))
         return st;
     const Derived d = derive(p->mu_a, p->mu_s, p->microns_per_shell, p->shells);
-    // results in pinned memory: the step count, then the tallies
-    const size_t bytes = sizeof(tmc_tally) * (size_t)p->shells;
     CallBuffers buf(*c);
     HostWalk w{};
-    if ((st = walk_into(buf, *c, n_photons, p, d, true, 64 + bytes, w)))
+    if ((st = walk_into(buf, *c, n_photons, p, d, true, w)))
         return st;
-    const tmc_tally *h = reinterpret_cast<const tmc_tally *>(buf.pin + 64);
-    cudaError_t e = cudaMemcpyAsync(buf.pin + 64, w.tally, bytes, cudaMemcpyDeviceToHost, c->stream);
+    cudaError_t e = cudaMemcpyAsync(c->pinned, w.steps, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(buf.pin, w.steps, sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(c->stream);
+        e = read_back(*c, w.tally, p->shells, [&](size_t first, size_t count, const tmc_tally *h) {
+            tmc_tally *t = tally + first;
+            for (size_t s = 0; s < count; ++s) {
+                unsigned __int128 a = ((unsigned __int128)t[s].w_hi << 64) | t[s].w_lo;
+                unsigned __int128 b = ((unsigned __int128)t[s].w2_hi << 64) | t[s].w2_lo;
+                a += ((unsigned __int128)h[s].w_hi << 64) | h[s].w_lo;
+                b += ((unsigned __int128)h[s].w2_hi << 64) | h[s].w2_lo;
+                t[s].w_lo = (uint64_t)a;
+                t[s].w_hi = (uint64_t)(a >> 64);
+                t[s].w2_lo = (uint64_t)b;
+                t[s].w2_hi = (uint64_t)(b >> 64);
+            }
+        });
     if (e != cudaSuccess)
         return set_cuda_error(e, "tmc_photon_batch_fx");
-    const uint64_t steps = *reinterpret_cast<const uint64_t *>(buf.pin);
-    for (uint32_t s = 0; s < p->shells; ++s) {
-        unsigned __int128 a = ((unsigned __int128)tally[s].w_hi << 64) | tally[s].w_lo;
-        unsigned __int128 b = ((unsigned __int128)tally[s].w2_hi << 64) | tally[s].w2_lo;
-        a += ((unsigned __int128)h[s].w_hi << 64) | h[s].w_lo;
-        b += ((unsigned __int128)h[s].w2_hi << 64) | h[s].w2_lo;
-        tally[s].w_lo = (uint64_t)a;
-        tally[s].w_hi = (uint64_t)(a >> 64);
-        tally[s].w2_lo = (uint64_t)b;
-        tally[s].w2_hi = (uint64_t)(b >> 64);
-    }
     if (photon_steps)
-        *photon_steps += steps;
+        *photon_steps += *reinterpret_cast<const uint64_t *>(c->pinned);
     return TMC_OK;
 }
 
@@ -394,24 +396,26 @@ int tmc_photon_batch(float *heat, float *heat2, uint64_t n_photons, const tmc_pa
     if ((st = check_sizes(n_photons, p)))
         return st;
     const Derived d = derive(p->mu_a, p->mu_s, p->microns_per_shell, p->shells);
-    const uint32_t S = p->shells;
-    const size_t bytes = 2 * sizeof(double) * (size_t)S;
+    const size_t S = p->shells;
     CallBuffers buf(*c);
     HostWalk w{};
-    if ((st = walk_into(buf, *c, n_photons, p, d, false, bytes, w)))
+    if ((st = walk_into(buf, *c, n_photons, p, d, false, w)))
         return st;
-    const double *h = reinterpret_cast<const double *>(buf.pin);
-    cudaError_t e = launch_tally_to_heat(w.tally, S, (double)d.c, w.heat, w.heat + S, c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(buf.pin, w.heat, bytes, cudaMemcpyDeviceToHost, c->stream);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(c->stream);
+    cudaError_t e = launch_tally_to_heat(w.tally, p->shells, (double)d.c, w.heat, w.heat + S, c->stream);
+    auto add = [](float *to, const double *h, size_t count) {
+        for (size_t s = 0; s < count; ++s)
+            to[s] = (float)((double)to[s] + h[s]);
+    };
+    if (e == cudaSuccess)   // S values of heat, then S of heat2
+        e = read_back(*c, w.heat, 2 * S, [&](size_t first, size_t count, const double *h) {
+            const size_t one = first < S ? std::min(count, S - first) : 0;
+            if (one)
+                add(heat + first, h, one);
+            if (count > one)
+                add(heat2 + (first + one - S), h + one, count - one);
+        });
     if (e != cudaSuccess)
         return set_cuda_error(e, "tmc_photon_batch");
-    for (uint32_t s = 0; s < S; ++s) {
-        heat[s] = (float)((double)heat[s] + h[s]);
-        heat2[s] = (float)((double)heat2[s] + h[S + s]);
-    }
     return TMC_OK;
 }
 

@@ -44,12 +44,11 @@ struct DeviceCtx {
     void *workspace = nullptr;          // tmc_workspace_bytes()
     // The host-array calls' own buffers, used under the library's lock on
     // `stream` and finished when a call returns: device scratch, grown to the
-    // largest call so far, and pinned host memory for results, each up to a
-    // bound (a larger call's is its own).
+    // largest call so far up to a bound (a larger call's is its own), and
+    // PINNED_BYTES of pinned host memory that results come through in pieces.
     void *scratch = nullptr;
     size_t scratch_cap = 0;
-    void *pinned = nullptr;
-    size_t pinned_cap = 0;
+    char *pinned = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ws_done = nullptr;      // recorded after the last use of workspace
 };
@@ -63,24 +62,27 @@ void set_error_text(const std::string &s);
 
 constexpr size_t WORKSPACE_BYTES = 256;
 
-// Device scratch and pinned memory for the length of one host-array call.  Kept
-// by the context up to a bound: allocating and freeing them in each call took
-// 140 us of a colour map's 205 (800 x 800) and 6 of a 20-photon call's 39 (stream-ordered
-// memory goes back to the driver at every synchronisation).
-// Bounds: the tallies and results of the largest walk (2^24 shells), images of
-// 64 MB, 4 MB of pinned memory (results beyond come through pageable memory).
-constexpr size_t WALK_KEEP = 1u << 30, IMAGE_KEEP = 64u << 20, PINNED_KEEP = 4u << 20;
+// Pinned memory is allocated with the context and stays: allocating or freeing it
+// can wait for all work on the device, which may itself wait for the host (a
+// persistent server launch).  Larger results come through its halves in turn (2^22
+// shells of heat, 67 MB: 4.0 ms, 7.3 through pageable memory).
+constexpr size_t PINNED_BYTES = 4u << 20;
+
+// Device scratch for the length of one host-array call.  Kept by the context up
+// to a bound: allocating and freeing it in each call took 140 us of a colour map's
+// 205 (800 x 800) and 6 of a 20-photon call's 39 (stream-ordered memory goes back to
+// the driver at every synchronisation).  Bounds: the tallies and results of the
+// largest walk (2^24 shells), images of 64 MB.
+constexpr size_t WALK_KEEP = 1u << 30, IMAGE_KEEP = 64u << 20;
 struct CallBuffers {
     explicit CallBuffers(DeviceCtx &c) : ctx(c) {}
     ~CallBuffers();
     CallBuffers(const CallBuffers &) = delete;
     CallBuffers &operator=(const CallBuffers &) = delete;
     cudaError_t device(size_t bytes, size_t keep);   // once; sets dev
-    cudaError_t host(size_t bytes);                  // once; sets pin
     DeviceCtx &ctx;
     char *dev = nullptr;
-    char *pin = nullptr;
-    bool own_dev = false, own_pin = false;
+    bool own_dev = false;
 };
 
 // The context's workspace (photon claim counter, step counter) is shared by
