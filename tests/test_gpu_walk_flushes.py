@@ -3,7 +3,7 @@ block takes enough photons that its warps empty them in the middle of the walk."
 import numpy as np
 import pytest
 
-from test_gpu_parity import gpu_fx, oracle_fx
+from test_gpu_parity import PARAMS_H, gpu_fx, oracle_fx
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +55,37 @@ def test_last_shell_is_shared_in_every_form(tmc_mod, thin):
             times.append(a.elapsed_time(b))
         ms[shells] = min(times)
     assert ms[other] < 4 * ms[4480], ms
+
+
+LOW_ALBEDO = dict(shells=101, microns_per_shell=50.0, mu_a=10.0, mu_s=1.0)
+
+
+def sms():
+    return pytest.importorskip("torch").cuda.get_device_properties(0).multi_processor_count
+
+
+# The photons per SM from which a launch counts steps instead of summing weights.
+@pytest.mark.parametrize("more", [-1, 0, 1])
+@pytest.mark.parametrize("optics,line", [(PARAMS_H, 900), (LOW_ALBEDO, 256)])
+def test_counts_line_equals_oracle(tmc_mod, oracle_mod, optics, line, more):
+    n = sms() * line + more
+    tmc_mod.set_plain_launch(0, 0, 0)
+    got, steps = gpu_fx(tmc_mod, n, seed=12, base=1 << 35, **optics)
+    ref, _, ref_steps = oracle_fx(oracle_mod, n, seed=12, base=1 << 35, **optics)
+    assert steps == ref_steps and np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("math", ["exact", "fast"])
+@pytest.mark.parametrize("optics,n", [(PARAMS_H, 1 << 25), (LOW_ALBEDO, 800_000_000)])
+def test_counts_emptied_mid_walk(tmc_mod, optics, n, math):
+    """A warp empties its block's counts every 2^22 iterations.  One block of 512
+    threads walks enough photons for that; spread over the device, the same photons
+    end long before it."""
+    tmc_mod.set_plain_launch(0, 1, 1)
+    try:
+        got, steps = gpu_fx(tmc_mod, n, seed=13, base=1 << 36, math=math, **optics)
+    finally:
+        tmc_mod.set_plain_launch(0, 0, 0)
+    assert steps / 512 > 1.1 * (1 << 22)             # iterations of a lane, and more
+    ref, ref_steps = gpu_fx(tmc_mod, n, seed=13, base=1 << 36, math=math, **optics)
+    assert steps == ref_steps and np.array_equal(got, ref)
