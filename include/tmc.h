@@ -388,9 +388,10 @@ int tmc_batch_means_rse(const uint64_t *probes, uint32_t items_per_batch, uint64
                         double *rse, double *mean);
 
 /*
- * Launch shape of the plain walk: threads per block (128, 256 or 512; 0 =
- * default, 512), resident blocks per SM (0 = occupancy limit) and a cap on the
- * grid (0 = none).  Results do not depend on it (integer tallies,
+ * Launch shape of the plain walk: threads per block (128, 256 or 512, which
+ * take the kernels that sum weights; 0 = 128, 512 or the kernel that counts
+ * steps, by the launch's size), resident blocks per SM (0 = occupancy limit)
+ * and a cap on the grid (0 = none).  Results do not depend on it (integer tallies,
  * photon-keyed streams); only speed does.
  */
 int tmc_set_plain_launch(int block, int blocks_per_sm, int max_blocks);

@@ -158,7 +158,8 @@ cudaError_t queue_blocks(const void *kernel, int block, size_t smem, int &per_sm
     const size_t own = 1024;   // shared memory the system takes per block
     auto room = [&](int n) {   // beside n blocks
         return regs - n * block * ((attr.numRegs + 7) / 8 * 8) >= BESIDE_THREADS * BESIDE_REGS &&
-               threads - n * block >= BESIDE_THREADS && (size_t)n * (smem + attr.sharedSizeBytes + own) + own <= (size_t)shared;
+               threads - n * block >= BESIDE_THREADS &&
+               (size_t)n * (smem + attr.sharedSizeBytes + own) + own <= (size_t)shared;
     };
     while (per_sm > 1 && !room(per_sm))
         --per_sm;
@@ -408,7 +409,9 @@ Spread spread(const std::vector<tmc_problem> &problems, const std::vector<double
 // estimated photon steps for `grid` resident blocks of `block` threads with
 // `items_per_block` items each, heaviest first.  Host only.
 // Problems of `whole` expected steps per photon and more, walked one photon to a
-// warp, get items a fifth of the size, down to a photon per warp, ahead of all.
+// warp, get items a fifth of the size, down to a photon per warp, ahead of all
+// (whole items to a twentieth: within 5% in walk_batch for batches of 60 to 4096
+// problems; what counts is that they come first).
 std::vector<BatchItemDev> plan_items(const std::vector<tmc_problem> &problems,
                                      const std::vector<double> &est_steps, int grid, int block,
                                      int items_per_block, double whole = 1e300)

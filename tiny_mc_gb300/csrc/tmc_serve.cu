@@ -422,7 +422,9 @@ uint32_t take_pending(tmc_server *s, uint64_t cap_n, uint64_t quota_base, Put pu
 // Where the launches in flight leave blocks idle, cut a wave's n items into equal
 // pieces for them, as many as the wave has room for, of two photons per thread
 // or more (the kernel's smallest item), or one where a photon is 4096 steps or
-// longer; the pieces with the longest walks of a lane go first.  An item is about
+// longer (12 to 48 requests: the same within 6% with that line anywhere from 0 to
+// 16384, 1.46 to 1.85 times as long with two always); the pieces with the longest
+// walks of a lane go first.  An item is about
 // 8e6 photon steps, 30 ms of one block; 48 requests of 16 such batches on 1216
 // blocks take 34 ms whole and 23 ms in pieces.  Not with a bound on the items
 // in flight, which counts items.  Returns the number of pieces.

@@ -115,13 +115,13 @@ __host__ __device__ constexpr uint32_t flush_steps(uint32_t lanes)
 }
 static_assert(512ull * 257ull * ((1ull << 23) / 512 + 1) < (1ull << 32), "high word bound");
 
-// Cells of a shared histogram or row of counts.  Every photon beyond the last shell deposits
-// into it (photon.c:27-29): in an optically thin problem nearly all lanes of a
-// warp at once, and shared atomics on one word take their turns.  So the last
-// shell has 32 cells, one per lane, which the flushes add up.  2^20 high-albedo
+// Cells of a shared histogram or row of counts.  Every photon beyond the last
+// shell deposits into it (photon.c:27-29): in an optically thin problem nearly all
+// lanes of a warp at once, and shared atomics on one word take their turns.  So the
+// last shell has 32 cells, one per lane, which the flushes add up.  2^20 high-albedo
 // photons (1001 shells of 10 um, many walks leave): 46.8 -> 44.8 ms; the reduced
-// 4096-problem sweep 609 -> 555 ms.  A histogram of sums has them before shell 0, lane
-// l's at -1 - l; counts have them in the last shell's place.
+// 4096-problem sweep 609 -> 555 ms.  A histogram of sums has them before shell 0,
+// lane l's at -1 - l; counts have them in the last shell's place.
 // The split form uses the one at -1 alone: as global atomics on one address 2^21
 // photons of params.h optics over 4600 shells of 0.53 um took 128.7 ms, 1.65 so, 1.16
 // with a cell per lane; but where few photons leave (2000003 photons, 20000 shells of
@@ -461,9 +461,9 @@ __device__ __forceinline__ void launch_photon(LanePhoton &p, unsigned long long 
 // for the next refill): move, deposit and decay unless its direction is still
 // sought, then two tries for the next direction and the roulette.
 // A radius below `last` shells goes to its shell's cell, any other (NaN too) to
-// cell `beyond`, which may be negative.  The tally keeps the photon's weight: step(p, cell) deposits
-// and decays it, low(p) says whether it is below the roulette's threshold,
-// survived(p) and died(p) are the roulette's outcomes.
+// cell `beyond`, which may be negative.  The tally keeps the photon's weight:
+// step(p, cell) deposits and decays it, low(p) says whether it is below the
+// roulette's threshold, survived(p) and died(p) are the roulette's outcomes.
 template <int BLOCK, class M, class Tally>
 __device__ __forceinline__ void step_photon(LanePhoton &p, const char *ring, float spm, float last, float beyond,
                                             Tally &tally)
@@ -1003,9 +1003,9 @@ __device__ __forceinline__ void walk_photons(const WalkConsts &c, float beyond, 
 // (low and high of sum w, then of sum w^2), flushed into g, the problem's global
 // 128-bit tally [shells][4], every flush_steps iterations (the caller flushes
 // what is left).  H = Split, Far: of 4 * hist_cells(near + 1) words, for the first
-// `near` (Far: no) shells and the last.  probe_acc / probe_hi (Block only, may be null):
-// receive the w sums those flushes take from shell
-// probe_shell.  Returns this thread's photon steps.
+// `near` (Far: no) shells and the last.  probe_acc / probe_hi (Block only, may be
+// null): receive the w sums those flushes take from shell probe_shell.  Returns
+// this thread's photon steps.
 template <int BLOCK, class M, class Source, Hist H, int BODY = TRIP>
 __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               const PhiloxKeys &keys, uint32_t *tally,
