@@ -66,7 +66,7 @@ NCU_WALK = {
     "capture": "profiles/walk_counts_fast_2p25photons_ncu_full.txt",
     "sources": ["tiny_mc_gb300/csrc/tmc_device.cuh", "tiny_mc_gb300/csrc/tmc_walk.cuh",
                 "tiny_mc_gb300/csrc/tmc_plain.cu"],
-    "sources_sha256": "a2f658ccba6d4ff1a4a3b6568480be7dae807b38030cf626e146ef28dc000ca1",
+    "sources_sha256": "2bcabed42d36253d34ece4ae4881ff9445a2c10bfa27a96f9e264fbd82f4da1c",
     # thread-instructions (predicated on) per photon step
     "thread_instr_per_step": 136.3,
     # busy fraction of each pipe
@@ -74,7 +74,7 @@ NCU_WALK = {
                    "shared_wavefronts": 0.339, "dram": 0.0},
     # DRAM bytes read + written by one launch (constant and code fetch; the
     # 101-shell tally stays in L2; not proportional to the photon count)
-    "dram_bytes_per_launch": 61184,
+    "dram_bytes_per_launch": 65536,
 }
 
 
