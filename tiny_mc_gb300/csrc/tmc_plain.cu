@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArg
         a.c, src, a.keys, smem, a.tally, my, near);
 
     __syncthreads();
-    flush_tally<BLOCK>(smem, near, S, a.tally);
+    flush_tally<BLOCK, H>(smem, near, S, a.tally);
     if (a.steps) {
         const unsigned long long tot = warp_sum_u64(steps);
         if ((threadIdx.x & 31u) == 0 && tot)

@@ -120,15 +120,28 @@ static_assert(512ull * 257ull * ((1ull << 23) / 512 + 1) < (1ull << 32), "high w
 // lanes of a warp at once, and shared atomics on one word take their turns.  So the
 // last shell has 32 cells, one per lane, which the flushes add up.  2^20 high-albedo
 // photons (1001 shells of 10 um, many walks leave): 46.8 -> 44.8 ms; the reduced
-// 4096-problem sweep 609 -> 555 ms.  A histogram of sums has them before shell 0,
-// lane l's at -1 - l; counts have them in the last shell's place.
-// The split form uses the one at -1 alone: as global atomics on one address 2^21
-// photons of params.h optics over 4600 shells of 0.53 um took 128.7 ms, 1.65 so, 1.16
-// with a cell per lane; but where few photons leave (2000003 photons, 20000 shells of
-// 5 um) 1.007 ms so, 1.023 with a lane's own constant held through the loop, 1.045
-// with the cells behind the near shells (a second compare and a branch's join).
+// 4096-problem sweep 609 -> 555 ms.
+// They stand in the last shell's place, in the split forms before shell 0, and those
+// use the one at -1 alone: as global atomics on one address 2^21 photons of params.h
+// optics over 4600 shells of 0.53 um took 128.7 ms, 1.65 so, 1.16 with a cell per lane;
+// but where few photons leave (2000003 photons, 20000 shells of 5 um) 1.007 ms so, 1.023
+// with a lane's own constant held through the loop, 1.045 with the cells behind the near
+// shells (a second compare and a branch's join).  (Before shell 0 in a whole histogram:
+// 7% slower in walk_batch's 256-thread blocks at albedo 0.99.)
 constexpr uint32_t LAST_CELLS = 32;
 __host__ __device__ constexpr uint32_t hist_cells(uint32_t shells) { return shells + LAST_CELLS - 1; }
+// Index of shell 0's cell, and of the last shell's first, in a histogram of `near`
+// shells and the last.
+template <Hist H>
+__device__ __forceinline__ uint32_t shell0_cell()
+{
+    return H == Hist::Block ? 0 : LAST_CELLS;
+}
+template <Hist H>
+__device__ __forceinline__ uint32_t last_cell(uint32_t near)
+{
+    return H == Hist::Block ? near : 0;
+}
 
 // Take the 64-bit sum of a cell, by atomic exchanges against zero.
 __device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *hi)
@@ -147,13 +160,14 @@ __device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *
 // null): the 128-bit running sum of the w words taken from shell
 // probe_shell.  Warp-collective.  The last shell's cells are added up first
 // (their total obeys the bound below, so it fits 64 bits).
+template <Hist H>
 __device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t near, uint32_t S, unsigned long long *g,
                                                  unsigned long long *probe_acc = nullptr,
                                                  uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
 {
     const uint32_t C = hist_cells(near + 1), lane = threadIdx.x & 31u;
     __syncwarp();
-    uint32_t *const first = tally + LAST_CELLS;
+    uint32_t *const first = tally + shell0_cell<H>(), *const last = tally + last_cell<H>(near);
     for (uint32_t s = lane; s < near; s += 32) {
         const unsigned long long v = take_cell(&first[s], &first[C + s]);
         flush128(&g[4 * s + 0], &g[4 * s + 1], v);
@@ -165,8 +179,8 @@ __device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t near,
         flush128(&g[4 * s + 2], &g[4 * s + 3], take_cell(&first[2 * C + s], &first[3 * C + s]));
     }
     __syncwarp();
-    const unsigned long long v = warp_sum_u64(take_cell(&tally[lane], &tally[C + lane]));
-    const unsigned long long v2 = warp_sum_u64(take_cell(&tally[2 * C + lane], &tally[3 * C + lane]));
+    const unsigned long long v = warp_sum_u64(take_cell(&last[lane], &last[C + lane]));
+    const unsigned long long v2 = warp_sum_u64(take_cell(&last[2 * C + lane], &last[3 * C + lane]));
     if (lane == 0) {
         unsigned long long *gl = g + 4 * (size_t)(S - 1);
         flush128(&gl[0], &gl[1], v);
@@ -1015,13 +1029,13 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
                                               uint32_t probe_shell = 0)
 {
     constexpr uint32_t FLUSH = flush_steps((uint32_t)BLOCK);
-    const float beyond = H != Hist::Block ? -1.0f : -1.0f - (float)(threadIdx.x & 31u);
+    const float beyond = H != Hist::Block ? -1.0f : c.last + (float)(threadIdx.x & 31u);
     if constexpr (H == Hist::Block)
         near = c.shells - 1;
-    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally + LAST_CELLS), 4 * hist_cells(near + 1), g, c.albedo,
-                        (int)near};
+    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally + shell0_cell<H>()), 4 * hist_cells(near + 1), g,
+                        c.albedo, (int)near};
     walk_photons<BLOCK, M, false, FLUSH, BODY>(c, beyond, src, keys, my, t, [&] {
-        warp_flush_tally(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
+        warp_flush_tally<H>(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
     });
     return t.steps;
 }
@@ -1029,17 +1043,17 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
 // Add what is left in a block's histogram (of the first `near` shells and the
 // last of S) to a 128-bit global tally [shells][4], after a barrier.
 // Block-collective.
-template <int BLOCK>
+template <int BLOCK, Hist H>
 __device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t near, uint32_t S, unsigned long long *g)
 {
     const uint32_t C = hist_cells(near + 1);
-    const uint32_t *const first = tally + LAST_CELLS;
+    const uint32_t *const first = tally + shell0_cell<H>();
     for (uint32_t s = threadIdx.x; s < near; s += BLOCK) {
         flush128(&g[4 * s + 0], &g[4 * s + 1], ((unsigned long long)first[C + s] << 32) | first[s]);
         flush128(&g[4 * s + 2], &g[4 * s + 3], ((unsigned long long)first[3 * C + s] << 32) | first[2 * C + s]);
     }
     if (threadIdx.x < 32) {
-        const uint32_t s = threadIdx.x;
+        const uint32_t s = last_cell<H>(near) + threadIdx.x;
         const unsigned long long v = warp_sum_u64(((unsigned long long)tally[C + s] << 32) | tally[s]);
         const unsigned long long v2 = warp_sum_u64(((unsigned long long)tally[3 * C + s] << 32) | tally[2 * C + s]);
         if (threadIdx.x == 0) {
@@ -1054,9 +1068,9 @@ __device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t near, uint
 __device__ __forceinline__ unsigned long long shell_sum(const uint32_t *tally, uint32_t S, uint32_t s)
 {
     const uint32_t C = hist_cells(S);
-    const uint32_t at = s + 1 < S ? LAST_CELLS + s : threadIdx.x & 31u;
     if (s + 1 < S)
-        return ((unsigned long long)tally[C + at] << 32) | tally[at];
+        return ((unsigned long long)tally[C + s] << 32) | tally[s];
+    const uint32_t at = s + (threadIdx.x & 31u);
     return warp_sum_u64(((unsigned long long)tally[C + at] << 32) | tally[at]);
 }
 
