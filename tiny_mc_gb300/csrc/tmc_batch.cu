@@ -379,7 +379,7 @@ Spread spread(const std::vector<tmc_problem> &problems, const std::vector<double
         const double w = k * block / 128.0;
         const double lane_rate = 2.15e11 * size / slow * w / (w + 2.3), lane_step = (0.29 + 0.045 * w) * 1e-6 * slow;
         const double warp_rate = 2.6e10 * size * std::min(1.0, w / 5.0), warp_step = std::max(0.043e-6, 0.016e-6 * w);
-        const double turns = std::ceil(least_items / ((double)k * sms)) * total / photons * lane_step;
+        const double turns = std::max(1.0, least_items / ((double)k * sms)) * total / photons * lane_step;
         double long_work = 0.0, long_rounds = 0.0;   // steps of those problems, and 32 for every round a warp takes
         for (size_t i = 0; i <= p.size(); ++i) {   // the i longest problems' photons one to a warp
             double t = (total - long_work) / lane_rate + long_rounds / warp_rate;
@@ -680,7 +680,7 @@ int tmc_batch_create(tmc_batch **out, const tmc_problem *problems, uint32_t n_pr
         b->est_steps.push_back(expected_steps(d.albedo));
         const double work = b->est_steps.back() * (double)q.n_photons;
         steps += work;
-        brief_steps += d.albedo < SHORT_ALBEDO ? work : 0.0;
+        brief_steps += brief_walk(d.albedo, math) ? work : 0.0;
         hp[i].c.albedo = d.albedo;
         hp[i].c.spm = d.spm;
         hp[i].c.last = d.last;

@@ -475,7 +475,7 @@ int launch_wave(tmc_server *s, Wave &w)
     for (uint32_t i = 0; i < n; ++i) {
         const Req &q = s->active.find(s->slot_req[w.h_items[i].problem])->second;
         steps += w.h_items[i].count * q.est_steps;
-        brief_steps += q.d.albedo < SHORT_ALBEDO ? w.h_items[i].count * q.est_steps : 0.0;
+        brief_steps += brief_walk(q.d.albedo, s->cfg.math) ? w.h_items[i].count * q.est_steps : 0.0;
     }
     w.n_items = n;
     w.head = 0;

@@ -65,8 +65,9 @@ constexpr int SLOTS = RING + MIRROR;
 // photons of params.h optics: 27.8 ms with 4, 27.3 with 6, 26.9 with 8; 2^20
 // high-albedo 44.1, 42.5, 42.3; 2^22 photons of three steps (albedo 0.09)
 // 0.152, 0.169, 0.175 ms.  (Two passes through a body of 4 per check: 27.9.)
-// walk_counts and walk_batch have a kernel of each length.  (Both loops in one
-// kernel, or one that leaves a body of 8 in its middle: 1.5% slower for long walks.)
+// walk_counts and walk_batch (brief_walk) have a kernel of each length.  (Both loops
+// in one kernel, or one that leaves a body of 8 in its middle: 1.5% slower for long
+// walks.)
 constexpr int TRIP = 8, SHORT_TRIP = 4;
 constexpr float SHORT_ALBEDO = 0.8f;   // below: walks of under 31 steps to the first roulette
 
