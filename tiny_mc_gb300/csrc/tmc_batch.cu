@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(bound_threads(BLOCK, QUEUE), 1024 / BLOCK) wal
             probe ? &sh_probe_hi : nullptr, ps);
 
         __syncthreads();
-        flush_tally<BLOCK, Hist::Block>(smem, S - 1, S, g);
+        flush_tally<BLOCK, Hist::Block>(smem, 0, S, g);
         // this item's own sum of w in the probe shell, 128-bit: what the
         // walk's flushes took from the shell plus what is left in it
         unsigned long long probe_lo = 0;

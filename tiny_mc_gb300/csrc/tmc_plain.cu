@@ -81,9 +81,9 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArg
 {
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t S = a.c.shells;
-    const uint32_t near = H == Hist::Split ? split_near(BLOCK, S) : H == Hist::Far ? 0 : S - 1;
+    const uint32_t near = H == Hist::Split ? split_near(BLOCK, S) : 0;   // (the whole form counts on S alone)
     // words per histogram
-    const uint32_t hist = 4 * (H == Hist::Split ? split_cells(BLOCK) : hist_cells(near + 1));
+    const uint32_t hist = 4 * (H == Hist::Split ? split_cells(BLOCK) : hist_cells(H == Hist::Far ? 1 : S));
     for (uint32_t s = threadIdx.x; s < hist; s += BLOCK)
         smem[s] = 0;
     __syncthreads();
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) walk_plain(const PlainArg
         a.c, src, a.keys, smem, a.tally, my, near);
 
     __syncthreads();
-    flush_tally<BLOCK, H>(smem, near, S, a.tally);
+    flush_tally<BLOCK, H>(smem, near, a.c.shells, a.tally);
     if (a.steps) {
         const unsigned long long tot = warp_sum_u64(steps);
         if ((threadIdx.x & 31u) == 0 && tot)

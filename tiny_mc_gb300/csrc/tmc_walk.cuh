@@ -151,21 +151,23 @@ __device__ __forceinline__ unsigned long long take_cell(uint32_t *lo, uint32_t *
     return ((unsigned long long)h << 32) | l;
 }
 
-// Add a histogram of the first `near` shells and the last of S into the 128-bit
-// global tally and clear it (near = S - 1: all shells), by one warp while the
-// others keep depositing: every word is taken with an atomic exchange against
-// zero.  Sums stay exact: a deposit's low-word overflow is
-// carried into a high word by the depositing lane, whichever side of an
-// exchange either add lands on, and every word's content reaches the global
-// tally at one flush or the next.  probe_acc / probe_hi (shared, may be
-// null): the 128-bit running sum of the w words taken from shell
-// probe_shell.  Warp-collective.  The last shell's cells are added up first
-// (their total obeys the bound below, so it fits 64 bits).
+// Add a histogram of the first `near` shells (H = Block: all) and the last of S into
+// the 128-bit global tally and clear it, by one warp while the others keep
+// depositing: every word is taken with an atomic exchange against zero.  Sums stay
+// exact: a deposit's low-word overflow is carried into a high word by the
+// depositing lane, whichever side of an exchange either add lands on, and every
+// word's content reaches the global tally at one flush or the next.  probe_acc /
+// probe_hi (shared, may be null): the 128-bit running sum of the w words taken from
+// shell probe_shell.  Warp-collective.  The last shell's cells are added up first
+// (their total obeys the bound above, so it fits 64 bits).  (Block's shell count is
+// not passed: a register held for it through the loop costs 0.5 - 4%.)
 template <Hist H>
 __device__ __forceinline__ void warp_flush_tally(uint32_t *tally, uint32_t near, uint32_t S, unsigned long long *g,
                                                  unsigned long long *probe_acc = nullptr,
                                                  uint32_t *probe_hi = nullptr, uint32_t probe_shell = 0)
 {
+    if constexpr (H == Hist::Block)
+        near = S - 1;
     const uint32_t C = hist_cells(near + 1), lane = threadIdx.x & 31u;
     __syncwarp();
     uint32_t *const first = tally + shell0_cell<H>(), *const last = tally + last_cell<H>(near);
@@ -1031,22 +1033,23 @@ __device__ __forceinline__ uint32_t walk_loop(const WalkConsts c, Source &src,
 {
     constexpr uint32_t FLUSH = flush_steps((uint32_t)BLOCK);
     const float beyond = H != Hist::Block ? -1.0f : c.last + (float)(threadIdx.x & 31u);
-    if constexpr (H == Hist::Block)
-        near = c.shells - 1;
-    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally + shell0_cell<H>()), 4 * hist_cells(near + 1), g,
-                        c.albedo, (int)near};
+    const uint32_t cells = hist_cells(H == Hist::Block ? c.shells : near + 1);
+    WeightTally<M, H> t{(uint32_t)__cvta_generic_to_shared(tally + shell0_cell<H>()), 4 * cells, g, c.albedo,
+                        (int)near};
     walk_photons<BLOCK, M, false, FLUSH, BODY>(c, beyond, src, keys, my, t, [&] {
         warp_flush_tally<H>(tally, near, c.shells, g, probe_acc, probe_hi, probe_shell);
     });
     return t.steps;
 }
 
-// Add what is left in a block's histogram (of the first `near` shells and the
-// last of S) to a 128-bit global tally [shells][4], after a barrier.
+// Add what is left in a block's histogram (of the first `near` shells, H = Block:
+// all, and the last of S) to a 128-bit global tally [shells][4], after a barrier.
 // Block-collective.
 template <int BLOCK, Hist H>
 __device__ __forceinline__ void flush_tally(uint32_t *tally, uint32_t near, uint32_t S, unsigned long long *g)
 {
+    if constexpr (H == Hist::Block)
+        near = S - 1;
     const uint32_t C = hist_cells(near + 1);
     const uint32_t *const first = tally + shell0_cell<H>();
     for (uint32_t s = threadIdx.x; s < near; s += BLOCK) {
