@@ -66,7 +66,7 @@ NCU_WALK = {
     "capture": "profiles/walk_counts_fast_2p25photons_ncu_full.txt",
     "sources": ["tiny_mc_gb300/csrc/tmc_device.cuh", "tiny_mc_gb300/csrc/tmc_walk.cuh",
                 "tiny_mc_gb300/csrc/tmc_plain.cu"],
-    "sources_sha256": "2bcabed42d36253d34ece4ae4881ff9445a2c10bfa27a96f9e264fbd82f4da1c",
+    "sources_sha256": "c4706b11c9cddeb150d298c6bfc49364cecf0febbb2bf1a34f38c4ebf9b0dab0",
     # thread-instructions (predicated on) per photon step
     "thread_instr_per_step": 136.3,
     # busy fraction of each pipe
@@ -74,7 +74,7 @@ NCU_WALK = {
                    "shared_wavefronts": 0.339, "dram": 0.0},
     # DRAM bytes read + written by one launch (constant and code fetch; the
     # 101-shell tally stays in L2; not proportional to the photon count)
-    "dram_bytes_per_launch": 65536,
+    "dram_bytes_per_launch": 61184,
 }
 
 
